@@ -29,6 +29,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "ieee_int.h"
 #include "kernels.h"
 #include "tci_functions.h"
 #include "tci_tasks.h"
@@ -62,6 +63,7 @@ struct CtlT {
   int r, c, K, stop, kmax, need_exact, bar_err;
   int status;
   double piv, maxerror, err;
+  int factors[2];  // flags of the entries that joined L and U, by pivot parity (JoinFlags)
   double red_s[W + 1];
   int red_k[W + 1];
   unsigned long long red_u[W + 1];
@@ -105,47 +107,37 @@ __device__ __forceinline__ bool is_nan_bits(double v) { return abs_bits(v) > 0x7
 // (matrices have at most 65535 rows and columns).
 __device__ __forceinline__ uint32_t pack_key(int i, int j) { return ((uint32_t)j << 16) | (uint32_t)i; }
 
-// One thread's running argmax of |v| in key order, integer pipe only: A = the
-// largest |v| bit pattern + 1, k = its first key, B = the largest bit pattern
-// + 1 below A (0 = none).  NaN never wins (the reference's scan starts from
-// typemin and compares with '>').
+// One thread's running argmax of |v| (pushed in any key order), integer pipe
+// only: A = the largest |v| bit pattern + 1, k = its smallest key, B = the
+// largest bit pattern + 1 below A (0 = none).  NaN never wins (the reference's
+// scan starts from typemin and compares with '>').
 struct ArgTrack {
   uint64_t A, B;
-  uint32_t k;
+  uint32_t k, sgn;  // sgn: the sign bit of the element at k
   __device__ __forceinline__ void init() {
     A = B = 0;
     k = 0xffffffffu;
+    sgn = 0;
   }
   __device__ __forceinline__ void push(double v, uint32_t key) {
     uint64_t b = abs_bits(v);
     if (b > NAN_FLOOR) return;
     b += 1;
-    if (b > A) {
-      B = A;
+    const bool win = b > A || (b == A && key < k);
+    B = b > A ? A : (b < A && b > B ? b : B);
+    if (win) {
       A = b;
       k = key;
-    } else if (b < A && b > B) {
-      B = b;
+      sgn = (uint32_t)__double2hiint(v) & 0x80000000u;
     }
   }
-};
-__device__ __forceinline__ void track_combine(uint64_t& A, uint32_t& k, uint64_t& B, uint64_t A2, uint32_t k2,
-                                              uint64_t B2) {
-  if (A2 > A) {
-    B = B2 > A ? B2 : A;
-    A = A2;
-    k = k2;
-  } else if (A2 == A) {
-    B = B2 > B ? B2 : B;
-    k = k2 < k ? k2 : k;
-  } else if (A2 > B) {
-    B = A2;
+  // the element at k
+  __device__ __forceinline__ double value() const {
+    return __longlong_as_double((long long)((A ? A - 1 : 0) | ((uint64_t)sgn << 32)));
   }
-}
-
+};
 // Warp-wide versions with the hardware reductions (redux.sync) instead of a
-// shuffle tree; every lane gets the result.  warp_track gives what folding
-// track_combine over the lanes gives in any order: the largest A, the smallest
+// shuffle tree; every lane gets the result.  warp_track: the largest A, the smallest
 // key among the lanes that hold it, and B = the largest value below A held
 // anywhere (a lane below the maximum offers its A, a lane at it its B).
 __device__ __forceinline__ uint64_t warp_max_u64(uint64_t x) {
@@ -197,6 +189,7 @@ __device__ void block_argmax(const ArgBest& a, Ctl& ctl, uint64_t& out_s, uint32
   uint64_t s = a.s;
   uint32_t key = a.key;
   warp_best(s, key);
+  __syncthreads();  // the slots may still be read
   if (lane == 0) {
     ctl.red_u[warp] = s;
     ctl.red_k[warp] = (int)key;
@@ -269,67 +262,67 @@ __device__ void exact_argmax(const double* A, int lda, int r0, int rows, int c0,
   block_argmax(ab, ctl, s, key);
 }
 
-// The pivot of the next step (submatrixargmax of abs2, matrixlu.jl:1-32) from
-// every thread's ArgTrack over the block A[r0:, c0:]; sets ctl.r / ctl.c and
-// ends with a barrier.  One integer reduction decides it unless some element
-// other than the largest |v| lies within 16 ulps of it (its square could tie)
-// or the magnitude is where squares underflow or overflow; then the exact
-// second pass runs.  `decide` runs on the one thread that sets ctl.r / ctl.c,
-// before the final barrier (the next pivot's decision without a barrier of its own).
-struct NoDecide {
-  __device__ void operator()() const {}
+// The pivot of the next step (submatrixargmax of abs2, matrixlu.jl:1-32): its
+// place and value.
+struct Pick {
+  int r, c;
+  double piv;
 };
-template <class Decide = NoDecide>
-__device__ void argmax_resolve(const ArgTrack& t, const double* A, int lda, int r0, int rows, int c0, int cols,
-                               Ctl& ctl, const Decide& decide = Decide()) {
+// Whether the largest |v| (A - 1, runner-up B - 1) decides the argmax of abs2:
+// no element other than the largest |v| lies within 16 ulps of it (its square
+// could tie), and the magnitude is not where squares underflow or overflow.
+__device__ __forceinline__ bool track_decides(uint64_t A, uint64_t B) {
+  const uint64_t M = A - 1;
+  return A != 0 && M >= SQ_SMALL && M < SQ_BIG && (B == 0 || (B - 1) + 16 < M);
+}
+
+// From every thread's ArgTrack over the block A[r0:, c0:] to every thread: one
+// barrier.  Each warp writes its winner, and every warp reduces the NW winners
+// itself: the pivot step needs no second barrier to hand the result out.  The
+// winner's value travels with it, so no thread reads A here (the next step's
+// swaps may already be under way in other warps).  The exact pass and a block
+// of NaNs only (the scan keeps its start) do read A, with barriers of their own.
+__device__ Pick argmax_pick(const ArgTrack& t, const double* A, int lda, int r0, int rows, int c0, int cols,
+                            Ctl& ctl) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint64_t a = t.A, b = t.B;
   uint32_t k = t.k;
   warp_track(a, k, b);
-  if (lane == 0) {
+  if (t.A == a && t.k == k) {  // one lane (any, when nothing was tracked)
     ctl.red_u[warp] = a;
     ctl.red_b[warp] = b;
     ctl.red_k[warp] = (int)k;
+    ctl.red_s[warp] = t.value();
   }
   __syncthreads();
-  if (warp == 0) {
-    a = lane < NW ? ctl.red_u[lane] : 0ULL;
-    b = lane < NW ? ctl.red_b[lane] : 0ULL;
-    k = lane < NW ? (uint32_t)ctl.red_k[lane] : 0xffffffffu;
-    warp_track(a, k, b);
-    if (lane == 0) {
-      const uint64_t Mstar = a ? a - 1 : 0;
-      const bool safe = Mstar >= SQ_SMALL && Mstar < SQ_BIG;
-      const bool close = b != 0 && (b - 1) + 16 >= Mstar;
-      if (a == 0) {  // every element NaN: the scan keeps its start
-        ctl.r = r0;
-        ctl.c = c0;
-        ctl.need_exact = 0;
-        decide();
-      } else if (safe && !close) {
-        ctl.r = (int)(k & 0xffffu);
-        ctl.c = (int)(k >> 16);
-        ctl.need_exact = 0;
-        decide();
-      } else {
-        ctl.need_exact = 1;
-      }
-      ctl.red_u[NW] = Mstar;
-    }
+  const uint64_t wa = lane < NW ? ctl.red_u[lane] : 0ULL;
+  const uint32_t wk = lane < NW ? (uint32_t)ctl.red_k[lane] : 0xffffffffu;
+  const double wv = lane < NW ? ctl.red_s[lane] : 0.0;
+  a = wa;
+  k = wk;
+  b = lane < NW ? ctl.red_b[lane] : 0ULL;
+  warp_track(a, k, b);
+  Pick p;
+  if (track_decides(a, b)) {
+    p.r = (int)(k & 0xffffu);
+    p.c = (int)(k >> 16);
+    p.piv = __shfl_sync(FULL, wv, __ffs(__ballot_sync(FULL, wa == a && wk == k)) - 1);
+    return p;
   }
-  __syncthreads();
-  if (ctl.need_exact) {
-    const uint64_t Mstar = ctl.red_u[NW];
+  p.r = r0;
+  p.c = c0;
+  if (a != 0) {
     uint64_t s;
     uint32_t key;
-    exact_argmax(A, lda, r0, rows, c0, cols, Mstar, ctl, s, key);
-    if (threadIdx.x == 0) {
-      ctl.r = s ? (int)(key & 0xffffu) : r0;
-      ctl.c = s ? (int)(key >> 16) : c0;
-      decide();
+    exact_argmax(A, lda, r0, rows, c0, cols, a - 1, ctl, s, key);
+    if (s) {
+      p.r = (int)(key & 0xffffu);
+      p.c = (int)(key >> 16);
     }
-    __syncthreads();
   }
+  p.piv = A[p.r + (size_t)p.c * lda];
+  __syncthreads();
+  return p;
 }
 
 __device__ int block_or(int v, Ctl& ctl) {
@@ -534,98 +527,279 @@ __device__ ResPtrs res_ptrs(char* resb, const tci_task& T) {
   return p;
 }
 
-// Pivot decision of _optimizerrlu! (matrixlu.jl:150-158) for the pivot at
-// (ctl.r, ctl.c): lu.error, the stopping rule, and the permutation bookkeeping of
-// addpivot!.  One thread.
-__device__ void rr_decide(Ctl& ctl, const double* A, int lda, int K, double reltol, double abstol, double* diag_out,
-                          int* rowperm, int* colperm) {
-  const int r = ctl.r, c = ctl.c;
-  const double piv = A[r + (size_t)c * lda];
-  const double e = fabs(piv);
-  ctl.err = e;
-  const int stop = ((e < reltol * ctl.maxerror || e < abstol) && K > 0) ? 1 : 0;
-  ctl.stop = stop;
-  if (!stop) {
-    ctl.maxerror = jmax(ctl.maxerror, e);
-    ctl.piv = piv;
-    diag_out[K] = e;
-    int t = rowperm[K];
-    rowperm[K] = rowperm[r];
-    rowperm[r] = t;
-    t = colperm[K];
-    colperm[K] = colperm[c];
-    colperm[c] = t;
+// Bit pattern of a stopping threshold for integer comparison with |pivot| (the
+// patterns of non-negative doubles order like their values): NaN and negative
+// thresholds, below which nothing lies, become zero.
+__device__ __forceinline__ uint64_t threshold_bits(double t) {
+  const uint64_t b = (uint64_t)__double_as_longlong(t);
+  return b > 0x7ff0000000000000ULL ? 0ull : b;
+}
+
+// State of the pivot loop, the same in every thread that runs it.
+struct PivotState {
+  uint64_t err, maxerror, thr;  // bit patterns of lu.error, maxerror and max(reltol * maxerror, abstol)
+  __device__ __forceinline__ void init(double reltol, double abstol) {
+    err = 0x7ff8000000000000ULL;
+    maxerror = 0;
+    thr = max(threshold_bits(reltol * 0.0), threshold_bits(abstol));
   }
+  // Decision of _optimizerrlu! (matrixlu.jl:150-158) for a pivot: lu.error and
+  // the stopping rule, on the integer pipe; reltol * maxerror is formed only
+  // when maxerror grows.  Returns whether to stop.
+  __device__ __forceinline__ bool decide(double piv, int K, double reltol, double abstol) {
+    const uint64_t e = abs_bits(piv);
+    err = e;
+    if (e < thr && K > 0) return true;
+    if (e > maxerror) {  // also when the pivot is NaN; a NaN maxerror stays
+      maxerror = (uint64_t)__double_as_longlong(
+          jmax(__longlong_as_double((long long)maxerror), __longlong_as_double((long long)e)));
+      thr = max(threshold_bits(reltol * __longlong_as_double((long long)maxerror)), threshold_bits(abstol));
+    }
+    return false;
+  }
+};
+// The permutation bookkeeping of addpivot! and the pivot's entry of diag, by one thread.
+__device__ __forceinline__ void record_pivot(const Pick& p, int K, double* diag_out, int* rowperm, int* colperm) {
+  diag_out[K] = __longlong_as_double((long long)abs_bits(p.piv));
+  const int a = rowperm[K], b = rowperm[p.r], c = colperm[K], d = colperm[p.c];
+  rowperm[K] = b;
+  rowperm[p.r] = a;
+  colperm[K] = d;
+  colperm[p.c] = c;
 }
 
 // swaprow!(K, R), swapcol!(K, C) and the scaling of addpivot! (matrixlu.jl:98-124)
 // in one pass: new(i, j) = old(pr(i), pc(j)) with pr, pc the two transpositions,
 // divided by the pivot in column K below the diagonal (leftorthogonal) or in row
-// K right of it.  The moved elements form disjoint pairs -- rows K/R outside
-// columns K/C, columns K/C outside rows K/R, and the corners -- and each pair is
-// read and written by one thread.  Ends with a barrier.
+// K right of it.  Written for the scaled direction: "line" K and line C are the
+// columns for leftorthogonal, and the rows otherwise (strides si within a line
+// and sj across).  Item i < mi swaps entry i of the two lines and scales the new
+// one; item R also does the four corners, so that one division site serves all
+// entries; items mi + j swap entries (K, j) and (R, j) of the other lines.
 // The body for threads t = 0, stride, ... of a group (no barrier).
-// nan: set when an entry of the new row K (columns >= K) or of the new column K
-// (rows >= K) is NaN -- the entries that join U and L at this pivot.  Every
-// other entry of L and U joined at an earlier pivot (swaps only move them), so
-// the flags of all pivots cover the NaN check of L and U (matrixlu.jl:162-169).
-__device__ __forceinline__ void swap_scale_body(double* A, int lda, int m, int n, int K, int R, int C, double piv,
-                                                bool leftorth, int t, int stride, bool& nan) {
-  for (int w = t; w < n + m + 1; w += stride) {
-    if (w < n) {  // row pair (K, j) <-> (R, j)
-      const int j = w;
-      if (j == K || j == C) continue;
-      double* col = A + (size_t)j * lda;
-      if (R != K) {
-        const double a = col[K], b = col[R];
-        const double v = (!leftorth && j > K) ? __ddiv_rn(b, piv) : b;
-        col[K] = v;
-        col[R] = a;
-        if (j > K && is_nan_bits(v)) nan = true;
-      } else if (j > K) {
-        const double v = !leftorth ? __ddiv_rn(col[K], piv) : col[K];
-        col[K] = v;
-        if (is_nan_bits(v)) nan = true;
-      }
-    } else if (w < n + m) {  // column pair (i, K) <-> (i, C)
-      const int i = w - n;
-      if (i == K || i == R) continue;
-      double* ck = A + (size_t)K * lda;
-      if (C != K) {
-        double* cc = A + (size_t)C * lda;
-        const double a = ck[i], b = cc[i];
-        const double v = (leftorth && i > K) ? __ddiv_rn(b, piv) : b;
-        ck[i] = v;
-        cc[i] = a;
-        if (i > K && is_nan_bits(v)) nan = true;
-      } else if (i > K) {
-        const double v = leftorth ? __ddiv_rn(ck[i], piv) : ck[i];
-        ck[i] = v;
-        if (is_nan_bits(v)) nan = true;
-      }
-    } else {  // the corners (K, K), (K, C), (R, K), (R, C)
-      const int rows[2] = {K, R}, cols[2] = {K, C};
-      const int nr = R != K ? 2 : 1, nc = C != K ? 2 : 1;
-      double old[2][2];
-      for (int p = 0; p < nr; ++p)
-        for (int q = 0; q < nc; ++q) old[p][q] = A[rows[p] + (size_t)cols[q] * lda];
-      for (int p = 0; p < nr; ++p)
-        for (int q = 0; q < nc; ++q) {
-          // source of (rows[p], cols[q]) is (rows[p^1], cols[q^1]) where swapped
-          const int sp = nr == 2 ? 1 - p : p, sq = nc == 2 ? 1 - q : q;
-          double v = old[sp][sq];
-          const int i = rows[p], j = cols[q];
-          if ((leftorth && j == K && i > K) || (!leftorth && i == K && j > K)) v = __ddiv_rn(v, piv);
-          A[i + (size_t)j * lda] = v;
-          if ((i == K || j == K) && is_nan_bits(v)) nan = true;
+// The entries of the new row K (columns >= K) and of the new column K (rows >=
+// K) join U and L at this pivot; every other entry of L and U joined at an
+// earlier one (swaps only move them), so the flags of all pivots cover the NaN
+// check of L and U (matrixlu.jl:162-169).
+struct JoinFlags {
+  bool nan;     // an entry that joined is NaN
+  int factors;  // of this pivot: 2 an entry is not int_safe, 1 one is not int_dense
+  __device__ __forceinline__ void join(double v) {
+    if (!int_dense(v)) factors |= 1;
+    if (!int_safe(v)) {
+      factors |= 2;
+      if (is_nan_bits(v)) nan = true;
+    }
+  }
+};
+// How the products of a rank-1 update are taken: all factors dense, some of
+// them not (decided per tile), or on the FP64 pipe.
+enum { PROD_DENSE = 0, PROD_MIXED = 1, PROD_FP64 = 2 };
+// The scaling divides a whole row or column by one pivot: on the integer pipe
+// (int_div) unless the pivot or the entry is outside its range.  An FP64
+// division holds an SM quarter's FP64 pipe for 548 cycles.
+struct PivotDivisor {
+  double piv;
+  bool safe;
+  IntDivisor d;
+  __device__ __forceinline__ explicit PivotDivisor(double p) : piv(p), safe(int_safe(p) && (abs_bits(p) != 0)) {
+    d = int_divisor(p);
+  }
+  __device__ __forceinline__ double quo(double v) const {
+    return safe && int_safe(v) ? int_div(v, d) : __ddiv_rn(v, piv);
+  }
+};
+__device__ __forceinline__ void swap_scale_body(double* A, int lda, int m, int n, int K, const Pick& p,
+                                                bool leftorth, int t, int stride, JoinFlags& fl) {
+  const PivotDivisor D(p.piv);
+  const int mi = leftorth ? m : n, nj = leftorth ? n : m;
+  const int R = leftorth ? p.r : p.c, C = leftorth ? p.c : p.r;
+  const int si = leftorth ? 1 : lda, sj = leftorth ? lda : 1;
+  for (int w = t; w < mi + nj; w += stride) {
+    if (w < mi) {
+      const int i = w;
+      if (i == K && R != K) continue;  // done by item R
+      double* const pk = A + (size_t)i * si + (size_t)K * sj;
+      double* const pc = A + (size_t)i * si + (size_t)C * sj;
+      double a = *pk, v = *pc;
+      if (i == R && R != K) {
+        double* const qk = A + (size_t)K * si + (size_t)K * sj;
+        double* const qc = A + (size_t)K * si + (size_t)C * sj;
+        const double ork = a;
+        a = *qk;
+        v = *qc;
+        *qk = p.piv;
+        if (C != K) {
+          *qc = ork;
+          fl.join(ork);
         }
+      }
+      if (i > K) {
+        v = D.quo(v);
+        fl.join(v);
+      }
+      *pk = v;
+      if (C != K) {
+        *pc = a;
+        if (i == K) fl.join(a);
+      }
+    } else {
+      const int j = w - mi;
+      if (j == K || j == C) continue;
+      double* const pk = A + (size_t)K * si + (size_t)j * sj;
+      if (R != K) {
+        double* const pr = A + (size_t)R * si + (size_t)j * sj;
+        const double a = *pk, v = *pr;
+        *pr = a;
+        *pk = v;
+        if (j > K) fl.join(v);
+      } else if (j > K) {
+        fl.join(*pk);
+      }
+    }
+  }
+  if (is_nan_bits(p.piv)) fl.nan = true;
+}
+// Every thread gets how the update's products are taken.  The flags go through
+// a shared word per pivot parity (a barrier with a reduction costs three plain
+// ones); rrlu_loop clears it.
+__device__ int swap_scale(double* A, int lda, int m, int n, int K, const Pick& p, bool leftorth, JoinFlags& fl,
+                          Ctl& ctl) {
+  fl.factors = 0;
+  swap_scale_body(A, lda, m, n, K, p, leftorth, threadIdx.x, NT, fl);
+  if (fl.factors) atomicOr(&ctl.factors[K & 1], fl.factors);
+  __syncthreads();
+  return min(ctl.factors[K & 1], (int)PROD_FP64);
+}
+
+// x_i * y_j of an R x C group per lane.  The subtraction that follows stays on
+// the FP64 pipe; the bits are those of the FP64 multiplication in every mode.
+template <int MODE, int R, int C>
+__device__ __forceinline__ void tile_products(const double (&x)[R], const double (&y)[C], double (&q)[R][C]) {
+  bool dense = MODE == PROD_DENSE;
+  if (MODE == PROD_MIXED) {
+    bool d = true;
+#pragma unroll
+    for (int a = 0; a < R; ++a) d = d && int_dense(x[a]);
+#pragma unroll
+    for (int b = 0; b < C; ++b) d = d && int_dense(y[b]);
+    dense = __all_sync(FULL, d);
+  }
+  if (MODE == PROD_FP64) {
+#pragma unroll
+    for (int b = 0; b < C; ++b)
+#pragma unroll
+      for (int a = 0; a < R; ++a) q[a][b] = __dmul_rn(x[a], y[b]);
+  } else if (dense) {
+    DenseFactor xf[R], yf[C];
+#pragma unroll
+    for (int a = 0; a < R; ++a) xf[a] = dense_split(x[a]);
+#pragma unroll
+    for (int b = 0; b < C; ++b) yf[b] = dense_split(y[b]);
+#pragma unroll
+    for (int b = 0; b < C; ++b)
+#pragma unroll
+      for (int a = 0; a < R; ++a) q[a][b] = int_mul_dense(xf[a], yf[b]);
+  } else {
+    IntFactor xf[R], yf[C];
+#pragma unroll
+    for (int a = 0; a < R; ++a) xf[a] = int_split(x[a]);
+#pragma unroll
+    for (int b = 0; b < C; ++b) yf[b] = int_split(y[b]);
+#pragma unroll
+    for (int b = 0; b < C; ++b)
+#pragma unroll
+      for (int a = 0; a < R; ++a) q[a][b] = int_mul(xf[a], yf[b]);
+  }
+}
+
+// A[K:, K:] -= x y^T by warp `warp` of `nw`, each element tracked for the next
+// pivot: x[i] and y[j * ystride] for i, j >= K, A column-major.
+//
+// FP64-bound: the products are taken on the integer pipes (ieee_int.h), so the
+// FP64 pipe is used once per element instead of twice.  A warp takes 16 x 8
+// tiles, its lanes laid out 8 x 4 with 2 x 2 elements each: x and y are taken
+// apart once per four products, the four chains of a thread overlap, and the
+// ragged ends waste at most half a tile.  Indices past the end repeat the last
+// row or column (not stored).  104 x 104, two 256-thread CTAs per SM: 0.68
+// cycles per element and SM (1.20 with FP64 products walked element by
+// element); 16 x 16 tiles 0.76, 16 x 4 tiles 0.72.
+// Tracking: only elements whose |v| has a top word of at least the warp's
+// largest so far less one can be the maximum or lie within 16 ulps of it, so
+// a tile costs one vote and is pushed element by element only if it reaches that.
+template <int MODE>
+__device__ __forceinline__ void rank1_tiles(double* A, int lda, int K, int m, int n, const double* x, const double* y,
+                                            int ystride, int warp, int nw, ArgTrack& at) {
+  const int lane = threadIdx.x & 31, lr = lane & 7, lc = lane >> 3;
+  const int nti = (m - K + 15) >> 4, ntj = (n - K + 7) >> 3;
+  int tj = warp / nti, ti = warp - tj * nti;
+  const int dj = nw / nti, di = nw - dj * nti;
+  uint32_t top = 0;  // top word of the largest |v| pushed by the warp
+  while (tj < ntj) {
+    const int i0 = K + 16 * ti + lr, j0 = K + 8 * tj + lc;
+    const bool vi[2] = {i0 < m, i0 + 8 < m}, vj[2] = {j0 < n, j0 + 4 < n};
+    const int ii[2] = {min(i0, m - 1), min(i0 + 8, m - 1)}, jj[2] = {min(j0, n - 1), min(j0 + 4, n - 1)};
+    double* const p[2] = {A + (size_t)jj[0] * lda, A + (size_t)jj[1] * lda};
+    double v[2][2], xv[2], yv[2], q[2][2];
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) v[a][b] = p[b][ii[a]];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      xv[a] = x[ii[a]];
+      yv[a] = y[(size_t)jj[a] * ystride];
+    }
+    tile_products<MODE>(xv, yv, q);
+    uint32_t h = 0;
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        v[a][b] = __dsub_rn(v[a][b], q[a][b]);
+        if (vi[a] && vj[b]) p[b][ii[a]] = v[a][b];
+        h = max(h, (uint32_t)__double2hiint(v[a][b]) & 0x7fffffffu);
+      }
+    if (__any_sync(FULL, h + 1 >= top)) {
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+          if (vi[a] && vj[b]) at.push(v[a][b], pack_key(ii[a], jj[b]));
+      top = __reduce_max_sync(FULL, at.A ? (uint32_t)((at.A - 1) >> 32) : 0u);
+    }
+    ti += di;
+    tj += dj;
+    if (ti >= nti) {
+      ti -= nti;
+      tj += 1;
     }
   }
 }
-__device__ void swap_scale(double* A, int lda, int m, int n, int K, int R, int C, double piv, bool leftorth,
-                           bool& nan) {
-  swap_scale_body(A, lda, m, n, K, R, C, piv, leftorth, threadIdx.x, NT, nan);
-  __syncthreads();
+// The two rarer modes are kept out of line: their code is shared by the CTA and
+// the one-warp loop.
+__device__ __noinline__ ArgTrack rank1_mixed(double* A, int lda, int K, int m, int n, const double* x,
+                                             const double* y, int ystride, int warp, int nw) {
+  ArgTrack at;
+  at.init();
+  rank1_tiles<PROD_MIXED>(A, lda, K, m, n, x, y, ystride, warp, nw, at);
+  return at;
+}
+__device__ __noinline__ ArgTrack rank1_fp64(double* A, int lda, int K, int m, int n, const double* x, const double* y,
+                                            int ystride, int warp, int nw) {
+  ArgTrack at;
+  at.init();
+  rank1_tiles<PROD_FP64>(A, lda, K, m, n, x, y, ystride, warp, nw, at);
+  return at;
+}
+__device__ __forceinline__ ArgTrack rank1_update(double* A, int lda, int K, int m, int n, const double* x,
+                                                 const double* y, int ystride, int warp, int nw, int mode) {
+  if (mode == PROD_MIXED) return rank1_mixed(A, lda, K, m, n, x, y, ystride, warp, nw);
+  if (mode == PROD_FP64) return rank1_fp64(A, lda, K, m, n, x, y, ystride, warp, nw);
+  ArgTrack at;
+  at.init();
+  rank1_tiles<PROD_DENSE>(A, lda, K, m, n, x, y, ystride, warp, nw, at);
+  return at;
 }
 
 // Trailing blocks of at most this many elements are finished by warp 0 alone:
@@ -633,200 +807,118 @@ __device__ void swap_scale(double* A, int lda, int m, int n, int K, int R, int C
 // per lane one warp beats the barriers of the whole CTA.
 constexpr int WARP_TAIL_RRLU = 192;
 
-// rrlu_loop from pivot K on (decision for K already taken, not stopped), warp 0
-// only; same arithmetic and argmax as the CTA path.  Returns the final K on
-// every lane of warp 0.
+// rrlu_loop from pivot K on (pick `p` taken, not stopped), warp 0 only; same
+// arithmetic and argmax as the CTA path.  Returns the final K on every lane.
 __device__ int rrlu_warp_tail(double* A, int lda, int m, int n, int K, int kmax, double reltol, double abstol,
-                              bool leftorth, int* rowperm, int* colperm, double* diag_out, Ctl& ctl, bool& nan) {
+                              bool leftorth, int* rowperm, int* colperm, double* diag_out, Pick p, PivotState& S,
+                              JoinFlags& fl) {
   const int lane = threadIdx.x & 31;
   while (true) {
-    swap_scale_body(A, lda, m, n, K, ctl.r, ctl.c, ctl.piv, leftorth, lane, 32, nan);
+    fl.factors = 0;
+    swap_scale_body(A, lda, m, n, K, p, leftorth, lane, 32, fl);
+    int mode = PROD_DENSE;
+    if (__any_sync(FULL, fl.factors != 0)) mode = __any_sync(FULL, fl.factors >= 2) ? PROD_FP64 : PROD_MIXED;
     __syncwarp();
     ++K;
     if (K == kmax) break;
-    ArgTrack at;
-    at.init();
-    {
-      const double* x = A + (size_t)(K - 1) * lda;
-      const int rows = m - K;
-      const int total = rows * (n - K);
-      const int sq = 32 / rows, sr = 32 % rows;
-      int jj = lane / rows, ii = lane % rows;
-      for (int e = lane; e < total; e += 32) {
-        const int i = K + ii, j = K + jj;
-        double* col = A + (size_t)j * lda;
-        const double v = __dsub_rn(col[i], __dmul_rn(x[i], col[K - 1]));
-        col[i] = v;
-        at.push(v, pack_key(i, j));
-        ii += sr;
-        jj += sq;
-        if (ii >= rows) {
-          ii -= rows;
-          jj += 1;
-        }
-      }
-    }
+    const ArgTrack at = rank1_update(A, lda, K, m, n, A + (size_t)(K - 1) * lda, A + (K - 1), lda, 0, 1, mode);
     uint64_t a = at.A, b = at.B;
     uint32_t k = at.k;
     warp_track(a, k, b);
-    __syncwarp();  // every lane's update is in place before the exact pass / decision
-    const uint64_t Mstar = a ? a - 1 : 0;
-    const bool safe = Mstar >= SQ_SMALL && Mstar < SQ_BIG;
-    const bool close = b != 0 && (b - 1) + 16 >= Mstar;
-    int r, c;
-    if (a == 0) {
-      r = K;
-      c = K;
-    } else if (safe && !close) {
-      r = (int)(k & 0xffffu);
-      c = (int)(k >> 16);
-    } else {  // squares of the elements near the maximum
-      ArgBest ab;
-      ab.init();
-      const int rows = m - K, total = rows * (n - K);
-      for (int e = lane; e < total; e += 32) {
-        const int i = K + e % rows, j = K + e / rows;
-        const double v = A[i + (size_t)j * lda];
-        if (near_max(abs_bits(v), Mstar)) ab.consider(v, pack_key(i, j));
+    __syncwarp();  // every lane's update is in place before the exact pass and the next swaps
+    if (track_decides(a, b)) {
+      p.r = (int)(k & 0xffffu);
+      p.c = (int)(k >> 16);
+      p.piv = __shfl_sync(FULL, at.value(), __ffs(__ballot_sync(FULL, at.A == a && at.k == k)) - 1);
+    } else {
+      p.r = p.c = K;
+      if (a != 0) {  // squares of the elements near the maximum
+        ArgBest ab;
+        ab.init();
+        const int rows = m - K, total = rows * (n - K);
+        for (int e = lane; e < total; e += 32) {
+          const int i = K + e % rows, j = K + e / rows;
+          const double v = A[i + (size_t)j * lda];
+          if (near_max(abs_bits(v), a - 1)) ab.consider(v, pack_key(i, j));
+        }
+        uint64_t sv = ab.s;
+        uint32_t key = ab.key;
+        warp_best(sv, key);
+        if (sv) {
+          p.r = (int)(key & 0xffffu);
+          p.c = (int)(key >> 16);
+        }
       }
-      uint64_t sv = ab.s;
-      uint32_t key = ab.key;
-      warp_best(sv, key);
-      r = sv ? (int)(key & 0xffffu) : K;
-      c = sv ? (int)(key >> 16) : K;
+      p.piv = A[p.r + (size_t)p.c * lda];
+      __syncwarp();
     }
-    if (lane == 0) {
-      ctl.r = r;
-      ctl.c = c;
-      rr_decide(ctl, A, lda, K, reltol, abstol, diag_out, rowperm, colperm);
-    }
-    __syncwarp();
-    if (ctl.stop) break;
+    if (S.decide(p.piv, K, reltol, abstol)) break;
+    if (lane == 0) record_pivot(p, K, diag_out, rowperm, colperm);
   }
   return K;
 }
 
-// The rrLU main loop (matrixlu.jl:141-181) on A (m x n, leading dim lda) with the
-// first argmax already in ctl.r/ctl.c.  rowperm/colperm are full permutations.
-// Per pivot: one swap/scale pass, the rank-1 update fused with the next argmax,
-// whose resolving thread also takes the next decision -- three barriers.
+// The rrLU main loop (matrixlu.jl:141-181) on A (m x n, leading dim lda) from
+// the first pick.  rowperm/colperm are full permutations.  Per pivot: one
+// swap/scale pass and the rank-1 update fused with the next argmax, whose
+// decision every thread takes itself -- two barriers.
 // xy: optional shared-memory copy (m + n doubles) of the pivot column and row
 // for a matrix in global memory, so that each element of the update costs one
 // load and one store.  Returns this thread's part of the NaN check of L and U
 // (an OR over the CTA gives it).
 __device__ bool rrlu_loop(double* A, int lda, int m, int n, int maxrank, double reltol, double abstol,
-                          bool leftorth, int* rowperm, int* colperm, double* diag_out, Ctl& ctl,
+                          bool leftorth, int* rowperm, int* colperm, double* diag_out, Pick p, Ctl& ctl,
                           double* xy = nullptr, int warp_tail = WARP_TAIL_RRLU) {
   const int tid = threadIdx.x;
   const int kmax = min(maxrank, min(m, n));
-  bool nan = false;
-  if (tid == 0) {
-    ctl.K = 0;
-    ctl.maxerror = 0.0;
-    ctl.err = __longlong_as_double(0x7ff8000000000000LL);
-    ctl.kmax = kmax;
-    ctl.stop = 1;
-    if (kmax > 0) rr_decide(ctl, A, lda, 0, reltol, abstol, diag_out, rowperm, colperm);
-  }
-  __syncthreads();
+  JoinFlags fl{false, 0};
+  PivotState S;
+  S.init(reltol, abstol);
   int K = 0;
+  bool go = kmax > 0 && !S.decide(p.piv, 0, reltol, abstol);
   bool tail = false;
-  while (!ctl.stop) {
+  if (go && tid == 0) record_pivot(p, 0, diag_out, rowperm, colperm);
+  if (tid < 2) ctl.factors[tid] = 0;
+  __syncthreads();
+  while (go) {
     TCI_PHASE(1);
     if ((m - K) * (n - K) <= warp_tail) {
       tail = true;
       break;
     }
-    swap_scale(A, lda, m, n, K, ctl.r, ctl.c, ctl.piv, leftorth, nan);
+    const int mode = swap_scale(A, lda, m, n, K, p, leftorth, fl, ctl);
     TCI_PHASE(3);
     ++K;
     if (K == kmax) break;  // the trailing update after the last pivot is not observable
-    // A[K:, K:] -= x * y^T fused with the argmax of abs2 for the next pivot.
-    // The trailing block is walked as one column-major sequence so that every
-    // lane of every warp has an element (no half-empty warps at column ends).
-    ArgTrack at;
-    at.init();
-    const int rows = m - K;
-    const long long total = (long long)rows * (n - K);
-    const int sq = NT / rows, sr = NT % rows;  // stride NT as (columns, rows)
-    if (xy) {
-      // x = A[K:, K-1] and y = A[K-1, K:] on chip, indexed from K
+    // A[K:, K:] -= x * y^T fused with the argmax of abs2 for the next pivot
+    const double *x = A + (size_t)(K - 1) * lda, *y = A + (K - 1);
+    int ystride = lda;
+    if (xy) {  // x = A[K:, K-1] and y = A[K-1, K:] on chip, indexed from K
       double* xs = xy;
       double* ys = xy + m;
-      for (int i = K + tid; i < m; i += NT) xs[i] = A[i + (size_t)(K - 1) * lda];
-      for (int j = K + tid; j < n; j += NT) ys[j] = A[(K - 1) + (size_t)j * lda];
+      for (int i = K + tid; i < m; i += NT) xs[i] = x[i];
+      for (int j = K + tid; j < n; j += NT) ys[j] = y[(size_t)j * lda];
       __syncthreads();
-      int jj = tid / rows, ii = tid % rows;
-      long long e = tid;
-      // four elements per step with their global loads issued first; the keys
-      // still reach the tracker in increasing order
-      for (; e + 3LL * NT < total; e += 4LL * NT) {
-        int i4[4], j4[4];
-        double a4[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          i4[q] = K + ii;
-          j4[q] = K + jj;
-          ii += sr;
-          jj += sq;
-          if (ii >= rows) {
-            ii -= rows;
-            jj += 1;
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) a4[q] = A[i4[q] + (size_t)j4[q] * lda];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const double v = __dsub_rn(a4[q], __dmul_rn(xs[i4[q]], ys[j4[q]]));
-          A[i4[q] + (size_t)j4[q] * lda] = v;
-          at.push(v, pack_key(i4[q], j4[q]));
-        }
-      }
-      for (; e < total; e += NT) {
-        const int i = K + ii, j = K + jj;
-        double* col = A + (size_t)j * lda;
-        const double v = __dsub_rn(col[i], __dmul_rn(xs[i], ys[j]));
-        col[i] = v;
-        at.push(v, pack_key(i, j));
-        ii += sr;
-        jj += sq;
-        if (ii >= rows) {
-          ii -= rows;
-          jj += 1;
-        }
-      }
-    } else {
-      const double* x = A + (size_t)(K - 1) * lda;
-      int jj = tid / rows, ii = tid % rows;
-      for (long long e = tid; e < total; e += NT) {
-        const int i = K + ii, j = K + jj;
-        double* col = A + (size_t)j * lda;
-        double v = __dsub_rn(col[i], __dmul_rn(x[i], col[K - 1]));
-        col[i] = v;
-        at.push(v, pack_key(i, j));
-        ii += sr;
-        jj += sq;
-        if (ii >= rows) {
-          ii -= rows;
-          jj += 1;
-        }
-      }
+      x = xs;
+      y = ys;
+      ystride = 1;
     }
+    const ArgTrack at = rank1_update(A, lda, K, m, n, x, y, ystride, tid >> 5, NW, mode);
     TCI_PHASE(4);
-    const int Kc = K;
-    argmax_resolve(at, A, lda, K, m - K, K, n - K, ctl,
-                   [&] { rr_decide(ctl, A, lda, Kc, reltol, abstol, diag_out, rowperm, colperm); });
+    p = argmax_pick(at, A, lda, K, m - K, K, n - K, ctl);
+    if (tid == 0) ctl.factors[(K - 1) & 1] = 0;  // read by all before the pick's barrier, set again two pivots on
+    go = !S.decide(p.piv, K, reltol, abstol);
+    if (go && tid == 0) record_pivot(p, K, diag_out, rowperm, colperm);
     TCI_PHASE(6);
   }
   if (tail && tid < 32) K = rrlu_warp_tail(A, lda, m, n, K, kmax, reltol, abstol, leftorth, rowperm, colperm,
-                                           diag_out, ctl, nan);
+                                           diag_out, p, S, fl);
   if (tid == 0) {
     ctl.K = K;
-    if (K >= min(m, n)) ctl.err = 0.0;
+    ctl.err = K >= min(m, n) ? 0.0 : __longlong_as_double((long long)S.err);
   }
   __syncthreads();
-  return nan;
+  return fl.nan;
 }
 
 // left(MatrixLUCI) for leftorthogonal (colstimespivotinv, matrixluci.jl:48-57):
@@ -935,15 +1027,28 @@ __device__ void task_rrlu(const tci_task& T, const char* blob, char* resb, char*
   if (T.ain) {
     // the input is read once: evict-first loads keep it from pushing the
     // working matrices (re-read every pivot) out of L2
-    for (int j = warp; j < n; j += NW) {
-      const double* src = T.ain + (size_t)j * m;
-      double* dst = A + (size_t)j * lda;
-      for (int i = lane; i < m; i += 32) {
-        double v = __ldcs(src + i);
-        dst[i] = v;
-        am.push(v, pack_key(i, j));
-        unsigned long long b = abs_bits(v);
-        mx = b > mx ? b : mx;
+    // the input is one contiguous run (lda = m); eight loads in flight per thread
+    const size_t total = (size_t)m * n;
+    const int sq = NT / m, sr = NT - sq * m;
+    int j = tid / m, i = tid - j * m;
+    for (size_t e0 = tid; e0 < total; e0 += 8 * NT) {
+      double v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = e0 + q * NT < total ? __ldcs(T.ain + e0 + q * NT) : 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (e0 + q * NT < total) {
+          A[e0 + q * NT] = v[q];
+          am.push(v[q], pack_key(i, j));
+          const unsigned long long b = abs_bits(v[q]);
+          mx = b > mx ? b : mx;
+        }
+        i += sr;
+        j += sq;
+        if (i >= m) {
+          i -= m;
+          j += 1;
+        }
       }
     }
   } else {
@@ -976,12 +1081,12 @@ __device__ void task_rrlu(const tci_task& T, const char* blob, char* resb, char*
   __syncthreads();
   unsigned long long mxall = block_max_u64(mx, ctl);
   if (tid == 0) ctl.status = 0;
-  argmax_resolve(am, A, lda, 0, m, 0, n, ctl);
+  const Pick first = argmax_pick(am, A, lda, 0, m, 0, n, ctl);
   const bool leftorth = T.leftorth != 0;
   double* xy = nullptr;
   if (T.smem_mode != 1 && (size_t)(cur.p - smem) + (size_t)(m + n) * 8 <= smem_bytes) xy = (double*)cur.take((size_t)(m + n) * 8);
   const bool nan_part = rrlu_loop(A, lda, m, n, T.maxrank, T.reltol, T.abstol, leftorth, rowperm, colperm, rp.diag,
-                                  ctl, xy, T.tail_elems > 0 ? T.tail_elems : WARP_TAIL_RRLU);
+                                  first, ctl, xy, T.tail_elems > 0 ? T.tail_elems : WARP_TAIL_RRLU);
   const int K = ctl.K;
   // NaN check of L = tril(A[:, 1:K]) and U = triu(A[1:K, :]) (matrixlu.jl:162-169),
   // gathered while the pivots were taken
@@ -2082,6 +2187,68 @@ struct BigArgs {
   double reltol, abstol;
 };
 
+// The rank-1 update of a CTA's block: the active rows and columns (lists of
+// local indices) of A at (r0, c0), x and y by list position, the logical
+// positions for the argmax keys.  As rank1_tiles, but a warp takes 32 x 4 tiles
+// with one row and four columns per lane: the block is read from L2 / L1, where
+// 32 rows of a column are two lines (8 x 4 lanes touched four, 14.6 ms instead
+// of 11.7 for a 2048 x 2048 matrix to rank 512).
+struct BigBlock {
+  double* A;
+  int m, r0, c0, nr, nc;
+  const double *xs, *ys;
+  const int *act_r, *act_c, *pos_r, *pos_c;
+  bool rev;
+};
+template <int MODE>
+__device__ __forceinline__ void big_update(const BigBlock B, BigTrack& bt) {
+  const int lane = threadIdx.x & 31;
+  const int nti = (B.nr + 31) >> 5, ntj = (B.nc + 3) >> 2;
+  const int di = BIG_NW % nti, dj = BIG_NW / nti;
+  int tj = (threadIdx.x >> 5) / nti, ti = (threadIdx.x >> 5) - tj * nti;
+  uint32_t top = 0;
+  while (tj < ntj) {
+    const int t = 32 * ti + lane, u0 = 4 * (B.rev ? ntj - 1 - tj : tj);
+    const bool vi = t < B.nr;
+    const int tt = min(t, B.nr - 1);
+    const int ri = B.r0 + B.act_r[tt];
+    double v[4], xv[1], yv[4], q[1][4];
+    double* p[4];
+    int cj[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int uu = min(u0 + b, B.nc - 1);
+      cj[b] = B.c0 + B.act_c[uu];
+      yv[b] = B.ys[uu];
+      p[b] = B.A + (size_t)cj[b] * B.m + ri;
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) v[b] = *p[b];
+    xv[0] = B.xs[tt];
+    tile_products<MODE>(xv, yv, q);
+    uint32_t h = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      v[b] = __dsub_rn(v[b], q[0][b]);
+      if (vi && u0 + b < B.nc) *p[b] = v[b];
+      h = max(h, (uint32_t)__double2hiint(v[b]) & 0x7fffffffu);
+    }
+    if (__any_sync(FULL, h + 1 >= top)) {
+      const int lr = B.pos_r[ri];
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        if (vi && u0 + b < B.nc) bt.push(v[b], pack_key(lr, B.pos_c[cj[b]]), pack_key(ri, cj[b]));
+      top = __reduce_max_sync(FULL, bt.A ? (uint32_t)((bt.A - 1) >> 32) : 0u);
+    }
+    ti += di;
+    tj += dj;
+    if (ti >= nti) {
+      ti -= nti;
+      tj += 1;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
   extern __shared__ __align__(16) char smem[];
   __shared__ BigCtl ctl;
@@ -2105,9 +2272,10 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
   for (int j = tid; j < n; j += BIG_NT) pos_c[j] = stor_c[j] = j;
   for (int t = tid; t < nrb; t += BIG_NT) act_r[t] = slot_r[t] = t;  // local indices
   for (int u = tid; u < ncb; u += BIG_NT) act_c[u] = slot_c[u] = u;
+  PivotState S;  // thread 0's
+  S.init(P.reltol, P.abstol);
   if (tid == 0) {
-    ctl.maxerror = 0.0;
-    ctl.err = __longlong_as_double(0x7ff8000000000000LL);
+    ctl.factors[0] = ctl.factors[1] = 0;
     ctl.stop = 0;
     ctl.r = nrb;  // active row / column counts
     ctl.c = ncb;
@@ -2141,13 +2309,12 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
     const int rl = (int)(key & 0xffffu), cl = (int)(key >> 16);
     const int R = (int)(ph & 0xffffu), Cc = (int)(ph >> 16);
     const double piv = ctl.piv;
-    const double e = fabs(piv);
-    ctl.err = e;
-    ctl.stop = ((e < P.reltol * ctl.maxerror || e < P.abstol) && K > 0) ? 1 : 0;
+    ctl.stop = S.decide(piv, K, P.reltol, P.abstol) ? 1 : 0;
+    ctl.err = __longlong_as_double((long long)S.err);
+    ctl.factors[(K + 1) & 1] = 0;  // the flags of pivot K - 1: every thread has passed them
     if (!ctl.stop) {
-      ctl.maxerror = jmax(ctl.maxerror, e);
       if (b == 0) {
-        diag[K] = e;
+        diag[K] = fabs(piv);
         P.pivs[K] = piv;
       }
       // swaprow!(K, rl), swapcol!(K, cl) on the maps
@@ -2277,68 +2444,32 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
     // ---- x (pivot column) for the active rows, y (pivot row) for the active columns
     // (one element per thread: the x and y entries on different threads)
     const int nr = ctl.r, nc = ctl.c;
+    const PivotDivisor D(piv);
+    JoinFlags fl{false, 0};
     for (int t = tid; t < nr + nc; t += BIG_NT) {
       if (t < nr) {
         const double v = __ldcg(&P.A[r0 + act_r[t] + (size_t)Cc * m]);
-        xs[t] = leftorth ? __ddiv_rn(v, piv) : v;
+        xs[t] = leftorth ? D.quo(v) : v;
+        fl.join(xs[t]);
       } else {
         const int u = t - nr;
         const double v = __ldcg(&P.A[R + (size_t)(c0 + act_c[u]) * m]);
-        ys[u] = leftorth ? v : __ddiv_rn(v, piv);
+        ys[u] = leftorth ? v : D.quo(v);
+        fl.join(ys[u]);
       }
     }
+    if (fl.factors) atomicOr(&ctl.factors[(K - 1) & 1], fl.factors);
     __syncthreads();
+    const int mode = min(ctl.factors[(K - 1) & 1], (int)PROD_FP64);
     // ---- rank-1 update of the block's active part, fused with its argmax.
-    // Four elements per step with their loads issued first (four L2 reads in
-    // flight per thread); the columns are walked in reverse on odd pivots, so
-    // the part of the block the last pass touched last is still in L1.
+    // The columns are walked in reverse on odd pivots, so the part of the block
+    // the last pass touched last is still in L1.
     bt.init();
     if (nr > 0 && nc > 0) {
-      const long long tot = (long long)nr * nc;
-      const int sq = BIG_NT / nr, sr = BIG_NT % nr;
-      const bool rev = (K & 1) != 0;
-      int tt = tid % nr, uu = tid / nr;
-      long long e = tid;
-      for (; e + 3LL * BIG_NT < tot; e += 4LL * BIG_NT) {
-        int ti[4], ui[4];
-        double* ap[4];
-        double av[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          ti[q] = tt;
-          ui[q] = rev ? nc - 1 - uu : uu;
-          ap[q] = P.A + (r0 + act_r[ti[q]]) + (size_t)(c0 + act_c[ui[q]]) * m;
-          tt += sr;
-          uu += sq;
-          if (tt >= nr) {
-            tt -= nr;
-            uu += 1;
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) av[q] = *ap[q];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const double v = __dsub_rn(av[q], __dmul_rn(xs[ti[q]], ys[ui[q]]));
-          *ap[q] = v;
-          const int i = r0 + act_r[ti[q]], j = c0 + act_c[ui[q]];
-          bt.push(v, pack_key(pos_r[i], pos_c[j]), pack_key(i, j));
-        }
-      }
-      for (; e < tot; e += BIG_NT) {
-        const int u = rev ? nc - 1 - uu : uu;
-        const int i = r0 + act_r[tt], j = c0 + act_c[u];
-        double* a = P.A + i + (size_t)j * m;
-        const double v = __dsub_rn(*a, __dmul_rn(xs[tt], ys[u]));
-        *a = v;
-        bt.push(v, pack_key(pos_r[i], pos_c[j]), pack_key(i, j));
-        tt += sr;
-        uu += sq;
-        if (tt >= nr) {
-          tt -= nr;
-          uu += 1;
-        }
-      }
+      const BigBlock B{P.A, m, r0, c0, nr, nc, xs, ys, act_r, act_c, pos_r, pos_c, (K & 1) != 0};
+      if (mode == PROD_DENSE) big_update<PROD_DENSE>(B, bt);
+      else if (mode == PROD_MIXED) big_update<PROD_MIXED>(B, bt);
+      else big_update<PROD_FP64>(B, bt);
     }
     block_track_to0(bt, ctl);
     // read at pivot K (already incremented); no grid barrier: the next gather

@@ -43,3 +43,8 @@ def test_index_sets_randomized(T, tmp_path):
     inputs (both union paths, many duplicates), and the task layouts' global
     scratch sizes."""
     _run_checker(T, tmp_path, "indexset_random_check")
+
+
+def test_integer_products_and_quotients(T, tmp_path):
+    """int_mul / int_div (ieee_int.h) equal the host's IEEE operations."""
+    _run_checker(T, tmp_path, "ieee_int_check")
