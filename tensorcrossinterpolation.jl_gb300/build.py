@@ -31,6 +31,7 @@ CU_SOURCES = [
     ("step_kernel.cu", "step_kernel_k512.cu.o",
      ["-fmad=false", "-DTCI_KNS=tci_k512", "-DTCI_STEP_THREADS=512", "-DTCI_CTAS_PER_SM=1", "-DTCI_SECONDARY"]),
     ("contract.cu", "contract.cu.o", ["-fmad=false"]),
+    ("tt_eval.cu", "tt_eval.cu.o", ["-fmad=false"]),
     ("peak.cu", "peak.cu.o", []),
     ("gather.cu", "gather.cu.o", []),
     ("fcache.cu", "fcache.cu.o", []),

@@ -593,20 +593,22 @@ int tci_get_history(const tci_solve* s, int64_t* ranks, double* errors, int64_t*
   return 0;
 }
 
+// Train values at packed points, in blocks of 2^22 points (device memory).
+static int train_values(tci_ctx* ctx, const Solve& s, const std::vector<uint8_t>& pts, int64_t np, double* out) {
+  const int64_t chunk = 1 << 22;
+  for (int64_t b = 0; b < np; b += chunk) {
+    int rc = ctx->eng_ref().eval_train(s, pts.data() + b * s.L, std::min(chunk, np - b), out + b);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
 int tci_evaluate(tci_solve* s, const int64_t* points, int64_t np, double* out) {
   std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
   std::vector<uint8_t> pts;
   int rc = pack_points(points, np, s->s.L, s->s.d, pts);
   if (rc) return rc;
-  // up to 2^20 points per engine step (split into tasks inside co_evaluate)
-  const int64_t chunk = 1 << 20;
-  for (int64_t b = 0; b < np; b += chunk) {
-    int64_t n = std::min(chunk, np - b);
-    CoTask t = co_evaluate(s->ctx->eng_ref(), s->s, pts.data() + b * s->s.L, n, nullptr, out + b);
-    rc = run_solve(s->ctx, s->s, t);
-    if (rc) return rc;
-  }
-  return 0;
+  return train_values(s->ctx, s->s, pts, np, out);
 }
 
 int tci_sum(tci_solve* s, double* out) {
@@ -1837,14 +1839,7 @@ int tci_tt_evaluate(tci_ctx* ctx, int32_t L, const int64_t* dims, const double* 
   if (rc) return rc;
   std::vector<uint8_t> pts;
   rc = pack_points(points, np, L, s.d, pts);
-  if (!rc) {
-    const int64_t chunk = 1 << 20;
-    for (int64_t b = 0; b < np && !rc; b += chunk) {
-      const int64_t n = std::min(chunk, np - b);
-      CoTask t = co_evaluate(e, s, pts.data() + b * L, n, nullptr, out + b);
-      rc = e.run(t);
-    }
-  }
+  if (!rc) rc = train_values(ctx, s, pts, np, out);
   e.release_cores(s);
   return rc;
 }

@@ -15,6 +15,9 @@
 #include <numeric>
 #include <thread>
 
+int tci_tt_eval_max_bond();
+cudaError_t tci_tt_eval_launch(const tci_core_ref* cores, int* cls, int L, int rmax, const uint8_t* pts, int64_t np,
+                               double* out, int num_sms, cudaStream_t st);
 cudaError_t tci_gather_launch(const void* table_dev, int n, double* dst_dev, int grid, cudaStream_t stream);
 using tci_k256::tci_rrlu_big_fits;
 using tci_k256::tci_rrlu_big_launch;
@@ -1794,6 +1797,46 @@ CoTask co_evaluate(Engine& e, Solve& s, const uint8_t* pts, i64 np, double* fout
     if (ttout) std::memcpy(ttout + p0, r.ttvals(), (size_t)r.t.m * 8);
   }
   co_return 0;
+}
+
+// Train values alone at np points (packed, 0-based): one launch over all of them.
+int Engine::eval_train(const Solve& s, const uint8_t* pts, int64_t np, double* out) {
+  if (fc_callback_depth()) return reentry();
+  if (!s.cores_valid) return fail(TCI_ERR_GENERIC, "site tensors are not available");
+  if (np <= 0) return 0;
+  std::vector<tci_core_ref> tab;
+  int rmax = 1;
+  core_table(s, tab, rmax);
+  if (rmax > tci_tt_eval_max_bond()) return fail(TCI_ERR_TOO_LARGE, "a bond exceeds the evaluation kernel's shared memory");
+  const size_t L = (size_t)s.L;
+  const size_t o_cls = a16(L * sizeof(tci_core_ref)), o_out = o_cls + a16(L * sizeof(int)),
+               o_pts = o_out + a16((size_t)np * 8), total = o_pts + (size_t)np * L;
+  char* d = (char*)alloc_core((total + 7) / 8);
+  if (!d) return fail(TCI_ERR_OOM, "device memory for evaluation");
+  cudaError_t ce = cudaMemcpyAsync(d, tab.data(), L * sizeof(tci_core_ref), cudaMemcpyHostToDevice, stream_);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(d + o_pts, pts, (size_t)np * L, cudaMemcpyHostToDevice, stream_);
+  if (ce == cudaSuccess && timing) ce = cudaEventRecord(ev0_, stream_);
+  if (ce == cudaSuccess)
+    ce = tci_tt_eval_launch((const tci_core_ref*)d, (int*)(d + o_cls), s.L, rmax, (const uint8_t*)(d + o_pts), np,
+                            (double*)(d + o_out), num_sms, stream_);
+  if (ce == cudaSuccess && timing) ce = cudaEventRecord(ev1_, stream_);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(out, d + o_out, (size_t)np * 8, cudaMemcpyDeviceToHost, stream_);
+  const cudaError_t sync = cudaStreamSynchronize(stream_);
+  free_core((double*)d);
+  if (ce == cudaSuccess) ce = sync;
+  if (ce != cudaSuccess) return fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
+  if (timing) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ev0_, ev1_);
+    stats.kernel_ms += ms;
+  }
+  stats.launches += 2;
+  stats.h2d_bytes += (int64_t)(L * sizeof(tci_core_ref) + (size_t)np * L);
+  stats.d2h_bytes += (int64_t)np * 8;
+  int64_t macs = 0;
+  for (const tci_core_ref& c : tab) macs += (int64_t)c.r0 * c.r1;
+  stats.dense_macs += macs * np;
+  return 0;
 }
 
 CoTask co_sum(Engine& e, Solve& s, double* out) {

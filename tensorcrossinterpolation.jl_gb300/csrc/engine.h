@@ -287,6 +287,8 @@ class Engine {
   // rrLU of a given matrix runs on the multi-CTA kernel (run_big).
   int run_tasks(std::vector<Req*>& reqs);
   int run_big(Req& r);
+  // evaluate(tt, points) for np packed 0-based points (np x L) of the solve's train.
+  int eval_train(const Solve& s, const uint8_t* pts, int64_t np, double* out);
   // Copy many device arrays to one host buffer: gather on the device into a
   // contiguous staging buffer, then a single device-to-host copy.
   int gather_to_host(const std::vector<const double*>& src, const std::vector<int64_t>& len,

@@ -1,0 +1,173 @@
+// evaluate(tt, indexset) (abstracttensortrain.jl:124-132) at many points in FP64:
+// v <- v * T_s[:, i_s, :] site by site, v[q] = sum_t v[t] T_s[t, i, q] summed in
+// order of t with separate multiply and add, as the oracle's loop.
+//
+// FP64-bound once every SM has work: one addition per multiply-add on the FP64
+// pipe, the product on the integer pipes (ieee_int.h).  A CTA carries a block of
+// P points through the train, their vectors in shared memory as [bond][point];
+// a thread takes one point and four outputs at a time, so each v[t] is loaded
+// and taken apart once per four products, the points of a warp share the lines
+// of the core (one per local value), and four independent sums hide the
+// latency.  100 000 points of a 30-site train with bonds of 80: 447 ms with a
+// warp per point in 25 tasks, 38 ms so (both with the copies).
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "ieee_int.h"
+#include "tci_tasks.h"
+
+namespace {
+
+constexpr int NT = 512;
+// What the entries of a core, or of the vectors of a CTA's points, allow.
+enum { VAL_DENSE = 0, VAL_ZEROS = 1, VAL_UNSAFE = 2 };
+
+__device__ __forceinline__ int val_class(double v) {
+  return int_safe(v) ? (int_dense(v) ? VAL_DENSE : VAL_ZEROS) : VAL_UNSAFE;
+}
+
+// Largest class of each core's entries into cls (cleared before).
+__global__ void __launch_bounds__(256) core_class_kernel(const tci_core_ref* cores, int* cls) {
+  const tci_core_ref c = cores[blockIdx.x];
+  const int64_t n = (int64_t)c.r0 * c.d * c.r1;
+  int k = VAL_DENSE;
+  for (int64_t e = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.y * blockDim.x)
+    k = max(k, val_class(c.p[e]));
+  k = __reduce_max_sync(0xffffffffu, k);
+  if ((threadIdx.x & 31) == 0 && k) atomicMax(&cls[blockIdx.x], k);
+}
+
+// acc[k] += v[t] * col[t + k * stride], t = 0 .. r0-1, k < Q; v has stride P.
+template <int MODE, int Q>
+__device__ __forceinline__ void row_times_cols(const double* __restrict__ v, int P, const double* __restrict__ col,
+                                               size_t stride, int r0, double (&acc)[Q]) {
+  double x = v[0], c[Q];
+#pragma unroll
+  for (int k = 0; k < Q; ++k) c[k] = __ldg(col + k * stride);
+  for (int t = 0; t < r0; ++t) {
+    // the next step's loads before this one's arithmetic
+    const int tn = t + 1 < r0 ? t + 1 : t;
+    const double xn = v[(size_t)tn * P];
+    double cn[Q];
+#pragma unroll
+    for (int k = 0; k < Q; ++k) cn[k] = __ldg(col + tn + k * stride);
+    double q[Q];
+    if (MODE == VAL_DENSE) {
+      const DenseFactor xf = dense_split(x);
+#pragma unroll
+      for (int k = 0; k < Q; ++k) q[k] = int_mul_dense(xf, dense_split(c[k]));
+    } else if (MODE == VAL_ZEROS) {
+      const IntFactor xf = int_split(x);
+#pragma unroll
+      for (int k = 0; k < Q; ++k) q[k] = int_mul(xf, int_split(c[k]));
+    } else {
+#pragma unroll
+      for (int k = 0; k < Q; ++k) q[k] = __dmul_rn(x, c[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+      acc[k] = __dadd_rn(acc[k], q[k]);
+      c[k] = cn[k];
+    }
+    x = xn;
+  }
+}
+
+// One site for the CTA's points: w = v * T[:, i, :].  Returns the largest class
+// of the values written by this thread.
+template <int MODE>
+__device__ __forceinline__ int site_step(const tci_core_ref& c, const uint8_t* __restrict__ pts, int L, int s, int np,
+                                         int P, const double* v, double* w) {
+  int cls = VAL_DENSE;
+  const int nq = (c.r1 + 3) >> 2;
+  for (int e = threadIdx.x; e < P * nq; e += NT) {
+    const int p = e % P, q0 = (e / P) * 4;  // P is a power of two
+    if (p >= np) continue;
+    const int i = pts[(size_t)p * L + s];
+    const size_t stride = (size_t)c.r0 * c.d;
+    const double* col = c.p + (size_t)c.r0 * i + stride * q0;
+    if (q0 + 4 <= c.r1) {
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      row_times_cols<MODE, 4>(v + p, P, col, stride, c.r0, acc);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        w[(size_t)(q0 + k) * P + p] = acc[k];
+        cls = max(cls, val_class(acc[k]));
+      }
+    } else {
+      for (int q = q0; q < c.r1; ++q) {
+        double acc[1] = {0.0};
+        row_times_cols<MODE, 1>(v + p, P, col + stride * (q - q0), stride, c.r0, acc);
+        w[(size_t)q * P + p] = acc[0];
+        cls = max(cls, val_class(acc[0]));
+      }
+    }
+  }
+  return cls;
+}
+
+__global__ void __launch_bounds__(NT) tt_eval_kernel(const tci_core_ref* __restrict__ cores, const int* __restrict__ cls,
+                                                     int L, int rmax, int P, const uint8_t* __restrict__ pts,
+                                                     int64_t np, double* __restrict__ out) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int vcls[2];
+  for (int64_t base = (int64_t)blockIdx.x * P; base < np; base += (int64_t)gridDim.x * P) {
+    const int n = (int)min((int64_t)P, np - base);
+    const uint8_t* my = pts + base * L;
+    double* v = smem;
+    double* w = smem + (size_t)rmax * P;
+    for (int p = threadIdx.x; p < P; p += NT) v[p] = 1.0;
+    if (threadIdx.x == 0) {
+      vcls[0] = VAL_ZEROS;  // 1 is not dense
+      vcls[1] = VAL_DENSE;
+    }
+    __syncthreads();
+    for (int s = 0; s < L; ++s) {
+      const tci_core_ref c = cores[s];
+      const int mode = max(cls[s], vcls[s & 1]);
+      int k;
+      if (mode == VAL_DENSE) k = site_step<VAL_DENSE>(c, my, L, s, n, P, v, w);
+      else if (mode == VAL_ZEROS) k = site_step<VAL_ZEROS>(c, my, L, s, n, P, v, w);
+      else k = site_step<VAL_UNSAFE>(c, my, L, s, n, P, v, w);
+      if (k) atomicMax(&vcls[(s + 1) & 1], k);
+      __syncthreads();
+      if (threadIdx.x == 0) vcls[s & 1] = VAL_DENSE;  // read by all; set again after the next barrier's step
+      __syncthreads();
+      double* t = v;
+      v = w;
+      w = t;
+    }
+    for (int p = threadIdx.x; p < n; p += NT) out[base + p] = v[p];
+    __syncthreads();
+  }
+}
+
+}  // namespace
+
+// Largest bond the kernel's shared memory takes.
+int tci_tt_eval_max_bond() { return 225 * 1024 / 16; }
+
+// cores: L records on the device, cls: L words of scratch, pts: np x L local
+// indices, rmax: the largest bond.
+cudaError_t tci_tt_eval_launch(const tci_core_ref* cores, int* cls, int L, int rmax, const uint8_t* pts, int64_t np,
+                               double* out, int num_sms, cudaStream_t st) {
+  if (np <= 0) return cudaSuccess;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(tt_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+  if (attr != cudaSuccess) return attr;
+  cudaError_t e = cudaMemsetAsync(cls, 0, (size_t)L * sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  core_class_kernel<<<dim3(L, 4), 256, 0, st>>>(cores, cls);
+  // Points per CTA: as many as shared memory takes, up to 256, but no more than
+  // leaves every SM a block.
+  const size_t per = (size_t)rmax * 2 * sizeof(double);
+  int P = 256;
+  while (P > 1 && (size_t)P * per > 225 * 1024) P >>= 1;
+  while (P > 1 && (np + P - 1) / P < num_sms) P >>= 1;
+  const int64_t blocks = (np + P - 1) / P;
+  tt_eval_kernel<<<(unsigned)std::min<int64_t>(blocks, 8 * (int64_t)num_sms), NT, (size_t)P * per, st>>>(
+      cores, cls, L, rmax, P, pts, np, out);
+  return cudaGetLastError();
+}
