@@ -22,6 +22,7 @@
 // first element in column-major order of the physically permuted matrix
 // (matrixlu.jl:16-31).  The comparison of v*v is skipped for elements whose |v|
 // is more than 16 ulps below the running maximum, where v*v is provably smaller.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -2527,6 +2528,392 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
   }
 }
 
+// ------------------------------------------------------------ cluster rrLU
+// One rank-revealing LU on a thread-block cluster: the matrix lives in the
+// shared memory of the cluster's CTAs (a pr x pc grid, CTA (p, q) owns row block
+// p x column block q), and nothing of it goes through L2 between the fill and
+// the factors.  As in the multi-CTA kernel above, rows and columns stay where
+// they are: logical positions are tracked as permutations, the argmax keys are
+// logical, and the stored factors are scaled when they are written out, so
+// pivots and factors are bit-identical to rrlu_loop's.
+// Per pivot: each CTA reduces its block's argmax and writes it into every CTA's
+// shared memory; one cluster barrier; every warp reduces the CTAs' winners and
+// takes the decision itself; x and y come from the owners' shared memory (the
+// pivot row and column have left the trailing block there, so they are stable);
+// one CTA barrier; the rank-1 update of the block's active part.
+// Bound by that chain (about 5 thousand cycles a pivot: block argmax and
+// exchange 1.7, decision 0.7, x and y 1.4, one tile 1.6 thousand) until the
+// update outgrows it.  381 x 517 to rank 140 on 16 CTAs: 1.03 ms; on one CTA,
+// from L2, 14.1 ms.
+namespace cg = cooperative_groups;
+constexpr int CL_NT = 512;
+constexpr int CL_NW = CL_NT / 32;
+constexpr int CL_MAX = 16;  // CTAs of a cluster at most
+
+struct ClusterCtl {
+  unsigned long long red_a[CL_NW], red_b[CL_NW];
+  unsigned red_k[CL_NW], red_p[CL_NW];
+  double red_v[CL_NW];
+  BigPartial parts[2][CL_MAX];
+  int factors[2];
+  int nr, nc;  // active rows and columns of the block
+  int bad[CL_MAX];
+};
+
+struct ClusterJob {
+  int m, n, kmax, leftorth;
+  int pr, pc, mb, nb;  // CTA grid and block sizes
+  int nres;            // columns of a block held in shared memory; the rest, if any, in `spill`
+  double* spill;       // ncta x mb x (nb - nres) doubles of device scratch
+  double reltol, abstol;
+  double* pivs;        // kmax signed pivots (device scratch)
+  double* fact;        // the factored m x n matrix, or null
+  int *rowperm, *colperm;  // full permutations (m, n)
+  double* diag;        // |pivots| (kmax), or null
+};
+struct ClusterResult {
+  int K, nan;  // nan: valid in CTA 0
+  double err;
+};
+
+// Column u of CTA `rank`'s block: in its shared memory (blk), or in the spill.
+template <bool SPILL>
+struct ClusterBlock {
+  double* blk;
+  double* spill;
+  int mb, nb, nres;
+  __device__ __forceinline__ double* col(int u, int rank) const {
+    if (SPILL && u >= nres) return spill + ((size_t)rank * (nb - nres) + (u - nres)) * mb;
+    return blk + u * mb;
+  }
+  // entry (t, u) of another CTA's block; its spilled columns come from L2
+  __device__ __forceinline__ double remote(const cg::cluster_group& cl, int t, int u, int rank) const {
+    if (SPILL && u >= nres) return __ldcg(col(u, rank) + t);
+    return cl.map_shared_rank(blk, rank)[t + u * mb];
+  }
+};
+
+// Shared memory of one CTA: the block, x and y, the maps (16-bit: logical ->
+// physical for all rows and columns; per block row and column its logical
+// position, the active list and the slot in it).
+__host__ __device__ inline size_t cluster_smem(int m, int n, int mb, int nb, int nres) {
+  return ((size_t)mb * nres + mb + nb) * 8 + ((size_t)m + n) * 2 + ((size_t)mb + nb) * 6 + 64;
+}
+
+// This CTA's partial to every CTA of the cluster, then the cluster barrier.
+__device__ __forceinline__ void cluster_exchange(const BigTrack& t, ClusterCtl& ctl, int par, const cg::cluster_group& cl) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t a = t.A, b = t.B;
+  uint32_t k = t.k, ph = t.ph;
+  double v = t.v;
+  warp_track5(a, k, ph, b, v);
+  if (lane == 0) {
+    ctl.red_a[warp] = a;
+    ctl.red_b[warp] = b;
+    ctl.red_k[warp] = k;
+    ctl.red_p[warp] = ph;
+    ctl.red_v[warp] = v;
+  }
+  __syncthreads();
+  // The CTA barrier orders the other warps' writes before warp 0's release, so
+  // only warp 0 pays for one (790 cycles a pivot when every warp did).
+  if (warp == 0) {
+    a = lane < CL_NW ? ctl.red_a[lane] : 0ULL;
+    b = lane < CL_NW ? ctl.red_b[lane] : 0ULL;
+    k = lane < CL_NW ? ctl.red_k[lane] : 0xffffffffu;
+    ph = lane < CL_NW ? ctl.red_p[lane] : 0u;
+    v = lane < CL_NW ? ctl.red_v[lane] : 0.0;
+    warp_track5(a, k, ph, b, v);
+    if (lane < (int)cl.num_blocks()) {
+      BigPartial* o = cl.map_shared_rank(&ctl.parts[par][cl.block_rank()], lane);
+      o->A = a;
+      o->B = b;
+      o->k = k;
+      o->ph = ph;
+      o->v = v;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  } else {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The winner over the CTAs, to every lane of every warp.
+__device__ __forceinline__ BigTrack cluster_winner(const ClusterCtl& ctl, int par, int ncta) {
+  const int lane = threadIdx.x & 31;
+  BigTrack g;
+  g.init();
+  if (lane < ncta) {
+    const BigPartial& q = ctl.parts[par][lane];
+    g.A = q.A;
+    g.B = q.B;
+    g.k = q.k;
+    g.ph = q.ph;
+    g.v = q.v;
+  }
+  warp_track5(g.A, g.k, g.ph, g.B, g.v);
+  return g;
+}
+
+template <int MODE, bool SPILL>
+__device__ __forceinline__ void cluster_update(const ClusterBlock<SPILL>& B, int rank, int r0, int c0, int nr, int nc, const double* xs,
+                                               const double* ys, const uint16_t* act_r, const uint16_t* act_c,
+                                               const uint16_t* pos_r, const uint16_t* pos_c, BigTrack& bt) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane & 7, lc = lane >> 3;
+  const int nti = (nr + 15) >> 4, ntj = (nc + 7) >> 3;
+  int tj = warp / nti, ti = warp - tj * nti;
+  const int dj = CL_NW / nti, di = CL_NW - dj * nti;
+  uint32_t top = 0;
+  while (tj < ntj) {
+    const int t0 = 16 * ti + lr, u0 = 8 * tj + lc;
+    const bool vi[2] = {t0 < nr, t0 + 8 < nr}, vj[2] = {u0 < nc, u0 + 4 < nc};
+    int ri[2], cj[2];
+    double v[2][2], xv[2], yv[2], q[2][2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      ri[a] = act_r[min(t0 + 8 * a, nr - 1)];
+      cj[a] = act_c[min(u0 + 4 * a, nc - 1)];
+      xv[a] = xs[ri[a]];
+      yv[a] = ys[cj[a]];
+    }
+    double* const p[2] = {B.col(cj[0], rank), B.col(cj[1], rank)};
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) v[a][b] = p[b][ri[a]];
+    tile_products<MODE>(xv, yv, q);
+    uint32_t h = 0;
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        v[a][b] = __dsub_rn(v[a][b], q[a][b]);
+        if (vi[a] && vj[b]) p[b][ri[a]] = v[a][b];
+        h = max(h, (uint32_t)__double2hiint(v[a][b]) & 0x7fffffffu);
+      }
+    if (__any_sync(FULL, h + 1 >= top)) {
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+          if (vi[a] && vj[b]) bt.push(v[a][b], pack_key(pos_r[ri[a]], pos_c[cj[b]]), pack_key(r0 + ri[a], c0 + cj[b]));
+      top = __reduce_max_sync(FULL, bt.A ? (uint32_t)((bt.A - 1) >> 32) : 0u);
+    }
+    ti += di;
+    tj += dj;
+    if (ti >= nti) {
+      ti -= nti;
+      tj += 1;
+    }
+  }
+}
+
+// The body, by every thread of every CTA of the cluster.  fill(i, j) gives the
+// matrix; `each` sees every value of this CTA's block once.
+template <bool SPILL, class Fill, class Each>
+__device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCtl& ctl, const Fill& fill,
+                                      const Each& each) {
+  const cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, ncta = P.pr * P.pc, rank = (int)cl.block_rank(), m = P.m, n = P.n;
+  const bool leftorth = P.leftorth != 0;
+  const int bp = rank / P.pc, bq = rank % P.pc, mb = P.mb, nb = P.nb;
+  const int r0 = bp * mb, c0 = bq * nb;
+  const int nrb = max(0, min(m, r0 + mb) - r0), ncb = max(0, min(n, c0 + nb) - c0);
+  double* blk = (double*)smem;  // column-major, leading dimension mb
+  const ClusterBlock<SPILL> B{blk, P.spill, mb, nb, P.nres};
+  double* xs = blk + (size_t)mb * P.nres;
+  double* ys = xs + mb;
+  uint16_t* stor_r = (uint16_t*)(ys + nb);
+  uint16_t* stor_c = stor_r + m;
+  uint16_t* pos_r = stor_c + n;
+  uint16_t* act_r = pos_r + mb;
+  uint16_t* slot_r = act_r + mb;
+  uint16_t* pos_c = slot_r + mb;
+  uint16_t* act_c = pos_c + nb;
+  uint16_t* slot_c = act_c + nb;
+  for (int i = tid; i < m; i += CL_NT) stor_r[i] = (uint16_t)i;
+  for (int j = tid; j < n; j += CL_NT) stor_c[j] = (uint16_t)j;
+  for (int t = tid; t < nrb; t += CL_NT) {
+    pos_r[t] = (uint16_t)(r0 + t);
+    act_r[t] = slot_r[t] = (uint16_t)t;
+  }
+  for (int u = tid; u < ncb; u += CL_NT) {
+    pos_c[u] = (uint16_t)(c0 + u);
+    act_c[u] = slot_c[u] = (uint16_t)u;
+  }
+  if (tid == 0) {
+    ctl.nr = nrb;
+    ctl.nc = ncb;
+    ctl.factors[0] = ctl.factors[1] = 0;
+  }
+  BigTrack bt;
+  bt.init();
+  if (nrb > 0 && ncb > 0) {
+    const int sq = CL_NT / nrb, sr = CL_NT - sq * nrb;
+    int u = tid / nrb, t = tid - u * nrb;
+#pragma unroll 4
+    for (int e = tid; e < nrb * ncb; e += CL_NT) {
+      const double v = fill(r0 + t, c0 + u);
+      B.col(u, rank)[t] = v;
+      each(v);
+      const uint32_t key = pack_key(r0 + t, c0 + u);
+      bt.push(v, key, key);
+      t += sr;
+      u += sq;
+      if (t >= nrb) {
+        t -= nrb;
+        u += 1;
+      }
+    }
+  }
+  PivotState S;
+  S.init(P.reltol, P.abstol);
+  int K = 0;
+  while (P.kmax > 0) {
+    // ---- the pivot: argmax of abs2 over the cluster's trailing blocks
+    const int par = K & 1;
+    cluster_exchange(bt, ctl, par, cl);
+    if (tid == 0 && K > 0) ctl.factors[(K - 1) & 1] = 0;  // read by all before the barrier
+    BigTrack g = cluster_winner(ctl, par, ncta);
+    if (!track_decides(g.A, g.B)) {
+      if (g.A == 0) {  // every element NaN: the scan keeps its start
+        g.k = (uint32_t)((K << 16) | K);
+        g.ph = pack_key(stor_r[K], stor_c[K]);
+        const int pi = stor_r[K], pj = stor_c[K];
+        g.v = B.remote(cl, pi % mb, pj % nb, (pi / mb) * P.pc + pj / nb);
+      } else {  // squares of the elements near the maximum
+        const int nr = ctl.nr, nc = ctl.nc;
+        BigTrack et;
+        et.init();
+        for (int e = tid; e < nr * nc; e += CL_NT) {
+          const int i = act_r[e % nr], j = act_c[e / nr];
+          const double v = B.col(j, rank)[i];
+          if (near_max(abs_bits(v), g.A - 1)) {
+            const uint32_t key = pack_key(pos_r[i], pos_c[j]);
+            const uint64_t q = (uint64_t)__double_as_longlong(__dmul_rn(v, v)) + 1;
+            if (q > et.A || (q == et.A && key < et.k)) {
+              et.A = q;
+              et.k = key;
+              et.ph = pack_key(r0 + i, c0 + j);
+              et.v = v;
+            }
+          }
+        }
+        cl.sync();  // everyone has read the partials
+        cluster_exchange(et, ctl, par, cl);
+        g = cluster_winner(ctl, par, ncta);
+      }
+    }
+    if (S.decide(g.v, K, P.reltol, P.abstol)) break;
+    const int rl = (int)(g.k & 0xffffu), cc = (int)(g.k >> 16), R = (int)(g.ph & 0xffffu), C = (int)(g.ph >> 16);
+    if (tid == CL_NT - 32) {  // swaprow!(K, rl) on the maps; the pivot row leaves its block's active set
+      const int sr = stor_r[K];
+      stor_r[K] = (uint16_t)R;
+      stor_r[rl] = (uint16_t)sr;
+      if (sr >= r0 && sr < r0 + nrb) pos_r[sr - r0] = (uint16_t)rl;
+      if (R >= r0 && R < r0 + nrb) {
+        pos_r[R - r0] = (uint16_t)K;
+        const int s = slot_r[R - r0], last = act_r[ctl.nr - 1];
+        act_r[s] = (uint16_t)last;
+        slot_r[last] = (uint16_t)s;
+        ctl.nr -= 1;
+      }
+    } else if (tid == CL_NT - 64) {  // swapcol!(K, cc)
+      const int sc = stor_c[K];
+      stor_c[K] = (uint16_t)C;
+      stor_c[cc] = (uint16_t)sc;
+      if (sc >= c0 && sc < c0 + ncb) pos_c[sc - c0] = (uint16_t)cc;
+      if (C >= c0 && C < c0 + ncb) {
+        pos_c[C - c0] = (uint16_t)K;
+        const int s = slot_c[C - c0], last = act_c[ctl.nc - 1];
+        act_c[s] = (uint16_t)last;
+        slot_c[last] = (uint16_t)s;
+        ctl.nc -= 1;
+      }
+    } else if (tid == CL_NT - 96 && rank == 0) {
+      P.pivs[K] = g.v;
+      if (P.diag) P.diag[K] = __longlong_as_double((long long)abs_bits(g.v));
+    }
+    ++K;
+    if (K == P.kmax) break;  // the trailing update after the last pivot is not observable
+    // ---- x (pivot column) and y (pivot row) for the block, by physical place
+    JoinFlags fl{false, 0};
+    {
+      const int xo = bp * P.pc + C / nb, yo = (R / mb) * P.pc + bq;  // owners
+      auto entry = [&](int t) {
+        return t < nrb ? B.remote(cl, t, C % nb, xo) : B.remote(cl, R % mb, t - nrb, yo);
+      };
+      double v = tid < nrb + ncb ? entry(tid) : 0.0;  // under way during the division set-up
+      const PivotDivisor D(g.v);
+      for (int t = tid; t < nrb + ncb; t += CL_NT) {
+        const bool isx = t < nrb;
+        if (t != tid) v = entry(t);
+        if (isx == leftorth) v = D.quo(v);
+        fl.join(v);
+        if (isx) xs[t] = v;
+        else ys[t - nrb] = v;
+      }
+    }
+    if (fl.factors) atomicOr(&ctl.factors[(K - 1) & 1], fl.factors);
+    __syncthreads();
+    const int mode = min(ctl.factors[(K - 1) & 1], (int)PROD_FP64);
+    bt.init();
+    const int nr = ctl.nr, nc = ctl.nc;
+    if (nr > 0 && nc > 0) {
+      if (mode == PROD_DENSE)
+        cluster_update<PROD_DENSE>(B, rank, r0, c0, nr, nc, xs, ys, act_r, act_c, pos_r, pos_c, bt);
+      else if (mode == PROD_MIXED)
+        cluster_update<PROD_MIXED>(B, rank, r0, c0, nr, nc, xs, ys, act_r, act_c, pos_r, pos_c, bt);
+      else
+        cluster_update<PROD_FP64>(B, rank, r0, c0, nr, nc, xs, ys, act_r, act_c, pos_r, pos_c, bt);
+    }
+  }
+  // ---- permutations, and the factors in logical order with the deferred
+  // scaling of addpivot! and the NaN check of L and U (matrixlu.jl:162-169)
+  cl.sync();  // the maps and every pivot value are in place; no CTA reads another's block any more
+  int bad = 0;
+  for (int u = tid >> 5; u < ncb; u += CL_NW) {
+    const int lc = pos_c[u];
+    const PivotDivisor D(leftorth && lc < K ? __ldcg(&P.pivs[lc]) : 1.0);
+    for (int t = tid & 31; t < nrb; t += 32) {
+      const int lr = pos_r[t];
+      double v = B.col(u, rank)[t];
+      if (leftorth && lc < K && lr > lc) v = D.quo(v);
+      if (!leftorth && lr < K && lc > lr) v = PivotDivisor(__ldcg(&P.pivs[lr])).quo(v);
+      if ((lc < K && lr >= lc) || (lr < K && lr <= lc)) bad |= is_nan_bits(v) ? 1 : 0;
+      if (P.fact) P.fact[lr + (size_t)lc * m] = v;
+    }
+  }
+  bad = __syncthreads_or(bad);
+  if (tid == 0) *cl.map_shared_rank(&ctl.bad[rank], 0) = bad;
+  if (rank == 0) {
+    for (int i = tid; i < m; i += CL_NT) P.rowperm[i] = stor_r[i];
+    for (int j = tid; j < n; j += CL_NT) P.colperm[j] = stor_c[j];
+  }
+  cl.sync();
+  ClusterResult r;
+  r.K = K;
+  r.nan = 0;
+  if (rank == 0)
+    for (int t = 0; t < ncta; ++t) r.nan |= ctl.bad[t];
+  r.err = K >= min(m, n) ? 0.0 : __longlong_as_double((long long)S.err);
+  return r;
+}
+
+// CTA grid of a cluster of `ncta` (a power of two) for an m x n matrix: the
+// smallest block perimeter (x and y exchanged per pivot).
+struct ClusterGrid {
+  int pr, pc, mb, nb;
+};
+inline ClusterGrid cluster_grid(int m, int n, int ncta) {
+  ClusterGrid best{1, ncta, m, (n + ncta - 1) / ncta};
+  for (int pr = 1; pr <= ncta; pr *= 2) {
+    const int pc = ncta / pr, mb = (m + pr - 1) / pr, nb = (n + pc - 1) / pc;
+    if (mb + nb < best.mb + best.nb) best = ClusterGrid{pr, pc, mb, nb};
+  }
+  return best;
+}
+
 }  // namespace
 
 // Shared-memory budget of one CTA of the step kernel.
@@ -2707,12 +3094,35 @@ namespace {
 
 constexpr int64_t NOALLOC_MAX_ELEMS = (int64_t)1 << 19;  // m * n
 constexpr int64_t NOALLOC_MAX_DIM = 16384;               // m and n
+constexpr int64_t NOALLOC_CLUSTER_ELEMS = 2500;          // from this size on a cluster
+constexpr size_t CL_SMEM = 224 * 1024;                   // dynamic shared memory of a cluster's CTA at most
 // working matrix | factors + full permutations | result record
 constexpr int64_t NOALLOC_FACT_DOUBLES = NOALLOC_MAX_ELEMS + NOALLOC_MAX_DIM;
 constexpr int64_t NOALLOC_RES_DOUBLES = 16 + 2 * NOALLOC_MAX_DIM;
 constexpr int64_t NOALLOC_SCRATCH_DOUBLES = NOALLOC_MAX_ELEMS + NOALLOC_FACT_DOUBLES + NOALLOC_RES_DOUBLES;
 
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_SCRATCH_DOUBLES];
+
+// The caller's output buffers.
+struct NoallocOut {
+  int32_t *rowperm, *colperm, *npivot;
+  double* error;
+  int32_t* status;
+};
+template <bool SPILL>
+__global__ void __launch_bounds__(CL_NT, 1) rrlu_noalloc_cluster_kernel(const double* __restrict__ ain, ClusterJob P,
+                                                                        NoallocOut O) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ ClusterCtl ctl;
+  const int m = P.m;
+  const ClusterResult r = cluster_rrlu<SPILL>(
+      P, smem, ctl, [&](int i, int j) { return __ldcs(ain + i + (size_t)j * m); }, [](double) {});
+  if (cg::this_cluster().block_rank() == 0 && threadIdx.x == 0) {
+    *O.npivot = r.K;
+    *O.error = r.err;
+    *O.status = r.nan ? TCI_ERR_NAN : 0;
+  }
+}
 
 __global__ void __launch_bounds__(NT, TCI_CTAS_PER_SM) rrlu_noalloc_kernel(const tci_task T, char* resb) {
   extern __shared__ __align__(16) char smem[];
@@ -2740,8 +3150,42 @@ __global__ void rrlu_noalloc_epilogue(const double* fact, const char* resb, int 
   }
 }
 
+void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int ncta, size_t smem, cudaStream_t stream) {
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)ncta;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)ncta);
+  cfg.blockDim = dim3(CL_NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+
+// CTAs of the cluster for an m x n matrix on a device whose clusters hold at
+// most `most`; 0: one CTA of the step kernel.  A pivot costs some 5 thousand
+// cycles on a cluster beside a large update, some 3 thousand on one CTA (swaps
+// and argmax); full-rank factorizations cross at about 50 x 50: 32 x 32 takes
+// 97 us on 8 CTAs and about 75 on one, 64 x 64 to rank 32 101 and 115, 104 x 104
+// to rank 52 164 and 275, 160 x 160 to rank 80 274 and 1126 (from L2), 381 x 517
+// to rank 140 1030 and 14100.
+// *nres: the columns of a block that shared memory takes; past the fixed
+// array's size nothing remains to spill to.
+int noalloc_cluster(int64_t m, int64_t n, int most, int* nres) {
+  if (m * n < NOALLOC_CLUSTER_ELEMS) return 0;
+  for (int c = m * n < NOALLOC_CLUSTER_ELEMS * 4 ? 8 : 16; c <= most; c *= 2) {
+    const ClusterGrid g = cluster_grid((int)m, (int)n, c);
+    const size_t fixed = cluster_smem((int)m, (int)n, g.mb, g.nb, 0);
+    if (fixed >= CL_SMEM) continue;
+    *nres = (int)std::min<size_t>((size_t)g.nb, (CL_SMEM - fixed) / ((size_t)g.mb * 8));
+    if (*nres == g.nb || (c == most && (int64_t)c * g.mb * (g.nb - *nres) <= NOALLOC_MAX_ELEMS)) return c;
+  }
+  return 0;
+}
+
 struct NoallocDevice {
   bool ready = false;
+  int most = 0;  // CTAs of the largest cluster the device runs (0: none)
   double* scratch = nullptr;  // device address of g_noalloc_scratch
 };
 
@@ -2751,7 +3195,7 @@ struct NoallocDevice {
 // See include/tci_gb300.h.  The first call on a device resolves the device
 // address of the scratch array (cudaGetSymbolAddress) and raises the kernel's
 // shared-memory limit, with that device current; make that first call before
-// any stream capture.  Later calls only launch two kernels on `stream_u`.  The
+// any stream capture.  Later calls only launch one or two kernels on `stream_u`.  The
 // address is cached per device for the life of the process, so a device reset
 // (cudaDeviceReset) after the first call is not supported.
 extern "C" int tci_rrlu_noalloc(const double* A_dev, int64_t m, int64_t n, int64_t maxrank, double reltol,
@@ -2795,6 +3239,21 @@ extern "C" int tci_rrlu_noalloc(const double* A_dev, int64_t m, int64_t n, int64
       if (ce == cudaSuccess)
         ce = cudaFuncSetAttribute(rrlu_noalloc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)tci_step_smem_bytes());
+      for (auto k : {rrlu_noalloc_cluster_kernel<false>, rrlu_noalloc_cluster_kernel<true>}) {
+        if (ce == cudaSuccess)
+          ce = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL_SMEM);
+        if (ce == cudaSuccess) ce = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      }
+      for (int c = CL_MAX; ce == cudaSuccess && c >= 8 && D.most == 0; c /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        cluster_config(cfg, at, c, CL_SMEM, nullptr);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, rrlu_noalloc_cluster_kernel<true>, &cfg) == cudaSuccess && fit > 0)
+          D.most = c;
+        else
+          (void)cudaGetLastError();
+      }
       if (ce != cudaSuccess) {
         tci::set_error(TCI_ERR_CUDA,std::string("tci_rrlu_noalloc set-up: ") + cudaGetErrorString(ce));
         return TCI_ERR_CUDA;
@@ -2823,12 +3282,46 @@ extern "C" int tci_rrlu_noalloc(const double* A_dev, int64_t m, int64_t n, int64
   T.ain = A_dev;
   T.core_out = fact;
   T.res = 0;
+  cudaStream_t stream = (cudaStream_t)stream_u;
+  int nres = 0;
+  if (const int c = noalloc_cluster(m, n, D.most, &nres)) {
+    const ClusterGrid g = cluster_grid((int)m, (int)n, c);
+    ClusterJob P;
+    P.m = (int)m;
+    P.n = (int)n;
+    P.kmax = (int)kmax;
+    P.leftorth = T.leftorth;
+    P.pr = g.pr;
+    P.pc = g.pc;
+    P.mb = g.mb;
+    P.nb = g.nb;
+    P.reltol = reltol;
+    P.abstol = abstol;
+    P.nres = nres;
+    P.spill = work;
+    P.pivs = fact;
+    P.fact = factors_dev;
+    P.rowperm = rowperm_dev;
+    P.colperm = colperm_dev;
+    P.diag = nullptr;
+    const NoallocOut O{rowperm_dev, colperm_dev, npivot_dev, error_dev, status_dev};
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cluster_config(cfg, at, c, cluster_smem((int)m, (int)n, g.mb, g.nb, nres), stream);
+    ce = cudaLaunchKernelEx(&cfg, nres < g.nb ? rrlu_noalloc_cluster_kernel<true> : rrlu_noalloc_cluster_kernel<false>,
+                            A_dev, P, O);
+    if (ce == cudaSuccess) ce = cudaGetLastError();
+    if (ce != cudaSuccess) {
+      tci::set_error(TCI_ERR_CUDA, std::string("tci_rrlu_noalloc: ") + cudaGetErrorString(ce));
+      return TCI_ERR_CUDA;
+    }
+    return 0;
+  }
   const size_t smem = tci_step_smem_bytes();
   auto a16 = [](size_t x) { return (x + 15) / 16 * 16; };
   const size_t perms = a16((size_t)m * 4) + a16((size_t)n * 4);
   T.smem_mode = a16((size_t)m * n * 8) + perms <= smem ? 1 : 0;
   T.work = T.smem_mode ? nullptr : work;
-  cudaStream_t stream = (cudaStream_t)stream_u;
   rrlu_noalloc_kernel<<<1, NT, smem, stream>>>(T, resb);
   rrlu_noalloc_epilogue<<<64, 256, 0, stream>>>(fact, resb, (int)m, (int)n, rowperm_dev, colperm_dev, npivot_dev,
                                                 error_dev, status_dev, factors_dev);
