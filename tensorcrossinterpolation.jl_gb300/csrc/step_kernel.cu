@@ -2185,20 +2185,23 @@ struct BigArgs {
   BigBar* bar;
   int m, n, kmax, kcap, leftorth;
   int pr, pc, mb, nb;     // CTA grid and block sizes
+  int nres;               // columns of a block held in shared memory as well
   double reltol, abstol;
 };
 
 // The rank-1 update of a CTA's block: the active rows and columns (lists of
 // local indices) of A at (r0, c0), x and y by list position, the logical
 // positions for the argmax keys.  As rank1_tiles, but a warp takes 32 x 4 tiles
-// with one row and four columns per lane: the block is read from L2 / L1, where
-// 32 rows of a column are two lines (8 x 4 lanes touched four, 14.6 ms instead
-// of 11.7 for a 2048 x 2048 matrix to rank 512).
+// with one row and four columns per lane, whole lines of A.  The first nres
+// columns are also kept in shared memory (blk, leading dimension mb) and read
+// from there; every result is written to A too, where the other CTAs read the
+// pivot row and column.  A 2048 x 2048 matrix to rank 512: 9.0 ms, 1.06 cycles
+// per element and SM in here; 10.5 ms and 1.3 when the block was read from L2.
 struct BigBlock {
-  double* A;
-  int m, r0, c0, nr, nc;
+  double *A, *blk;
+  int m, mb, nres, r0, c0, nr, nc;
   const double *xs, *ys;
-  const int *act_r, *act_c, *pos_r, *pos_c;
+  const uint16_t *act_r, *act_c, *pos_r, *pos_c;
   bool rev;
 };
 template <int MODE>
@@ -2212,33 +2215,35 @@ __device__ __forceinline__ void big_update(const BigBlock B, BigTrack& bt) {
     const int t = 32 * ti + lane, u0 = 4 * (B.rev ? ntj - 1 - tj : tj);
     const bool vi = t < B.nr;
     const int tt = min(t, B.nr - 1);
-    const int ri = B.r0 + B.act_r[tt];
+    const int ri = B.act_r[tt];
     double v[4], xv[1], yv[4], q[1][4];
-    double* p[4];
     int cj[4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int uu = min(u0 + b, B.nc - 1);
-      cj[b] = B.c0 + B.act_c[uu];
+      cj[b] = B.act_c[uu];
       yv[b] = B.ys[uu];
-      p[b] = B.A + (size_t)cj[b] * B.m + ri;
     }
+    double* const g = B.A + B.r0 + ri + (size_t)B.c0 * B.m;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) v[b] = *p[b];
+    for (int b = 0; b < 4; ++b) v[b] = cj[b] < B.nres ? B.blk[ri + cj[b] * B.mb] : g[(size_t)cj[b] * B.m];
     xv[0] = B.xs[tt];
     tile_products<MODE>(xv, yv, q);
     uint32_t h = 0;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       v[b] = __dsub_rn(v[b], q[0][b]);
-      if (vi && u0 + b < B.nc) *p[b] = v[b];
+      if (vi && u0 + b < B.nc) {
+        if (cj[b] < B.nres) B.blk[ri + cj[b] * B.mb] = v[b];
+        g[(size_t)cj[b] * B.m] = v[b];
+      }
       h = max(h, (uint32_t)__double2hiint(v[b]) & 0x7fffffffu);
     }
     if (__any_sync(FULL, h + 1 >= top)) {
       const int lr = B.pos_r[ri];
 #pragma unroll
       for (int b = 0; b < 4; ++b)
-        if (vi && u0 + b < B.nc) bt.push(v[b], pack_key(lr, B.pos_c[cj[b]]), pack_key(ri, cj[b]));
+        if (vi && u0 + b < B.nc) bt.push(v[b], pack_key(lr, B.pos_c[cj[b]]), pack_key(B.r0 + ri, B.c0 + cj[b]));
       top = __reduce_max_sync(FULL, bt.A ? (uint32_t)((bt.A - 1) >> 32) : 0u);
     }
     ti += di;
@@ -2258,21 +2263,28 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
   const int r0 = (b / P.pc) * P.mb, c0 = (b % P.pc) * P.nb;
   const int r1 = min(m, r0 + P.mb), c1 = min(n, c0 + P.nb);
   const int nrb = max(0, r1 - r0), ncb = max(0, c1 - c0);  // block extent
-  double* xs = (double*)smem;          // x of the active rows (mb)
+  double* blk = (double*)smem;         // the block's first nres columns (mb x nres)
+  double* xs = blk + (size_t)P.mb * P.nres;  // x of the active rows (mb)
   double* ys = xs + P.mb;              // y of the active columns (nb)
-  int* pos_r = (int*)(ys + P.nb);      // physical row -> logical (m)
-  int* stor_r = pos_r + m;             // logical row -> physical (m)
-  int* pos_c = stor_r + m;             // (n)
-  int* stor_c = pos_c + n;             // (n)
-  int* act_r = stor_c + n;             // active rows of the block, and the slot of each (mb each)
-  int* slot_r = act_r + P.mb;
-  int* act_c = slot_r + P.mb;          // (nb each)
-  int* slot_c = act_c + P.nb;
+  uint16_t* stor_r = (uint16_t*)(ys + P.nb);  // logical row -> physical (m)
+  uint16_t* stor_c = stor_r + m;              // (n)
+  uint16_t* pos_r = stor_c + n;        // logical position of each block row, active rows, slot of each (mb each)
+  uint16_t* act_r = pos_r + P.mb;
+  uint16_t* slot_r = act_r + P.mb;
+  uint16_t* pos_c = slot_r + P.mb;     // (nb each)
+  uint16_t* act_c = pos_c + P.nb;
+  uint16_t* slot_c = act_c + P.nb;
   unsigned gen = 0;
-  for (int i = tid; i < m; i += BIG_NT) pos_r[i] = stor_r[i] = i;
-  for (int j = tid; j < n; j += BIG_NT) pos_c[j] = stor_c[j] = j;
-  for (int t = tid; t < nrb; t += BIG_NT) act_r[t] = slot_r[t] = t;  // local indices
-  for (int u = tid; u < ncb; u += BIG_NT) act_c[u] = slot_c[u] = u;
+  for (int i = tid; i < m; i += BIG_NT) stor_r[i] = (uint16_t)i;
+  for (int j = tid; j < n; j += BIG_NT) stor_c[j] = (uint16_t)j;
+  for (int t = tid; t < nrb; t += BIG_NT) {
+    pos_r[t] = (uint16_t)(r0 + t);
+    act_r[t] = slot_r[t] = (uint16_t)t;
+  }
+  for (int u = tid; u < ncb; u += BIG_NT) {
+    pos_c[u] = (uint16_t)(c0 + u);
+    act_c[u] = slot_c[u] = (uint16_t)u;
+  }
   PivotState S;  // thread 0's
   S.init(P.reltol, P.abstol);
   if (tid == 0) {
@@ -2290,6 +2302,7 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
       const int i = r0 + (int)(e % nrb), j = c0 + (int)(e / nrb);
       const double v = P.ain[i + (size_t)j * m];
       P.A[i + (size_t)j * m] = v;
+      if (j - c0 < P.nres) blk[i - r0 + (j - c0) * P.mb] = v;
       bt.push(v, pack_key(i, j), pack_key(i, j));
     }
   }
@@ -2320,26 +2333,26 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
       }
       // swaprow!(K, rl), swapcol!(K, cl) on the maps
       const int sr = stor_r[K];
-      stor_r[K] = R;
-      stor_r[rl] = sr;
-      pos_r[R] = K;
-      pos_r[sr] = rl;
+      stor_r[K] = (uint16_t)R;
+      stor_r[rl] = (uint16_t)sr;
+      if (sr >= r0 && sr < r1) pos_r[sr - r0] = (uint16_t)rl;
       const int sc = stor_c[K];
-      stor_c[K] = Cc;
-      stor_c[cl] = sc;
-      pos_c[Cc] = K;
-      pos_c[sc] = cl;
+      stor_c[K] = (uint16_t)Cc;
+      stor_c[cl] = (uint16_t)sc;
+      if (sc >= c0 && sc < c1) pos_c[sc - c0] = (uint16_t)cl;
       // the pivot row and column leave this block's active sets
       if (R >= r0 && R < r1) {
+        pos_r[R - r0] = (uint16_t)K;
         const int s = slot_r[R - r0], last = act_r[ctl.r - 1];
-        act_r[s] = last;
-        slot_r[last] = s;
+        act_r[s] = (uint16_t)last;
+        slot_r[last] = (uint16_t)s;
         ctl.r -= 1;
       }
       if (Cc >= c0 && Cc < c1) {
+        pos_c[Cc - c0] = (uint16_t)K;
         const int s = slot_c[Cc - c0], last = act_c[ctl.c - 1];
-        act_c[s] = last;
-        slot_c[last] = s;
+        act_c[s] = (uint16_t)last;
+        slot_c[last] = (uint16_t)s;
         ctl.c -= 1;
       }
     }
@@ -2390,7 +2403,7 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
         const int i = r0 + act_r[(int)(e % nr)], j = c0 + act_c[(int)(e / nr)];
         const double v = P.A[i + (size_t)j * m];
         if (near_max(abs_bits(v), Mstar)) {
-          const uint32_t key = pack_key(pos_r[i], pos_c[j]);
+          const uint32_t key = pack_key(pos_r[i - r0], pos_c[j - c0]);
           const uint64_t q = (uint64_t)__double_as_longlong(__dmul_rn(v, v)) + 1;
           if (q > ab.s || (q == ab.s && key < ab.key)) {
             ab.s = q;
@@ -2467,7 +2480,7 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
     // the last pass touched last is still in L1.
     bt.init();
     if (nr > 0 && nc > 0) {
-      const BigBlock B{P.A, m, r0, c0, nr, nc, xs, ys, act_r, act_c, pos_r, pos_c, (K & 1) != 0};
+      const BigBlock B{P.A, blk, m, P.mb, P.nres, r0, c0, nr, nc, xs, ys, act_r, act_c, pos_r, pos_c, (K & 1) != 0};
       if (mode == PROD_DENSE) big_update<PROD_DENSE>(B, bt);
       else if (mode == PROD_MIXED) big_update<PROD_MIXED>(B, bt);
       else big_update<PROD_FP64>(B, bt);
@@ -2489,10 +2502,10 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
     const long long tot = (long long)nrb * ncb;
     for (long long e = tid; e < tot; e += BIG_NT) {
       const int i = r0 + (int)(e % nrb), j = c0 + (int)(e / nrb);
-      const int lr = pos_r[i], lc = pos_c[j];
+      const int lr = pos_r[i - r0], lc = pos_c[j - c0];
       double v = P.A[i + (size_t)j * m];
-      if (leftorth && lc < K && lr > lc) v = __ddiv_rn(v, __ldcg(&P.pivs[lc]));
-      if (!leftorth && lr < K && lc > lr) v = __ddiv_rn(v, __ldcg(&P.pivs[lr]));
+      if (leftorth && lc < K && lr > lc) v = PivotDivisor(__ldcg(&P.pivs[lc])).quo(v);
+      if (!leftorth && lr < K && lc > lr) v = PivotDivisor(__ldcg(&P.pivs[lr])).quo(v);
       const bool inL = lc < K && lr >= lc;
       const bool inU = lr < K && lr <= lc;
       if ((inL || inU) && is_nan_bits(v)) bad = 1;
@@ -2941,9 +2954,9 @@ cudaError_t tci_step_configure() {
 }
 
 // Multi-CTA rrLU (rrlu_big_kernel).  The CTA grid: pr x pc <= G CTAs with the
-// largest count, then the most square blocks.  Shared memory per CTA: both
-// permutation maps (8 (m + n) bytes) and, per block row / column, x or y, the
-// active list and the slot map (16 bytes each).
+// largest count, then the most square blocks.  Shared memory per CTA: the
+// permutations and lists (16-bit), x and y, and as many columns of the block as
+// the rest takes.
 namespace {
 struct BigGrid {
   int pr, pc, mb, nb;
@@ -2971,7 +2984,7 @@ BigGrid big_grid(int64_t m, int64_t n, int G) {
 }  // namespace
 size_t tci_rrlu_big_smem(int64_t m, int64_t n, int G) {
   const BigGrid g = big_grid(m, n, G);
-  return (size_t)(8 * (m + n) + 16 * ((int64_t)g.mb + g.nb) + 64);
+  return (size_t)(2 * (m + n) + 14 * ((int64_t)g.mb + g.nb) + 64);
 }
 bool tci_rrlu_big_fits(int64_t m, int64_t n, int G) {
   return m >= 1 && n >= 1 && m <= 65535 && n <= 65535 && tci_rrlu_big_smem(m, n, G) <= tci_big_smem_limit();
@@ -3009,21 +3022,9 @@ cudaError_t tci_rrlu_big_launch(const double* ain, double* work, double* fact, c
   a.nb = g.nb;
   a.reltol = reltol;
   a.abstol = abstol;
-  // Most of the SM's on-chip memory as L1 (the CTA's block of the working matrix
-  // is re-read every pivot), but enough shared memory for the CTAs that share
-  // an SM: the carveout is what the occupancy of a cooperative launch is
-  // computed with.
-  const size_t smem = tci_rrlu_big_smem(m, n, grid);
-  const int nsm = std::max(1, grid / TCI_CTAS_PER_SM);
-  const int per_sm = (g.pr * g.pc + nsm - 1) / nsm;
-  const double need = (double)per_sm * (double)(smem + 3 * 1024) / (228.0 * 1024.0);
-  const int pct = std::min(100, std::max(25, (int)std::ceil(100.0 * need)));
-  static int carve = -1;
-  if (pct != carve) {
-    e = cudaFuncSetAttribute((const void*)rrlu_big_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-    if (e != cudaSuccess) return e;
-    carve = pct;
-  }
+  const size_t fixed = tci_rrlu_big_smem(m, n, grid);
+  a.nres = (int)std::min<size_t>((size_t)g.nb, (tci_big_smem_limit() - fixed) / ((size_t)g.mb * 8));
+  const size_t smem = fixed + (size_t)a.nres * g.mb * 8;
   void* args[] = {(void*)&a};
   return cudaLaunchCooperativeKernel((const void*)rrlu_big_kernel, dim3(g.pr * g.pc), dim3(BIG_NT), args, smem,
                                      stream);
