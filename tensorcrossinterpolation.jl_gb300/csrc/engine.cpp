@@ -847,14 +847,15 @@ ResidentQueue::~ResidentQueue() {
   if (slots) cudaFreeHost(slots);
 }
 
-int ResidentQueue::start(const tci_kernel_set* k) {
+int ResidentQueue::start(const tci_kernel_set* k, int clusters, int cluster_ctas) {
   std::lock_guard<std::mutex> lk(mu);
-  if (running) return k == ks ? 0 : fail(TCI_ERR_GENERIC, "resident kernel already running in another variant");
+  if (running) return k == ks && cluster == cluster_ctas ? 0 : fail(TCI_ERR_GENERIC, "resident kernel already running in another variant");
   ks = k;
-  grid = num_sms * ks->ctas_per_sm;
+  cluster = cluster_ctas;
+  grid = clusters > 0 ? clusters * cluster : num_sms * ks->ctas_per_sm;
   std::atomic_ref<int32_t>(qc->stop).store(0, std::memory_order_release);
   CUDA_TRY(cudaEventRecord(ev0, stream));
-  CUDA_TRY(ks->resident_launch(slots, mask, st_dev, qc, grid, wait_ns, stream));
+  CUDA_TRY(ks->resident_launch(slots, mask, st_dev, qc, grid, cluster, wait_ns, stream));
   CUDA_TRY(cudaEventRecord(ev1, stream));
   running = true;
   ++launches;
@@ -879,7 +880,7 @@ int ResidentQueue::ensure_alive() {
     return fail(TCI_ERR_TIMEOUT, "resident kernel: a wait for a task hit its limit");
   }
   CUDA_TRY(cudaEventRecord(ev0, stream));
-  CUDA_TRY(ks->resident_launch(slots, mask, st_dev, qc, grid, wait_ns, stream));
+  CUDA_TRY(ks->resident_launch(slots, mask, st_dev, qc, grid, cluster, wait_ns, stream));
   CUDA_TRY(cudaEventRecord(ev1, stream));
   ++launches;
   return 0;
@@ -931,6 +932,21 @@ void Engine::set_resident(ResidentQueue* q, BlockPool* host_pool, BlockPool* scr
   spool_ = scratch_pool;
   res_smem_ = q ? q->ks->resident_smem_bytes() : 0;
   res_threads_ = q ? q->ks->threads : 0;
+}
+
+// A lone RRLU task of a single solve from this many elements on runs on a
+// cluster beside the resident kernel (a launch, some 5 us, instead of a ring
+// ticket).  A 30-site quantics solve of rank 80 takes 143 ms without, and with
+// the line at 256 elements 44.5, at 1024 45.6, at 6000 50.3; a 40-site one of
+// rank 11 11.04, 10.81, 11.04, 11.04; an 8-site Lorentzian 4.51 and 3.0 at any.
+static constexpr int64_t COOP_ELEMS = 256;
+
+int Engine::cooperative_ctas(const Req& r, size_t batch) const {
+  const tci_task& t = r.t;
+  if (!coop_most_ || batch != 1 || inflight_tasks_ != 0 || t.kind != TCI_TASK_RRLU || t.post != TCI_POST_NONE ||
+      t.ain || r.ain_host || (int64_t)t.m * t.n < COOP_ELEMS)
+    return 0;
+  return tci_k256::tci_rrlu_cluster_ctas(t, coop_most_);
 }
 
 int Engine::submit() {
@@ -1009,6 +1025,25 @@ int Engine::submit() {
         f.dblocks.push_back(d);
         if (t.smem_mode != 1) t.work = d;
         if (lut) t.lut = d + we;
+      }
+      if (const int ncta = cooperative_ctas(r, batch.size())) {
+        double* pivs = (double*)spool_->alloc((size_t)std::max(t.maxrank, 1) * sizeof(double));
+        if (!pivs) {
+          rc = fail(TCI_ERR_OOM, "device scratch for a task");
+          break;
+        }
+        f.dblocks.push_back(pivs);
+        r.ticket = t.ticket = ++coop_seq_;
+        const cudaError_t ce = tci_k256::tci_rrlu_cluster_launch(t, ncta, pivs, stream_);
+        if (ce != cudaSuccess) {
+          rc = fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
+          break;
+        }
+        stats.launches += 1;
+        stats.h2d_bytes += (int64_t)o_res;
+        stats.d2h_bytes += (int64_t)r.res_bytes;
+        f.reqs.push_back(&r);
+        continue;
       }
       t.cost = task_cost(t);
       // small inputs are copied to shared memory in one parallel pass when the
@@ -1189,10 +1224,16 @@ static CoTask co_tasks(Engine& e, std::vector<Req*> reqs) {
 
 // A rank-revealing LU of a given matrix large enough to spread over every SM:
 // the multi-CTA kernel instead of one CTA working out of global memory.
+// Elements of a given matrix from which one CTA, then one cluster, is the slower
+// choice.  A cluster pays from about 50 x 50 on (tci_rrlu_noalloc's rule and
+// figures); the multi-CTA kernel's pivot costs 13 thousand cycles beside its
+// update against 5 on a cluster, but it has ten times the SMs: 381 x 517 to rank
+// 140 takes 1.03 ms on a cluster, 530 x 517 to rank 517 3.1 ms on every SM.
+static constexpr int64_t CLUSTER_ELEMS = 2500, BIG_ELEMS = (int64_t)1 << 18;
 static bool big_eligible(const Req& r, bool resident, int grid) {
   const tci_task& t = r.t;
   return !resident && t.kind == TCI_TASK_RRLU && (t.ain || r.ain_host) &&
-         (t.post == TCI_POST_FACTORS || t.post == TCI_POST_NONE) && (int64_t)t.m * t.n >= ((int64_t)1 << 18) &&
+         (t.post == TCI_POST_FACTORS || t.post == TCI_POST_NONE) && (int64_t)t.m * t.n >= BIG_ELEMS &&
          tci_rrlu_big_fits(t.m, t.n, grid);
 }
 
@@ -1247,8 +1288,59 @@ int Engine::run_big(Req& r) {
   return rc;
 }
 
+// One RRLU of a given matrix on a thread-block cluster.
+int Engine::run_cluster(Req& r, int ncta) {
+  tci_task& t = r.t;
+  const int64_t m = t.m, n = t.n;
+  const size_t rb = result_bytes(t), in_elems = r.ain_host ? (size_t)(m * n) : 0;
+  const size_t pivs = a16(rb) / 8, input = pivs + (size_t)std::max(t.maxrank, 1);
+  double* blk = alloc_core(input + in_elems);
+  if (!blk) return fail(TCI_ERR_OOM, "device memory for the rrLU");
+  t.res = (int64_t)(uintptr_t)blk;
+  t.ticket = 0;
+  cudaError_t ce = cudaSuccess;
+  if (r.ain_host) {
+    ce = cudaMemcpyAsync(blk + input, r.ain_host, in_elems * 8, cudaMemcpyHostToDevice, stream_);
+    t.ain = blk + input;
+  }
+  if (ce == cudaSuccess && timing) ce = cudaEventRecord(ev0_, stream_);
+  if (ce == cudaSuccess) ce = tci_k256::tci_rrlu_cluster_launch(t, ncta, blk + pivs, stream_);
+  if (ce == cudaSuccess && timing) ce = cudaEventRecord(ev1_, stream_);
+  big_res_.resize(rb);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(big_res_.data(), blk, rb, cudaMemcpyDeviceToHost, stream_);
+  const cudaError_t sync = cudaStreamSynchronize(stream_);
+  free_core(blk);
+  if (ce == cudaSuccess) ce = sync;
+  if (ce != cudaSuccess) return fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
+  if (timing) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ev0_, ev1_);
+    stats.kernel_ms += ms;
+  }
+  r.res = big_res_.data();
+  r.res_bytes = rb;
+  stats.launches += 1;
+  stats.tasks += 1;
+  stats.h2d_bytes += (int64_t)(in_elems * 8);
+  stats.d2h_bytes += (int64_t)rb;
+  for (int64_t k = 1; k < r.head()->npivot; ++k) stats.lu_updates += (m - k) * (n - k);
+  return 0;
+}
+
 int Engine::run_tasks(std::vector<Req*>& reqs) {
   if (fc_callback_depth()) return reentry();
+  if (reqs.size() == 1) {  // a given matrix below the multi-CTA kernel's range
+    Req& r = *reqs[0];
+    const tci_task& t = r.t;
+    if (!resident() && t.kind == TCI_TASK_RRLU && (t.ain || r.ain_host) &&
+        (t.post == TCI_POST_FACTORS || t.post == TCI_POST_NONE) && (int64_t)t.m * t.n >= CLUSTER_ELEMS &&
+        (int64_t)t.m * t.n < BIG_ELEMS) {
+      tci_task probe = t;
+      probe.ain = (const double*)1;  // given, wherever it is
+      if (const int ncta = tci_k256::tci_rrlu_cluster_ctas(probe, tci_k256::tci_rrlu_cluster_most(nullptr)))
+        return run_cluster(r, ncta);
+    }
+  }
   if (reqs.size() == 1 && big_eligible(*reqs[0], resident(), num_sms * tci_k256::kernels.ctas_per_sm))
     return run_big(*reqs[0]);
   CoTask t = co_tasks(*this, reqs);
@@ -1256,7 +1348,13 @@ int Engine::run_tasks(std::vector<Req*>& reqs) {
 }
 
 int Engine::run_resident(CoTask& t) {
-  int rc = att_rq_->start(&tci_k512::kernels);  // one solve: its tasks run one at a time
+  // One solve: its RRLU tasks run one at a time, the large ones on a cluster of
+  // SMs.  The resident kernel then takes four clusters' worth of SMs, for the
+  // small tasks and the sets of independent ones (site tensors, searches).
+  int clusters = 0;
+  const int most = tci_k256::tci_rrlu_cluster_most(&clusters);
+  coop_most_ = most >= 16 && clusters > 4 ? most : 0;
+  int rc = coop_most_ ? att_rq_->start(&tci_k512::kernels, 4, coop_most_) : att_rq_->start(&tci_k512::kernels);
   if (rc) return rc;
   set_resident(att_rq_, att_h_, att_s_);
   t.h.resume();
@@ -1292,6 +1390,8 @@ int Engine::run_resident(CoTask& t) {
     }
   }
   const int src = att_rq_->stop();
+  if (coop_most_ && has_flights()) cudaStreamSynchronize(stream_);  // after an error: no task may outlive its record
+  coop_most_ = 0;
   abandon();
   set_resident(nullptr, nullptr, nullptr);
   if (rc) return rc;

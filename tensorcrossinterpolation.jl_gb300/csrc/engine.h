@@ -166,7 +166,7 @@ class BlockPool {
 // The ring of the resident kernel, shared by the engines of a context.
 struct ResidentQueue {
   int device = 0;
-  int grid = 0, num_sms = 0;
+  int grid = 0, cluster = 0, num_sms = 0;
   const tci_kernel_set* ks = &tci_k256::kernels;  // the variant of the running (or last) launch
   uint32_t nslots = 0, mask = 0;
   tci_queue_slot* slots = nullptr;       // mapped pinned host memory
@@ -184,7 +184,9 @@ struct ResidentQueue {
   ~ResidentQueue();
   // launch the kernel unless it is running: the throughput variant (k256) for
   // batched and served solves, the latency variant (k512) for a single solve
-  int start(const tci_kernel_set* k);
+  // clusters > 0: that many clusters of `cluster` CTAs instead of every SM, with
+  // the rest of the device left to cluster kernels
+  int start(const tci_kernel_set* k, int clusters = 0, int cluster = 0);
   int ensure_alive(); // relaunch it if every CTA has left (idle limit)
   int stop();         // ask the CTAs to leave once the ring is drained; wait
   int publish(const tci_task& t, uint64_t& ticket);
@@ -287,6 +289,7 @@ class Engine {
   // rrLU of a given matrix runs on the multi-CTA kernel (run_big).
   int run_tasks(std::vector<Req*>& reqs);
   int run_big(Req& r);
+  int run_cluster(Req& r, int ncta);
   // evaluate(tt, points) for np packed 0-based points (np x L) of the solve's train.
   int eval_train(const Solve& s, const uint8_t* pts, int64_t np, double* out);
   // Copy many device arrays to one host buffer: gather on the device into a
@@ -323,6 +326,7 @@ class Engine {
     size_t first, count;
   };
   int ensure(size_t blob, size_t res, size_t work);
+  int cooperative_ctas(const Req& r, size_t batch) const;
   void account(const Req& r, int smem_mode);
   int device_ = 0;
   // resident mode
@@ -343,6 +347,10 @@ class Engine {
   size_t plan_limit_ = SIZE_MAX;  // TCI_PLAN_SMEM
   std::vector<Flight> flights_;
   size_t inflight_tasks_ = 0;  // tasks of flights_
+  // one solve at a time: its large RRLU tasks run on a thread-block cluster
+  // beside the resident kernel (0: none)
+  int coop_most_ = 0;
+  uint64_t coop_seq_ = 0;
   std::vector<char> big_res_;  // host copy of the last multi-CTA rrLU's result record
   cudaStream_t stream_ = nullptr;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;

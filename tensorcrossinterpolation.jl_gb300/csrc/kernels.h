@@ -24,7 +24,8 @@ struct tci_kernel_set {
                              int* counter_dev, int grid, double* cta_area, size_t cta_stride,
                              cudaStream_t stream);
   cudaError_t (*resident_launch)(tci_queue_slot* slots, uint32_t mask, tci_resident_state* st,
-                                 tci_queue_ctl* qc, int grid, unsigned long long wait_ns, cudaStream_t stream);
+                                 tci_queue_ctl* qc, int grid, int cluster, unsigned long long wait_ns,
+                                 cudaStream_t stream);
 };
 
 namespace tci_k256 {
@@ -35,6 +36,10 @@ size_t tci_rrlu_big_scratch_bytes(int grid, int kmax);
 cudaError_t tci_rrlu_big_launch(const double* ain, double* work, double* fact, char* res, void* scratch, int m,
                                 int n, int kmax, int kcap, int leftorth, double reltol, double abstol, int grid,
                                 cudaStream_t stream);
+// RRLU tasks on a thread-block cluster (post NONE or FACTORS).
+int tci_rrlu_cluster_most(int* clusters);
+int tci_rrlu_cluster_ctas(const tci_task& t, int most);
+cudaError_t tci_rrlu_cluster_launch(const tci_task& t, int ncta, double* pivs, cudaStream_t stream);
 }  // namespace tci_k256
 namespace tci_k512 {
 extern const tci_kernel_set kernels;

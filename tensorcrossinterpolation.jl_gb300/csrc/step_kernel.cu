@@ -27,8 +27,10 @@
 #include <algorithm>
 #include <cmath>
 #include <limits.h>
+#include <mutex>
 #include <stddef.h>
 #include <stdint.h>
+#include <string>
 
 #include "ieee_int.h"
 #include "kernels.h"
@@ -2571,6 +2573,7 @@ struct ClusterCtl {
   int factors[2];
   int nr, nc;  // active rows and columns of the block
   int bad[CL_MAX];
+  unsigned long long mx[CL_MAX];
 };
 
 struct ClusterJob {
@@ -2581,12 +2584,14 @@ struct ClusterJob {
   double reltol, abstol;
   double* pivs;        // kmax signed pivots (device scratch)
   double* fact;        // the factored m x n matrix, or null
-  int *rowperm, *colperm;  // full permutations (m, n)
+  int *rowperm, *colperm;  // full permutations (m, n), or null
+  int *rowk, *colk;        // their first npivot entries, or null
   double* diag;        // |pivots| (kmax), or null
 };
 struct ClusterResult {
-  int K, nan;  // nan: valid in CTA 0
+  int K, nan;  // nan and mx (largest |value| bit pattern): valid in CTA 0
   double err;
+  unsigned long long mx;
 };
 
 // Column u of CTA `rank`'s block: in its shared memory (blk), or in the spill.
@@ -2722,10 +2727,9 @@ __device__ __forceinline__ void cluster_update(const ClusterBlock<SPILL>& B, int
 }
 
 // The body, by every thread of every CTA of the cluster.  fill(i, j) gives the
-// matrix; `each` sees every value of this CTA's block once.
-template <bool SPILL, class Fill, class Each>
-__device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCtl& ctl, const Fill& fill,
-                                      const Each& each) {
+// matrix.
+template <bool SPILL, class Fill>
+__device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCtl& ctl, const Fill& fill) {
   const cg::cluster_group cl = cg::this_cluster();
   const int tid = threadIdx.x, ncta = P.pr * P.pc, rank = (int)cl.block_rank(), m = P.m, n = P.n;
   const bool leftorth = P.leftorth != 0;
@@ -2761,6 +2765,7 @@ __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCt
   }
   BigTrack bt;
   bt.init();
+  unsigned long long mx = 0;
   if (nrb > 0 && ncb > 0) {
     const int sq = CL_NT / nrb, sr = CL_NT - sq * nrb;
     int u = tid / nrb, t = tid - u * nrb;
@@ -2768,7 +2773,7 @@ __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCt
     for (int e = tid; e < nrb * ncb; e += CL_NT) {
       const double v = fill(r0 + t, c0 + u);
       B.col(u, rank)[t] = v;
-      each(v);
+      mx = max(mx, (unsigned long long)abs_bits(v));
       const uint32_t key = pack_key(r0 + t, c0 + u);
       bt.push(v, key, key);
       t += sr;
@@ -2882,7 +2887,9 @@ __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCt
     }
   }
   // ---- permutations, and the factors in logical order with the deferred
-  // scaling of addpivot! and the NaN check of L and U (matrixlu.jl:162-169)
+  // scaling of addpivot! and the NaN check of L and U (matrixlu.jl:162-169);
+  // without factors to write only L and U are visited, and dividing by a finite
+  // pivot neither makes nor loses a NaN
   cl.sync();  // the maps and every pivot value are in place; no CTA reads another's block any more
   int bad = 0;
   for (int u = tid >> 5; u < ncb; u += CL_NW) {
@@ -2890,25 +2897,48 @@ __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCt
     const PivotDivisor D(leftorth && lc < K ? __ldcg(&P.pivs[lc]) : 1.0);
     for (int t = tid & 31; t < nrb; t += 32) {
       const int lr = pos_r[t];
+      if (!P.fact && lr >= K && lc >= K) continue;
       double v = B.col(u, rank)[t];
-      if (leftorth && lc < K && lr > lc) v = D.quo(v);
-      if (!leftorth && lr < K && lc > lr) v = PivotDivisor(__ldcg(&P.pivs[lr])).quo(v);
+      if (leftorth && lc < K && lr > lc && (P.fact || !D.safe)) v = D.quo(v);
+      if (!leftorth && lr < K && lc > lr) {
+        const double piv = __ldcg(&P.pivs[lr]);
+        if (P.fact || !int_safe(piv) || abs_bits(piv) == 0) v = PivotDivisor(piv).quo(v);
+      }
       if ((lc < K && lr >= lc) || (lr < K && lr <= lc)) bad |= is_nan_bits(v) ? 1 : 0;
       if (P.fact) P.fact[lr + (size_t)lc * m] = v;
     }
   }
   bad = __syncthreads_or(bad);
-  if (tid == 0) *cl.map_shared_rank(&ctl.bad[rank], 0) = bad;
+  mx = warp_max_u64(mx);
+  if ((tid & 31) == 0) ctl.red_a[tid >> 5] = mx;
+  __syncthreads();
+  if (tid < 32) {
+    mx = warp_max_u64(tid < CL_NW ? ctl.red_a[tid] : 0ULL);
+    if (tid == 0) {
+      *cl.map_shared_rank(&ctl.bad[rank], 0) = bad;
+      *cl.map_shared_rank(&ctl.mx[rank], 0) = mx;
+    }
+  }
   if (rank == 0) {
-    for (int i = tid; i < m; i += CL_NT) P.rowperm[i] = stor_r[i];
-    for (int j = tid; j < n; j += CL_NT) P.colperm[j] = stor_c[j];
+    for (int i = tid; i < m; i += CL_NT) {
+      if (P.rowperm) P.rowperm[i] = stor_r[i];
+      if (P.rowk && i < K) P.rowk[i] = stor_r[i];
+    }
+    for (int j = tid; j < n; j += CL_NT) {
+      if (P.colperm) P.colperm[j] = stor_c[j];
+      if (P.colk && j < K) P.colk[j] = stor_c[j];
+    }
   }
   cl.sync();
   ClusterResult r;
   r.K = K;
   r.nan = 0;
+  r.mx = 0;
   if (rank == 0)
-    for (int t = 0; t < ncta; ++t) r.nan |= ctl.bad[t];
+    for (int t = 0; t < ncta; ++t) {
+      r.nan |= ctl.bad[t];
+      r.mx = max(r.mx, ctl.mx[t]);
+    }
   r.err = K >= min(m, n) ? 0.0 : __longlong_as_double((long long)S.err);
   return r;
 }
@@ -3033,12 +3063,31 @@ cudaError_t tci_rrlu_big_launch(const double* ain, double* work, double* fact, c
 // Launch the resident kernel: one CTA per SM, all resident at once
 // (cooperative launch), after clearing the per-launch part of its state.
 // slots/qc are mapped pinned host memory, st device memory.
+// cluster > 1: in clusters of that many CTAs, which leaves the other GPCs whole
+// for a cluster kernel beside it (the grid is then far below one CTA per SM, so
+// all of it is resident without a cooperative launch).
 cudaError_t tci_resident_launch(tci_queue_slot* slots, uint32_t mask, tci_resident_state* st, tci_queue_ctl* qc,
-                                int grid, unsigned long long wait_ns, cudaStream_t stream) {
+                                int grid, int cluster, unsigned long long wait_ns, cudaStream_t stream) {
   const size_t off = offsetof(tci_resident_state, count);
   cudaError_t e = cudaMemsetAsync((char*)st + off, 0, sizeof(tci_resident_state) - off, stream);
   if (e != cudaSuccess) return e;
   size_t smem = tci_resident_smem_bytes();
+  if (cluster > 1) {
+    e = cudaFuncSetAttribute(tci_resident_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, tci_resident_kernel, slots, mask, st, qc, smem, wait_ns);
+  }
   void* args[] = {(void*)&slots, (void*)&mask, (void*)&st, (void*)&qc, (void*)&smem, (void*)&wait_ns};
   return cudaLaunchCooperativeKernel((const void*)tci_resident_kernel, dim3(grid), dim3(NT), args, smem, stream);
 }
@@ -3060,8 +3109,194 @@ extern const tci_kernel_set kernels = {TCI_STEP_THREADS, TCI_CTAS_PER_SM, tci_st
 
 }  // namespace TCI_KNS
 
-// The entry point without allocation is built once (in the throughput variant).
+// What follows is built once (in the throughput variant).
 #ifndef TCI_SECONDARY
+
+// ------------------------------------------------- RRLU tasks on a cluster
+namespace TCI_KNS {
+namespace {
+
+constexpr size_t CL_SMEM = 224 * 1024;  // dynamic shared memory of a cluster's CTA at most
+
+void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int ncta, size_t smem, cudaStream_t stream) {
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)ncta;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)ncta);
+  cfg.blockDim = dim3(CL_NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+
+// Shared memory of a task's CTA after the factorization's own: f's row and
+// column states, and the index lists they are formed from.
+__host__ __device__ inline size_t cluster_state_smem(int mb, int nb, int nl, int nr) {
+  const size_t b = ((size_t)mb + nb) * 16 + (size_t)mb * nl + (size_t)nb * nr;
+  return (b + 15) / 16 * 16;
+}
+__host__ __device__ inline size_t cluster_smem16(int m, int n, int mb, int nb) {
+  return (cluster_smem(m, n, mb, nb, nb) + 15) / 16 * 16;
+}
+
+// One RRLU task (a given matrix, or f over its index lists) on the launched
+// cluster, with post-processing NONE or FACTORS; the record as task_rrlu writes
+// it.  A task's inputs may be in host memory: each CTA copies the lists of its
+// own rows and columns in one pass.
+__global__ void __launch_bounds__(CL_NT, 1) rrlu_cluster_task_kernel(const tci_task T, ClusterJob P) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ ClusterCtl ctl;
+  __shared__ double s_params[RES_MAX_PARAMS];
+  const long long t0 = clock64();
+  const int tid = threadIdx.x, rank = (int)cg::this_cluster().block_rank();
+  const int m = P.m, n = P.n, mb = P.mb, nb = P.nb, r0 = rank / P.pc * mb, c0 = rank % P.pc * nb;
+  tci_result_head* head = (tci_result_head*)(uintptr_t)T.res;
+  ClusterResult r;
+  if (T.ain) {
+    r = cluster_rrlu<false>(P, smem, ctl, [&](int i, int j) { return __ldcs(T.ain + i + (size_t)j * m); });
+  } else {
+    const int nrb = max(0, min(m, r0 + mb) - r0), ncb = max(0, min(n, c0 + nb) - c0), nl = T.nl, nr = T.nr;
+    double* rs0 = (double*)(smem + cluster_smem16(m, n, mb, nb));
+    double *rs1 = rs0 + mb, *cs0 = rs1 + mb, *cs1 = cs0 + nb;
+    uint8_t* li = (uint8_t*)(cs1 + nb);
+    uint8_t* lj = li + (size_t)mb * nl;
+    const uint8_t* gi = (const uint8_t*)(uintptr_t)T.rows + (size_t)r0 * nl;
+    const uint8_t* gj = (const uint8_t*)(uintptr_t)T.cols + (size_t)c0 * nr;
+    const double* prm = (const double*)(uintptr_t)T.params;
+    for (int e = tid; e < nrb * nl; e += CL_NT) li[e] = gi[e];
+    for (int e = tid; e < ncb * nr; e += CL_NT) lj[e] = gj[e];
+    if (T.nparams <= RES_MAX_PARAMS) {
+      for (int k = tid; k < T.nparams; k += CL_NT) s_params[k] = prm[k];
+      prm = s_params;
+    }
+    __syncthreads();
+    const bool tables = T.lut_full != 0;  // exact integer sums, kept in the same slots
+    for (int e = tid; e < nrb + ncb; e += CL_NT) {
+      const bool row = e < nrb;
+      const int q = row ? e : e - nrb, len = row ? nl : nr, site0 = row ? 0 : nl;
+      const uint8_t* v = row ? li + (size_t)q * nl : lj + (size_t)q * nr;
+      double* d0 = (row ? rs0 : cs0) + q;
+      double* d1 = (row ? rs1 : cs1) + q;
+      if (tables) {
+        long long a0 = 0, a1 = 0;
+        for (int p = 0; p < len; ++p) tci_f_term_int(T.fid, prm, site0 + p, v[p], &a0, &a1);
+        *(long long*)d0 = a0;
+        *(long long*)d1 = a1;
+      } else {
+        double a0 = 0.0, a1 = 0.0;
+        for (int p = 0; p < len; ++p) tci_f_term(T.fid, prm, site0 + p, v[p], &a0, &a1);
+        *d0 = a0;
+        *d1 = a1;
+      }
+    }
+    __syncthreads();
+    Filler F;
+    F.fid = T.fid;
+    F.nparams = T.nparams;
+    F.prm = prm;
+    F.lut0 = tables ? T.lut : nullptr;
+    F.lut1 = tables && tci_f_tables(T.fid) > 1 ? T.lut + T.lutcap0 : nullptr;
+    F.lo0 = T.lut_base0;
+    F.lo1 = 0;
+    r = cluster_rrlu<false>(P, smem, ctl, [&](int i, int j) { return F.val(rs0, rs1, i - r0, cs0, cs1, j - c0); });
+  }
+  if (rank != 0) return;
+  __syncthreads();  // the record's arrays before its head
+  if (tid == 0) {
+    head->status = r.nan ? TCI_ST_NAN : 0;
+    head->npivot = r.K;
+    head->error = r.err;
+    head->maxabs = __longlong_as_double((long long)r.mx);
+    head->maxabs_nan = r.mx > NAN_FLOOR ? 1 : 0;
+    head->lut_used = !T.ain && T.lut_full;
+    head->cycles = clock64() - t0;
+    __threadfence_system();
+    st_release_sys(&head->done, T.ticket + 1);
+  }
+}
+
+}  // namespace
+
+// CTAs of the largest cluster the device runs with a full CTA per SM, and how
+// many such clusters at once (0: none).
+int tci_rrlu_cluster_most(int* clusters) {
+  static std::mutex mu;
+  static int most[64], count[64];
+  static bool ready[64];
+  int dev = 0;
+  if (clusters) *clusters = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!ready[dev]) {
+    cudaError_t ce = cudaFuncSetAttribute(rrlu_cluster_task_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)CL_SMEM);
+    if (ce == cudaSuccess)
+      ce = cudaFuncSetAttribute(rrlu_cluster_task_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int c = CL_MAX; ce == cudaSuccess && c >= 8 && most[dev] == 0; c /= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      cluster_config(cfg, at, c, CL_SMEM, nullptr);
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, rrlu_cluster_task_kernel, &cfg) == cudaSuccess && fit > 0) {
+        most[dev] = c;
+        count[dev] = fit;
+      } else {
+        (void)cudaGetLastError();
+      }
+    }
+    ready[dev] = true;
+  }
+  if (clusters) *clusters = count[dev];
+  return most[dev];
+}
+
+// CTAs for an RRLU task on clusters of at most `most`; 0 if it does not fit.
+int tci_rrlu_cluster_ctas(const tci_task& t, int most) {
+  if (t.m > 65535 || t.n > 65535 || t.m < 1 || t.n < 1) return 0;
+  for (int c = 8; c <= most; c *= 2) {
+    if (c == 8 && most > 8 && (int64_t)t.m * t.n >= 10000) continue;
+    const ClusterGrid g = cluster_grid(t.m, t.n, c);
+    const size_t state = t.ain ? 0 : cluster_state_smem(g.mb, g.nb, t.nl, t.nr);
+    if (cluster_smem16(t.m, t.n, g.mb, g.nb) + state <= CL_SMEM) return c;
+  }
+  return 0;
+}
+
+// The task (absolute addresses, as in resident mode) on `ncta` CTAs; pivs: room
+// for its largest rank in device memory.
+cudaError_t tci_rrlu_cluster_launch(const tci_task& t, int ncta, double* pivs, cudaStream_t stream) {
+  const ClusterGrid g = cluster_grid(t.m, t.n, ncta);
+  ClusterJob P;
+  P.m = t.m;
+  P.n = t.n;
+  P.kmax = std::min(t.maxrank, std::min(t.m, t.n));
+  P.leftorth = t.leftorth;
+  P.pr = g.pr;
+  P.pc = g.pc;
+  P.mb = g.mb;
+  P.nb = g.nb;
+  P.nres = g.nb;
+  P.spill = nullptr;
+  P.reltol = t.reltol;
+  P.abstol = t.abstol;
+  P.pivs = pivs;
+  P.fact = t.post == TCI_POST_FACTORS ? t.core_out : nullptr;
+  P.rowperm = P.fact ? (int*)(t.core_out + (size_t)t.m * t.n) : nullptr;
+  P.colperm = P.fact ? P.rowperm + t.m : nullptr;
+  char* arrays = (char*)(uintptr_t)t.res + sizeof(tci_result_head);
+  const size_t kbytes = ((size_t)t.kcap * 4 + 7) / 8 * 8;
+  P.rowk = (int*)arrays;
+  P.colk = (int*)(arrays + kbytes);
+  P.diag = (double*)(arrays + 2 * kbytes);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  const size_t state = t.ain ? 0 : cluster_state_smem(g.mb, g.nb, t.nl, t.nr);
+  cluster_config(cfg, at, ncta, cluster_smem16(t.m, t.n, g.mb, g.nb) + state, stream);
+  return cudaLaunchKernelEx(&cfg, rrlu_cluster_task_kernel, t, P);
+}
+
+}  // namespace TCI_KNS
 
 // ===================================================================== rrLU
 // without allocation (tci_rrlu_noalloc; no counterpart in the reference).
@@ -3077,8 +3312,6 @@ extern const tci_kernel_set kernels = {TCI_STEP_THREADS, TCI_CTAS_PER_SM, tci_st
 // different streams, or interleaved with no ordering) race on it; calls issued
 // on one stream are ordered and safe.  Nothing in it needs clearing between
 // calls: every element a call reads is written earlier in the same call.
-#include <mutex>
-#include <string>
 
 // error codes of include/tci_gb300.h (that header's function ids clash with
 // tci_functions.h, so it is not included here)
@@ -3096,7 +3329,6 @@ namespace {
 constexpr int64_t NOALLOC_MAX_ELEMS = (int64_t)1 << 19;  // m * n
 constexpr int64_t NOALLOC_MAX_DIM = 16384;               // m and n
 constexpr int64_t NOALLOC_CLUSTER_ELEMS = 2500;          // from this size on a cluster
-constexpr size_t CL_SMEM = 224 * 1024;                   // dynamic shared memory of a cluster's CTA at most
 // working matrix | factors + full permutations | result record
 constexpr int64_t NOALLOC_FACT_DOUBLES = NOALLOC_MAX_ELEMS + NOALLOC_MAX_DIM;
 constexpr int64_t NOALLOC_RES_DOUBLES = 16 + 2 * NOALLOC_MAX_DIM;
@@ -3116,8 +3348,8 @@ __global__ void __launch_bounds__(CL_NT, 1) rrlu_noalloc_cluster_kernel(const do
   extern __shared__ __align__(16) char smem[];
   __shared__ ClusterCtl ctl;
   const int m = P.m;
-  const ClusterResult r = cluster_rrlu<SPILL>(
-      P, smem, ctl, [&](int i, int j) { return __ldcs(ain + i + (size_t)j * m); }, [](double) {});
+  const ClusterResult r =
+      cluster_rrlu<SPILL>(P, smem, ctl, [&](int i, int j) { return __ldcs(ain + i + (size_t)j * m); });
   if (cg::this_cluster().block_rank() == 0 && threadIdx.x == 0) {
     *O.npivot = r.K;
     *O.error = r.err;
@@ -3149,18 +3381,6 @@ __global__ void rrlu_noalloc_epilogue(const double* fact, const char* resb, int 
     *error = h->error;
     *status = (h->status & TCI_ST_NAN) ? TCI_ERR_NAN : 0;
   }
-}
-
-void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int ncta, size_t smem, cudaStream_t stream) {
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)ncta;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)ncta);
-  cfg.blockDim = dim3(CL_NT);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
 }
 
 // CTAs of the cluster for an m x n matrix on a device whose clusters hold at
@@ -3304,6 +3524,7 @@ extern "C" int tci_rrlu_noalloc(const double* A_dev, int64_t m, int64_t n, int64
     P.fact = factors_dev;
     P.rowperm = rowperm_dev;
     P.colperm = colperm_dev;
+    P.rowk = P.colk = nullptr;
     P.diag = nullptr;
     const NoallocOut O{rowperm_dev, colperm_dev, npivot_dev, error_dev, status_dev};
     cudaLaunchConfig_t cfg = {};
