@@ -42,12 +42,39 @@ struct tci_ctx {
   std::recursive_mutex mu;
   int64_t peak_live = 0;  // most solves live at once in a batched / serving drive (stats)
   Engine& eng_ref() { return *engp; }
+  // Solves destroyed while another thread held `mu` (a server holds it until it
+  // stops): released by the next holder.  Waiting for the lock instead would
+  // deadlock a thread whose garbage collector finalizes an old solve while that
+  // thread is the one to stop the server.
+  std::mutex dead_mu;
+  std::vector<tci_solve*> dead;
+  void bury(tci_solve* s) {
+    std::lock_guard<std::mutex> lk(dead_mu);
+    dead.push_back(s);
+  }
+  void release_dead();  // with `mu` held
+  ~tci_ctx();
 };
 
 struct tci_solve {
   tci_ctx* ctx = nullptr;
   Solve s;
 };
+
+void tci_ctx::release_dead() {
+  std::vector<tci_solve*> gone;
+  {
+    std::lock_guard<std::mutex> lk(dead_mu);
+    gone.swap(dead);
+  }
+  for (tci_solve* s : gone) {
+    engp->release_solve(s->s);
+    delete s;
+  }
+}
+tci_ctx::~tci_ctx() {
+  if (engp) release_dead();
+}
 
 namespace {
 
@@ -298,6 +325,7 @@ static int run_solve(tci_ctx* ctx, Solve& s, CoTask& t) {
 int tci_solve_create(tci_ctx* ctx, int32_t L, const int64_t* localdims, int32_t fid, const double* fparams,
                      int64_t nparams, const int64_t* pivots, int64_t np, tci_solve** out) {
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  ctx->release_dead();
   int rc = make_solve(ctx, L, localdims, fid, fparams, nparams, out);
   if (rc) return rc;
   auto piv = to_pivots(pivots, np, L, (*out)->s.d, &rc);
@@ -315,9 +343,10 @@ int tci_solve_create(tci_ctx* ctx, int32_t L, const int64_t* localdims, int32_t 
 
 int tci_solve_destroy(tci_solve* s) {
   if (!s) return 0;
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
-  s->ctx->eng_ref().release_solve(s->s);
-  delete s;
+  tci_ctx* ctx = s->ctx;
+  ctx->bury(s);
+  std::unique_lock<std::recursive_mutex> lk(ctx->mu, std::try_to_lock);
+  if (lk.owns_lock()) ctx->release_dead();
   return 0;
 }
 
@@ -334,6 +363,7 @@ int tci_crossinterpolate2(tci_ctx* ctx, int32_t L, const int64_t* localdims, int
                           const double* fparams, int64_t nparams, const int64_t* pivots, int64_t np,
                           const tci_opts* opts, tci_solve** out) {
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  ctx->release_dead();
   int rc = make_solve(ctx, L, localdims, fid, fparams, nparams, out);
   if (rc) return rc;
   std::vector<int64_t> ones;
@@ -996,6 +1026,7 @@ int drive(tci_ctx* ctx, std::deque<Job>& jobs, bool use_arrival, int64_t max_liv
 int tci_crossinterpolate2_batched(tci_ctx* ctx, int64_t n, const tci_request* reqs, int64_t max_live,
                                   tci_solve** out) {
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  ctx->release_dead();
   std::deque<Job> jobs((size_t)n);
   for (int64_t i = 0; i < n; ++i) jobs[i].req = reqs[i];
   int rc = drive(ctx, jobs, false, max_live, true, nullptr);

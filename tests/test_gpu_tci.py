@@ -438,3 +438,30 @@ def test_trivial_mps_one_pivot(T):
     assert len(tci) == n
     assert tci.rank() == 1
     assert list(tci.linkdims()) == [1] * (n - 1)
+
+
+def test_destroying_a_solve_while_a_server_runs(T):
+    """A solve finalized while a server owns the context (as by a garbage
+    collection in the thread that will stop it) is released later: nothing waits."""
+    import threading
+
+    f = T.DeviceFunction("lorentz")
+    old = [T.crossinterpolate2(float, f, [4] * 4, tolerance=1e-6)[0] for _ in range(3)]
+    srv = T.Server(max_live=4)
+    rid = srv.submit(f, [4] * 4, tolerance=1e-6)
+    done = threading.Event()
+
+    def drop():
+        old.clear()
+        done.set()
+
+    th = threading.Thread(target=drop, daemon=True)
+    th.start()
+    ok = done.wait(20)
+    got = []
+    while not got:
+        got = srv.poll(timeout_ms=100)
+    srv.stop()
+    th.join(20)
+    assert ok and got[0][0] == rid and got[0][1] == 0
+    assert T.crossinterpolate2(float, f, [4] * 4, tolerance=1e-6)[0].rank() > 1
