@@ -1151,6 +1151,58 @@ __device__ int site_col_pivot(const double* col, int j, int r) {
   return s > d + 1 ? si : j;
 }
 
+// What a value, or the largest of several, allows: PROD_DENSE, PROD_MIXED
+// (int_safe) or PROD_FP64.
+__device__ __forceinline__ int prod_class(double v) {
+  return int_safe(v) ? (int_dense(v) ? PROD_DENSE : PROD_MIXED) : PROD_FP64;
+}
+
+// w[i * ws] -= a[i * as] * b for i0 <= i < i1 (separate multiply and subtract),
+// the products as MODE says: four elements at a time with their loads first, so
+// that their chains overlap.  One warp alone is faster with FP64 products (one
+// instruction instead of two dozen), many warps with integer ones.
+template <int MODE>
+__device__ __forceinline__ void row_axpy(double* w, size_t ws, const double* a, size_t as, int i0, int i1, double b) {
+  const DenseFactor bd = dense_split(b);
+  const IntFactor bi = int_split(b);
+  auto mul = [&](double y) {
+    return MODE == PROD_DENSE ? int_mul_dense(dense_split(y), bd)
+                              : (MODE == PROD_MIXED ? int_mul(int_split(y), bi) : __dmul_rn(y, b));
+  };
+  int i = i0;
+  for (; i + 4 <= i1; i += 4) {
+    double x[4], y[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      x[q] = w[(size_t)(i + q) * ws];
+      y[q] = a[(size_t)(i + q) * as];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) y[q] = mul(y[q]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w[(size_t)(i + q) * ws] = __dsub_rn(x[q], y[q]);
+  }
+  if (i < i1) {  // up to three more, the last one repeated (not stored)
+    double x[3], y[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int k = min(i + q, i1 - 1);
+      x[q] = w[(size_t)k * ws];
+      y[q] = a[(size_t)k * as];
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) y[q] = mul(y[q]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (i + q < i1) w[(size_t)(i + q) * ws] = __dsub_rn(x[q], y[q]);
+  }
+}
+__device__ __forceinline__ void row_axpy_by(int mode, double* w, size_t ws, const double* a, int i0, int i1, double b) {
+  if (mode == PROD_DENSE) row_axpy<PROD_DENSE>(w, ws, a, 1, i0, i1, b);
+  else if (mode == PROD_MIXED) row_axpy<PROD_MIXED>(w, ws, a, 1, i0, i1, b);
+  else row_axpy<PROD_FP64>(w, ws, a, 1, i0, i1, b);
+}
+
 // getrf with partial pivoting of the r x r matrix A (lda = r), in the oracle's
 // order: per column j, the pivot row p (site_col_pivot), a whole-row swap of
 // rows j and p, the column below the diagonal times the IEEE reciprocal of the
@@ -1167,26 +1219,35 @@ __device__ int site_getrf(double* A, int r, int* ipiv, Ctl& ctl) {
     if (warp == 0) {
       int sing = 0;
       for (int j = 0; j < r; ++j) {
-        const int p = site_col_pivot(A + (size_t)j * r, j, r);
-        const double piv = A[p + (size_t)j * r];
-        if (piv == 0.0) {
+        // lane i holds A[i, j]; the pivot rule of site_col_pivot by warp reductions
+        double* cj = A + (size_t)j * r;
+        const double v = lane < r ? cj[lane] : 0.0;
+        const uint64_t bits = abs_bits(v);
+        const uint64_t s = lane > j && lane < r && bits <= NAN_FLOOR ? bits + 1 : 0;
+        const uint64_t best = warp_max_u64(s);
+        const uint64_t d = __shfl_sync(FULL, bits, j);
+        const int first = __ffs(__ballot_sync(FULL, s == best && s != 0)) - 1;
+        const int p = d <= NAN_FLOOR && best > d + 1 ? first : j;
+        const double piv = __shfl_sync(FULL, v, p), vj = __shfl_sync(FULL, v, j);
+        if (abs_bits(piv) == 0) {
           sing = 1;
           break;
         }
         if (lane == 0) ipiv[j] = p;
-        __syncwarp();
-        if (p != j && lane < r) {
-          const double a = A[j + (size_t)lane * r], b = A[p + (size_t)lane * r];
-          A[j + (size_t)lane * r] = b;
-          A[p + (size_t)lane * r] = a;
+        double y = 0.0;  // lane c: the new A[j, c]
+        if (lane < r) {
+          y = A[p + (size_t)lane * r];
+          if (p != j) {
+            const double a = A[j + (size_t)lane * r];
+            A[j + (size_t)lane * r] = y;
+            A[p + (size_t)lane * r] = a;
+          }
         }
+        const double rcp = PivotDivisor(piv).quo(1.0);
+        const double l = __dmul_rn(lane == p ? vj : v, rcp);
         __syncwarp();
-        const double rcp = 1.0 / A[j + (size_t)j * r];
-        if (lane > j && lane < r) A[lane + (size_t)j * r] = A[lane + (size_t)j * r] * rcp;
-        __syncwarp();
-        if (lane > j && lane < r)
-          for (int c = j + 1; c < r; ++c)
-            A[lane + (size_t)c * r] = A[lane + (size_t)c * r] - A[lane + (size_t)j * r] * A[j + (size_t)c * r];
+        if (lane > j && lane < r) cj[lane] = l;
+        if (lane > j && lane < r) row_axpy<PROD_FP64>(A + lane, (size_t)r, A + j, (size_t)r, j + 1, r, l);
         __syncwarp();
       }
       if (lane == 0) ctl.status = sing;
@@ -1207,7 +1268,7 @@ __device__ int site_getrf(double* A, int r, int* ipiv, Ctl& ctl) {
   for (int j = 0; j < r; ++j) {
     const int p = ctl.r;
     const double piv = ctl.piv;
-    if (piv == 0.0) {
+    if (abs_bits(piv) == 0) {
       __syncthreads();
       return 1;
     }
@@ -1216,7 +1277,7 @@ __device__ int site_getrf(double* A, int r, int* ipiv, Ctl& ctl) {
       double* cj = A + (size_t)j * r;
       const double djj = cj[j];
       __syncwarp();
-      const double rcp = 1.0 / piv;
+      const double rcp = PivotDivisor(piv).quo(1.0);
       for (int i = j + 1 + lane; i < r; i += 32) {
         const double v = i == p ? djj : cj[i];
         cj[i] = v * rcp;
@@ -1240,7 +1301,7 @@ __device__ int site_getrf(double* A, int r, int* ipiv, Ctl& ctl) {
       if (j + 1 < r) {
         double* c1 = A + (size_t)(j + 1) * r;
         const double y = c1[j];
-        for (int i = j + 1 + lane; i < r; i += 32) c1[i] = c1[i] - lj[i] * y;
+        for (int i = j + 1 + lane; i < r; i += 32) c1[i] = __dsub_rn(c1[i], __dmul_rn(lj[i], y));
         __syncwarp();
         const int pn = site_col_pivot(c1, j + 1, r);
         if (lane == 0) {
@@ -1249,11 +1310,10 @@ __device__ int site_getrf(double* A, int r, int* ipiv, Ctl& ctl) {
         }
       }
     } else {
-      for (int c = j + 2 + (warp - 1); c < r; c += NW - 1) {
-        double* cc = A + (size_t)c * r;
-        const double y = cc[j];
-        for (int i = j + 1 + lane; i < r; i += 32) cc[i] = cc[i] - lj[i] * y;
-      }
+      // four columns of a warp at a time: lane rows, loads first
+      for (int c = j + 2 + 4 * (warp - 1); c < r; c += 4 * (NW - 1))
+        for (int i = j + 1 + lane; i < r; i += 32)
+          row_axpy<PROD_FP64>(A + i, (size_t)r, A + j, (size_t)r, c, min(c + 4, r), lj[i]);
     }
     __syncthreads();
   }
@@ -1274,7 +1334,7 @@ __device__ void task_site(const tci_task& T, const char* blob, char* resb, char*
   SmemCursor cur{smem};
   double* A = T.smem_mode == 1 ? (double*)cur.take((size_t)r * r * 8) : T.work;
   int* ipiv = (int*)cur.take((size_t)r * 4);
-  (void)cur.take((size_t)r * 4);  // unused slot (keeps the host's shared-memory plan)
+  int* colcls = (int*)cur.take((size_t)r * 4);  // prod_class of each column of the factored P
   double* ps0 = (double*)cur.take((size_t)r * 8);
   double* ps1 = (double*)cur.take((size_t)r * 8);
   double* cs0 = (double*)cur.take((size_t)r * 8);
@@ -1295,7 +1355,17 @@ __device__ void task_site(const tci_task& T, const char* blob, char* resb, char*
     for (int i = lane; i < r; i += 32) A[i + (size_t)j * r] = F.val(ps0, ps1, j, cs0, cs1, i);
   __syncthreads();
   const int singular = site_getrf(A, r, ipiv, ctl);
-  (void)cur.take((size_t)r * 8);  // unused slot (keeps the host's shared-memory plan)
+  // reciprocals of the diagonal (int_divisor), for the back substitution of every row
+  uint64_t* rec = (uint64_t*)cur.take((size_t)r * 8);
+  for (int j = tid; j < r; j += NT) rec[j] = int_divisor(A[j + (size_t)j * r]).R;
+  // (up to one warp of rows per SM quarter: FP64 products, see row_axpy)
+  for (int j = warp; j < r; j += NW) {
+    int c = m <= 128 ? PROD_FP64 : PROD_DENSE;
+    for (int i = lane; i < r; i += 32)
+      if (i != j) c = max(c, prod_class(A[i + (size_t)j * r]));
+    c = __reduce_max_sync(FULL, c);
+    if (lane == 0) colcls[j] = c;
+  }
   size_t used = (size_t)(cur.p - smem);
   int RB = (int)((smem_bytes > used ? smem_bytes - used : 0) / ((size_t)r * 8 + 8));
   RB = RB > NT ? NT : RB;
@@ -1305,13 +1375,13 @@ __device__ void task_site(const tci_task& T, const char* blob, char* resb, char*
   int nanflag = 0;
   for (int base = 0; base < m; base += RB) {
     const int rows_here = min(RB, m - base);
-    for (int e = tid; e < rows_here * r; e += NT) {
-      int rr = e % rows_here, q = e / rows_here;
-      double v = F.val(rs0, rs1, base + rr, cs0, cs1, q);
-      W[rr + (size_t)q * RB] = v;
-      unsigned long long b = abs_bits(v);
-      mx = b > mx ? b : mx;
-    }
+    for (int q = warp; q < r; q += NW)
+      for (int rr = lane; rr < rows_here; rr += 32) {
+        const double v = F.val(rs0, rs1, base + rr, cs0, cs1, q);
+        W[rr + (size_t)q * RB] = v;
+        const unsigned long long b = abs_bits(v);
+        mx = b > mx ? b : mx;
+      }
     __syncthreads();
     if (!singular) {
       for (int rr = tid; rr < rows_here; rr += NT) {
@@ -1324,24 +1394,34 @@ __device__ void task_site(const tci_task& T, const char* blob, char* resb, char*
             w[(size_t)p * RB] = a;
           }
         }
-        for (int j = 0; j < r; ++j) {
+        for (int j = 0; j + 1 < r; ++j) {
           const double bj = w[(size_t)j * RB];
-          for (int i = j + 1; i < r; ++i) w[(size_t)i * RB] = w[(size_t)i * RB] - A[i + (size_t)j * r] * bj;
+          const int cc = colcls[j];
+          row_axpy_by(cc == PROD_FP64 ? cc : max(cc, prod_class(bj)), w, (size_t)RB, A + (size_t)j * r, j + 1, r, bj);
         }
         for (int j = r - 1; j >= 0; --j) {
-          const double bj = w[(size_t)j * RB] / A[j + (size_t)j * r];
+          const double d = A[j + (size_t)j * r], x = w[(size_t)j * RB];
+          double bj;
+          if (int_safe(d) && int_safe(x) && abs_bits(d) != 0) {
+            const uint32_t dh = ii_hi(d);
+            bj = int_div(x, IntDivisor{((uint64_t)((dh & 0xfffffu) | 0x100000u) << 32) | ii_lo(d), rec[j],
+                                       dh & 0xfff00000u});
+          } else {
+            bj = __ddiv_rn(x, d);
+          }
           w[(size_t)j * RB] = bj;
-          for (int i = 0; i < j; ++i) w[(size_t)i * RB] = w[(size_t)i * RB] - A[i + (size_t)j * r] * bj;
+          const int cc = colcls[j];
+          row_axpy_by(cc == PROD_FP64 ? cc : max(cc, prod_class(bj)), w, (size_t)RB, A + (size_t)j * r, 0, j, bj);
         }
       }
     }
     __syncthreads();
-    for (int e = tid; e < rows_here * r; e += NT) {
-      int rr = e % rows_here, q = e / rows_here;
-      double v = W[rr + (size_t)q * RB];
-      if (is_nan_bits(v)) nanflag = 1;
-      T.core_out[(base + rr) + (size_t)q * m] = v;
-    }
+    for (int q = warp; q < r; q += NW)
+      for (int rr = lane; rr < rows_here; rr += 32) {
+        const double v = W[rr + (size_t)q * RB];
+        if (is_nan_bits(v)) nanflag = 1;
+        T.core_out[(base + rr) + (size_t)q * m] = v;
+      }
     __syncthreads();
   }
   unsigned long long mxall = block_max_u64(mx, ctl);
@@ -1484,7 +1564,58 @@ __device__ void task_eval(const tci_task& T, const char* blob, char* resb, char*
 // right environments Re_p = C_{p+1}[i_{p+1}] ... C_{L-1}[i_{L-1}] of the start,
 // value(p, v) = sum_b (sum_a Le_p[a] C_p[a, v, b]) Re_p[b], every sum in index
 // order with separate multiply and add (the oracle uses the same order).
-__device__ void task_search(const tci_task& T, const char* blob, char* resb, char* smem) {
+// The order of every sum is fixed, so its additions are a serial chain; the
+// products before it are not (chain_dot loads and multiplies eight at a time, on
+// the integer pipes where many warps share the FP64 pipe).
+// The two environment chains run side by side on the two halves of the CTA, and
+// the inner sums of all (p, v, b) are spread over the threads before the outer
+// ones.
+template <bool INT>
+__device__ __forceinline__ double chain_dot(double acc, const double* __restrict__ x, const double* __restrict__ y,
+                                            size_t ystride, int n) {
+  int t = 0;
+  for (; t + 8 <= n; t += 8) {
+    double p[8], q[8];
+    bool safe = INT, dense = INT;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      p[k] = x[t + k];
+      q[k] = y[(size_t)(t + k) * ystride];
+    }
+    if (INT) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        safe = safe && int_safe(p[k]) && int_safe(q[k]);
+        dense = dense && int_dense(p[k]) && int_dense(q[k]);
+      }
+    }
+    if (safe && dense) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) q[k] = int_mul_dense(dense_split(p[k]), dense_split(q[k]));
+    } else if (safe) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) q[k] = int_mul(int_split(p[k]), int_split(q[k]));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) q[k] = __dmul_rn(p[k], q[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc = __dadd_rn(acc, q[k]);
+  }
+  if (t < n) {  // the rest, its loads first as well
+    double q[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) q[k] = y[(size_t)min(t + k, n - 1) * ystride];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      if (t + k >= n) break;
+      acc = __dadd_rn(acc, __dmul_rn(x[t + k], q[k]));
+    }
+  }
+  return acc;
+}
+
+__device__ void task_search(const tci_task& T, const char* blob, char* resb, char* smem, size_t smem_bytes) {
   const int L = T.L, tid = threadIdx.x;
   const double* prm = (const double*)at(blob, T.params);
   const uint8_t* st = (const uint8_t*)at(blob, T.rows);
@@ -1521,57 +1652,71 @@ __device__ void task_search(const tci_task& T, const char* blob, char* resb, cha
     ioff[L] = c;
   }
   __syncthreads();
-  // left environments
-  if (tid == 0) env[loff[0]] = 1.0;
+  // left environments on the first half of the threads, right ones on the second
+  if (tid == 0) {
+    env[loff[0]] = 1.0;
+    env[roff[L - 1]] = 1.0;
+  }
   __syncthreads();
-  for (int p = 0; p + 1 < L; ++p) {
+  for (int k = 0; k + 1 < L; ++k) {
+    const bool left = tid < NT / 2;
+    const int p = left ? k : L - 1 - k;
     const tci_core_ref c = cr[p];
-    const int i = st[p];
-    const double* le = env + loff[p];
-    double* nx = env + loff[p + 1];
-    for (int b = tid; b < c.r1; b += NT) {
-      double acc = 0.0;
-      const double* col = c.p + (size_t)c.r0 * (i + (size_t)c.d * b);
-      for (int a = 0; a < c.r0; ++a) acc = __dadd_rn(acc, __dmul_rn(le[a], col[a]));
-      nx[b] = acc;
+    const double* col0 = c.p + (size_t)c.r0 * st[p];
+    const size_t slice = (size_t)c.r0 * c.d;
+    if (left) {
+      for (int b = tid; b < c.r1; b += NT / 2)
+        env[loff[p + 1] + b] = chain_dot<false>(0.0, env + loff[p], col0 + slice * b, 1, c.r0);
+    } else {
+      for (int a = tid - NT / 2; a < c.r0; a += NT / 2)
+        env[roff[p - 1] + a] = chain_dot<false>(0.0, env + roff[p], col0 + a, slice, c.r1);
     }
     __syncthreads();
   }
-  // right environments
-  if (tid == 0) env[roff[L - 1]] = 1.0;
-  __syncthreads();
-  for (int p = L - 1; p > 0; --p) {
-    const tci_core_ref c = cr[p];
-    const int i = st[p];
-    const double* re = env + roff[p];
-    double* nx = env + roff[p - 1];
-    for (int a = tid; a < c.r0; a += NT) {
-      double acc = 0.0;
-      for (int b = 0; b < c.r1; ++b)
-        acc = __dadd_rn(acc, __dmul_rn(c.p[a + (size_t)c.r0 * (i + (size_t)c.d * b)], re[b]));
-      nx[a] = acc;
-    }
-    __syncthreads();
-  }
-  // every (p, v)
+  // every (p, v): the inner sums of a block of items, then their outer sums
   const int nitems = ioff[L];
+  double* wbuf = (double*)((char*)cr + align_up((size_t)L * sizeof(tci_core_ref), 16));
+  const size_t used = (size_t)((char*)wbuf - smem);
+  const int rmax = max(T.r, 1), block = (int)((smem_bytes > used ? smem_bytes - used : 0) / ((size_t)rmax * 8));
+  for (int j0 = 0; block > 0 && j0 < nitems; j0 += block) {
+    const int j1 = min(nitems, j0 + block);
+    for (int e = tid; e < (j1 - j0) * rmax; e += NT) {
+      const int it = j0 + e / rmax, b = e % rmax;
+      int p = 0;
+      while (ioff[p + 1] <= it) ++p;
+      const tci_core_ref c = cr[p];
+      if (b >= c.r1) continue;
+      wbuf[e] = chain_dot<true>(0.0, env + loff[p], c.p + (size_t)c.r0 * ((it - ioff[p]) + (size_t)c.d * b), 1, c.r0);
+    }
+    __syncthreads();
+    for (int it = j0 + tid; it < j1; it += NT) {
+      int p = 0;
+      while (ioff[p + 1] <= it) ++p;
+      tout[it] = chain_dot<false>(0.0, wbuf + (size_t)(it - j0) * rmax, env + roff[p], 1, cr[p].r1);
+    }
+    __syncthreads();
+  }
   for (int it = tid; it < nitems; it += NT) {
     int p = 0;
     while (ioff[p + 1] <= it) ++p;
     const int v = it - ioff[p];
-    const tci_core_ref c = cr[p];
-    const double* le = env + loff[p];
-    const double* re = env + roff[p];
-    double val = 0.0;
-    for (int b = 0; b < c.r1; ++b) {
-      const double* col = c.p + (size_t)c.r0 * (v + (size_t)c.d * b);
-      double w = 0.0;
-      for (int a = 0; a < c.r0; ++a) w = __dadd_rn(w, __dmul_rn(le[a], col[a]));
-      val = __dadd_rn(val, __dmul_rn(w, re[b]));
+    if (block == 0) {  // no room for one item's inner sums: each thread takes a whole item
+      const tci_core_ref c = cr[p];
+      double val = 0.0;
+      for (int b = 0; b < c.r1; ++b)
+        val = __dadd_rn(val, __dmul_rn(chain_dot<true>(0.0, env + loff[p], c.p + (size_t)c.r0 * (v + (size_t)c.d * b),
+                                                       1, c.r0), env[roff[p] + b]));
+      tout[it] = val;
     }
-    tout[it] = val;
     double a0 = 0.0, a1 = 0.0;
-    for (int s = 0; s < L; ++s) tci_f_term(T.fid, prm, s, s == p ? v : st[s], &a0, &a1);
+    if (tci_f_tables(T.fid) > 0) {  // the same sums, exact integers, off the FP64 pipe
+      long long i0 = 0, i1 = 0;
+      for (int s = 0; s < L; ++s) tci_f_term_int(T.fid, prm, s, s == p ? v : st[s], &i0, &i1);
+      a0 = (double)i0;
+      a1 = (double)i1;
+    } else {
+      for (int s = 0; s < L; ++s) tci_f_term(T.fid, prm, s, s == p ? v : st[s], &a0, &a1);
+    }
     fout[it] = tci_f_finish(T.fid, prm, T.nparams, a0, a1);
   }
   if (tid == 0) {
@@ -1645,7 +1790,7 @@ __device__ void run_task(const tci_task& T, const char* blob, char* resb, char* 
     case TCI_TASK_CORE: task_core(T, blob, resb, smem, ctl); break;
     case TCI_TASK_EVAL: task_eval(T, blob, resb, smem, ctl); break;
     case TCI_TASK_SUM: task_sum(T, blob, resb, smem); break;
-    case TCI_TASK_SEARCH: task_search(T, blob, resb, smem); break;
+    case TCI_TASK_SEARCH: task_search(T, blob, resb, smem, smem_bytes); break;
     case TCI_TASK_TABLE: task_table(T, blob, resb); break;
     default: break;
   }
