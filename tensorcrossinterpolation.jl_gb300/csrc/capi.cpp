@@ -20,6 +20,9 @@
 #include "engine.h"
 #include "tc_gemm.h"
 
+cudaError_t tci_lu_factors_launch(const double* F, int m, int n, int K, int leftorth, double* L, double* U,
+                                  cudaStream_t st);
+
 using namespace tci;
 
 // A context owns a pool of engines, each with its own stream and buffers.
@@ -100,40 +103,6 @@ std::vector<std::vector<uint8_t>> to_pivots(const int64_t* piv, int64_t np, int 
     out.push_back(v);
   }
   return out;
-}
-
-// Points (np x L, row-major, 1-based int64) -> flat 0-based uint8 multi-indices,
-// range-checked; large inputs are split over host threads.
-int pack_points(const int64_t* pts, int64_t np, int L, const std::vector<int>& d, std::vector<uint8_t>& out) {
-  out.resize((size_t)np * (size_t)L);
-  auto run = [&](int64_t p0, int64_t p1) {
-    bool ok = true;
-    for (int64_t p = p0; p < p1; ++p) {
-      const int64_t* x = pts + p * L;
-      uint8_t* o = out.data() + (size_t)p * L;
-      for (int q = 0; q < L; ++q) {
-        ok &= x[q] >= 1 && x[q] <= d[q];
-        o[q] = (uint8_t)(x[q] - 1);
-      }
-    }
-    return ok;
-  };
-  const int64_t work = np * (int64_t)L;
-  int nt = work >= (1 << 22) ? (int)std::min<int64_t>(8, std::max(1u, std::thread::hardware_concurrency())) : 1;
-  bool ok = true;
-  if (nt == 1) {
-    ok = run(0, np);
-  } else {
-    std::vector<std::thread> th;
-    std::vector<char> res(nt, 1);
-    const int64_t per = (np + nt - 1) / nt;
-    for (int t = 0; t < nt; ++t)
-      th.emplace_back([&, t] { res[t] = run(std::min(np, t * per), std::min(np, (t + 1) * per)); });
-    for (auto& x : th) x.join();
-    for (char r : res) ok &= r != 0;
-  }
-  if (!ok) return fail(TCI_ERR_ARG, "pivot index out of range");
-  return 0;
 }
 
 double now_s() {
@@ -623,11 +592,11 @@ int tci_get_history(const tci_solve* s, int64_t* ranks, double* errors, int64_t*
   return 0;
 }
 
-// Train values at packed points, in blocks of 2^22 points (device memory).
-static int train_values(tci_ctx* ctx, const Solve& s, const std::vector<uint8_t>& pts, int64_t np, double* out) {
+// Train values, in blocks of 2^22 points (device memory).
+static int train_values(tci_ctx* ctx, const Solve& s, const int64_t* points, int64_t np, double* out) {
   const int64_t chunk = 1 << 22;
   for (int64_t b = 0; b < np; b += chunk) {
-    int rc = ctx->eng_ref().eval_train(s, pts.data() + b * s.L, std::min(chunk, np - b), out + b);
+    int rc = ctx->eng_ref().eval_train(s, points + b * s.L, std::min(chunk, np - b), out + b);
     if (rc) return rc;
   }
   return 0;
@@ -635,10 +604,7 @@ static int train_values(tci_ctx* ctx, const Solve& s, const std::vector<uint8_t>
 
 int tci_evaluate(tci_solve* s, const int64_t* points, int64_t np, double* out) {
   std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
-  std::vector<uint8_t> pts;
-  int rc = pack_points(points, np, s->s.L, s->s.d, pts);
-  if (rc) return rc;
-  return train_values(s->ctx, s->s, pts, np, out);
+  return train_values(s->ctx, s->s, points, np, out);
 }
 
 int tci_sum(tci_solve* s, double* out) {
@@ -649,11 +615,10 @@ int tci_sum(tci_solve* s, double* out) {
 
 namespace {
 
-// evaluate() of the train held in s.cores at np points (packed 0-based local
-// indices) with TF32 hi/lo split products on the tensor cores
+// evaluate() of the train held in s.cores at np points (1-based) with TF32 hi/lo split products on the tensor cores
 // (tci_tc_evaluate_split); the first min(np, 256) points are also evaluated in
 // FP64 and *err_est = max |split - fp64| / max |fp64| over them.
-int split_evaluate(tci_ctx* ctx, Solve& s, const std::vector<uint8_t>& pts, int64_t np, double* out, double* err_est) {
+int split_evaluate(tci_ctx* ctx, Solve& s, const int64_t* points, int64_t np, double* out, double* err_est) {
   const int L = s.L;
   std::vector<int64_t> dims((size_t)(3 * L));
   std::vector<const double*> cores((size_t)L);
@@ -689,7 +654,7 @@ int split_evaluate(tci_ctx* ctx, Solve& s, const std::vector<uint8_t>& pts, int6
   auto ck = [&](cudaError_t ce) {
     if (!rc && ce != cudaSuccess) rc = fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
   };
-  if (!rc && np > 0) ck(cudaMemcpyAsync(dpts, pts.data(), (size_t)np * L, cudaMemcpyHostToDevice, e.stream()));
+  if (!rc && np > 0) rc = e.upload_points(s, points, np, (uint8_t*)dpts);
   if (!rc) ck(cudaMemsetAsync(derr, 0, sizeof(int), e.stream()));
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (!rc) ck(cudaEventCreate(&ev0));
@@ -739,10 +704,7 @@ int tci_evaluate_prec(tci_solve* s, const int64_t* points, int64_t np, double* o
   }
   if (precision != TCI_PREC_TF32X3) return fail(TCI_ERR_ARG, "unknown precision");
   std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
-  std::vector<uint8_t> pts;
-  int rc = pack_points(points, np, s->s.L, s->s.d, pts);
-  if (rc) return rc;
-  return split_evaluate(s->ctx, s->s, pts, np, out, err_est);
+  return split_evaluate(s->ctx, s->s, points, np, out, err_est);
 }
 
 // ---------------------------------------------------------------- batches / serving
@@ -1274,32 +1236,45 @@ int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxran
   if (!dout) return fail(TCI_ERR_OOM, "device memory");
   r.t.core_out = dout;
   std::vector<Req*> reqs{&r};
+  // A fresh L or U has no pages yet; a device copy into it would fault them in one
+  // by one, and far from the core that reads them next.  Another thread touches
+  // them (contents kept) while the device works.
+  std::thread toucher;
+  const size_t touch = (size_t)std::max(m, n) * (size_t)kmax * 8;
+  if (touch >= ((size_t)1 << 20))
+    toucher = std::thread([=] {
+      const size_t nl = L ? (size_t)m * (size_t)kmax * 8 : 0, nu = U ? (size_t)kmax * (size_t)n * 8 : 0;
+      for (size_t q = 0; q < nl; q += 4096) ((volatile char*)L)[q] = ((volatile char*)L)[q];
+      for (size_t q = 0; q < nu; q += 4096) ((volatile char*)U)[q] = ((volatile char*)U)[q];
+    });
   int rc = e.run_tasks(reqs);
+  if (toucher.joinable()) toucher.join();
   if (rc) {
     e.free_core(dout);
     return rc;
   }
   const tci_result_head* h = r.head();
   const int K = h->npivot;
-  std::vector<double> F(out_elems);
-  cudaError_t ce = cudaMemcpyAsync(F.data(), dout, out_elems * 8, cudaMemcpyDeviceToHost, e.stream());
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(e.stream());
+  // the permutations, and L and U as compact matrices, straight to the caller
+  std::vector<int32_t> perms((size_t)(m + n));
+  const size_t nl = (size_t)m * K, nu = (size_t)K * n;
+  double* lu = (L || U) && nl + nu > 0 ? e.alloc_core(nl + nu) : nullptr;
+  cudaError_t ce = (L || U) && nl + nu > 0 && !lu ? cudaErrorMemoryAllocation : cudaSuccess;
+  if (ce == cudaSuccess && m + n > 0)
+    ce = cudaMemcpyAsync(perms.data(), dout + m * n, perms.size() * 4, cudaMemcpyDeviceToHost, e.stream());
+  if (ce == cudaSuccess && lu)
+    ce = tci_lu_factors_launch(dout, (int)m, (int)n, K, leftorthogonal ? 1 : 0, lu, lu + nl, e.stream());
+  if (ce == cudaSuccess && lu && L) ce = cudaMemcpyAsync(L, lu, nl * 8, cudaMemcpyDeviceToHost, e.stream());
+  if (ce == cudaSuccess && lu && U) ce = cudaMemcpyAsync(U, lu + nl, nu * 8, cudaMemcpyDeviceToHost, e.stream());
+  const cudaError_t sync = cudaStreamSynchronize(e.stream());
+  if (lu) e.free_core(lu);
   e.free_core(dout);
-  if (ce != cudaSuccess) return fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
-  const int32_t* perms = (const int32_t*)(F.data() + m * n);
+  if (ce == cudaSuccess) ce = sync;
+  if (ce != cudaSuccess) return fail(ce == cudaErrorMemoryAllocation ? TCI_ERR_OOM : TCI_ERR_CUDA, cudaGetErrorString(ce));
   if (rowperm)
     for (int64_t i = 0; i < m; ++i) rowperm[i] = perms[i] + 1;
   if (colperm)
     for (int64_t j = 0; j < n; ++j) colperm[j] = perms[m + j] + 1;
-  // L = tril(A[:, 1:K]), U = triu(A[1:K, :]), unit diagonal on L or U (matrixlu.jl:162-174)
-  if (L)
-    for (int64_t j = 0; j < K; ++j)
-      for (int64_t i = 0; i < m; ++i)
-        L[i + j * m] = i < j ? 0.0 : (i == j && leftorthogonal ? 1.0 : F[i + j * m]);
-  if (U)
-    for (int64_t j = 0; j < n; ++j)
-      for (int64_t i = 0; i < K; ++i)
-        U[i + j * K] = i > j ? 0.0 : (i == j && !leftorthogonal ? 1.0 : F[i + j * m]);
   if (npivot) *npivot = K;
   if (error) *error = h->error;
   if (h->status & TCI_ST_NAN) return fail(TCI_ERR_NAN, "lu.L contains NaNs");
@@ -1868,9 +1843,7 @@ int tci_tt_evaluate(tci_ctx* ctx, int32_t L, const int64_t* dims, const double* 
   Solve s;
   int rc = upload_tt3(e, L, dims, cores, s);
   if (rc) return rc;
-  std::vector<uint8_t> pts;
-  rc = pack_points(points, np, L, s.d, pts);
-  if (!rc) rc = train_values(ctx, s, pts, np, out);
+  rc = train_values(ctx, s, points, np, out);
   e.release_cores(s);
   return rc;
 }
@@ -1888,9 +1861,7 @@ int tci_tt_evaluate_prec(tci_ctx* ctx, int32_t L, const int64_t* dims, const dou
   Solve s;
   int rc = upload_tt3(e, L, dims, cores, s);
   if (rc) return rc;
-  std::vector<uint8_t> pts;
-  rc = pack_points(points, np, L, s.d, pts);
-  if (!rc) rc = split_evaluate(ctx, s, pts, np, out, err_est);
+  rc = split_evaluate(ctx, s, points, np, out, err_est);
   e.release_cores(s);
   return rc;
 }

@@ -248,6 +248,23 @@ __global__ void lu_left_right_kernel(const double* __restrict__ F, const int32_t
   }
 }
 
+// L = tril(A[:, 1:K]) (m x K) and U = triu(A[1:K, :]) (K x n) with the unit
+// diagonal (matrixlu.jl:162-174) from the factored m x n matrix F.
+__global__ void lu_factors_kernel(const double* __restrict__ F, int m, int n, int K, int leftorth,
+                                  double* __restrict__ L, double* __restrict__ U) {
+  const int64_t nl = (int64_t)m * K, nu = (int64_t)K * n;
+  for (int64_t e = gtid(); e < nl + nu; e += gstride()) {
+    if (e < nl) {
+      const int i = (int)(e % m), j = (int)(e / m);
+      L[e] = i < j ? 0.0 : (i == j && leftorth ? 1.0 : F[e]);
+    } else {
+      const int64_t f = e - nl;
+      const int i = (int)(f % K), j = (int)(f / K);
+      U[f] = i > j ? 0.0 : (i == j && !leftorth ? 1.0 : F[i + (int64_t)m * j]);
+    }
+  }
+}
+
 // MatrixLUCI left/right (matrixluci.jl:40-84) from the factored matrix F as
 // above: one thread per row of left (m threads), then one per column of right
 // (n threads), each in the order of the oracle's loops (separate multiply,
@@ -435,6 +452,14 @@ cudaError_t tci_lu_left_right_launch(const double* F, const int32_t* rowperm, co
   const int64_t total = (left ? (int64_t)m * K : 0) + (right ? (int64_t)K * n : 0);
   if (total == 0) return cudaSuccess;
   lu_left_right_kernel<<<grid_for(total), CT, 0, st>>>(F, rowperm, colperm, m, n, K, leftorth, left, right);
+  return cudaGetLastError();
+}
+
+cudaError_t tci_lu_factors_launch(const double* F, int m, int n, int K, int leftorth, double* L, double* U,
+                                  cudaStream_t st) {
+  const int64_t total = ((int64_t)m + n) * K;
+  if (total == 0) return cudaSuccess;
+  lu_factors_kernel<<<grid_for(total), CT, 0, st>>>(F, m, n, K, leftorth, L, U);
   return cudaGetLastError();
 }
 

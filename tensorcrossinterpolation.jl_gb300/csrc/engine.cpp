@@ -15,6 +15,8 @@
 #include <numeric>
 #include <thread>
 
+cudaError_t tci_pack_points_launch(const int64_t* pts, int64_t np, int L, const int* dims, uint8_t* out, int* bad,
+                                   int num_sms, cudaStream_t st);
 int tci_tt_eval_max_bond();
 cudaError_t tci_tt_eval_launch(const tci_core_ref* cores, int* cls, int L, int rmax, const uint8_t* pts, int64_t np,
                                double* out, int num_sms, cudaStream_t st);
@@ -268,6 +270,9 @@ int Engine::init() {
   if (const char* s = std::getenv("TCI_PLAN_SMEM")) plan_limit_ = (size_t)std::max(1024L, std::atol(s));
   CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device_));
   CUDA_TRY(cudaMalloc(&dcounter_, 64));
+  int pageable = 0;
+  CUDA_TRY(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device_));
+  host_direct_ = pageable != 0;
   cudaMemPool_t pool;
   CUDA_TRY(cudaDeviceGetDefaultMemPool(&pool, device_));
   uint64_t thr = UINT64_MAX;
@@ -577,7 +582,7 @@ int Engine::launch() {
     o_cores[i] = off;
     off = a16(off + (size_t)r.ncores * sizeof(tci_core_ref));
     o_ain[i] = off;
-    if (r.ain_host) off = a16(off + (size_t)r.t.m * r.t.n * 8);
+    if (r.ain_host && !host_direct_) off = a16(off + (size_t)r.t.m * r.t.n * 8);
     o_res[i] = res_total;
     r.res_bytes = result_bytes(r.t);
     res_total += r.res_bytes;
@@ -615,7 +620,9 @@ int Engine::launch() {
     t.res = (int64_t)o_res[i];
     t.work = nullptr;  // the kernel points it (and a per-task table) into its CTA's area
     if (!t.lut_full) t.lut = nullptr;
-    if (r.ain_host) t.ain = (const double*)(dblob_ + o_ain[i]);
+    // a given matrix is read once: in place across the host link (190 GB/s, against
+    // 14 for one thread copying it to the upload buffer) where the device can
+    if (r.ain_host) t.ain = host_direct_ ? r.ain_host : (const double*)(dblob_ + o_ain[i]);
     t.cost = task_cost(t);
     tasks[i] = t;
     if (t.nparams) std::memcpy(hblob_ + o_params[i], r.params, (size_t)t.nparams * 8);
@@ -623,7 +630,7 @@ int Engine::launch() {
     if (r.cols_bytes) std::memcpy(hblob_ + o_cols[i], r.cols, r.cols_bytes);
     if (r.prows_bytes) std::memcpy(hblob_ + o_prows[i], r.prows, r.prows_bytes);
     if (r.ncores) std::memcpy(hblob_ + o_cores[i], r.cores, (size_t)r.ncores * sizeof(tci_core_ref));
-    if (r.ain_host) std::memcpy(hblob_ + o_ain[i], r.ain_host, (size_t)r.t.m * r.t.n * 8);
+    if (r.ain_host && !host_direct_) std::memcpy(hblob_ + o_ain[i], r.ain_host, (size_t)r.t.m * r.t.n * 8);
   }
   int* order = (int*)(hblob_ + off_order);
   std::iota(order, order + nt, 0);
@@ -1899,8 +1906,72 @@ CoTask co_evaluate(Engine& e, Solve& s, const uint8_t* pts, i64 np, double* fout
   co_return 0;
 }
 
-// Train values alone at np points (packed, 0-based): one launch over all of them.
-int Engine::eval_train(const Solve& s, const uint8_t* pts, int64_t np, double* out) {
+// Points (np x L, row-major, 1-based int64) -> flat 0-based uint8 multi-indices,
+// range-checked; large inputs are split over host threads.
+int pack_points(const int64_t* pts, int64_t np, int L, const std::vector<int>& d, std::vector<uint8_t>& out) {
+  out.resize((size_t)np * (size_t)L);
+  auto run = [&](int64_t p0, int64_t p1) {
+    bool ok = true;
+    for (int64_t p = p0; p < p1; ++p) {
+      const int64_t* x = pts + p * L;
+      uint8_t* o = out.data() + (size_t)p * L;
+      for (int q = 0; q < L; ++q) {
+        ok &= x[q] >= 1 && x[q] <= d[q];
+        o[q] = (uint8_t)(x[q] - 1);
+      }
+    }
+    return ok;
+  };
+  const int64_t work = np * (int64_t)L;
+  int nt = work >= (1 << 22) ? (int)std::min<int64_t>(8, std::max(1u, std::thread::hardware_concurrency())) : 1;
+  bool ok = true;
+  if (nt == 1) {
+    ok = run(0, np);
+  } else {
+    std::vector<std::thread> th;
+    std::vector<char> res(nt, 1);
+    const int64_t per = (np + nt - 1) / nt;
+    for (int t = 0; t < nt; ++t)
+      th.emplace_back([&, t] { res[t] = run(std::min(np, t * per), std::min(np, (t + 1) * per)); });
+    for (auto& x : th) x.join();
+    for (char r : res) ok &= r != 0;
+  }
+  if (!ok) return fail(TCI_ERR_ARG, "pivot index out of range");
+  return 0;
+}
+
+// Values below which the host packs points itself (a launch costs more).
+static constexpr int64_t PACK_DIRECT = 1 << 16;
+
+int Engine::upload_points(const Solve& s, const int64_t* points, int64_t np, uint8_t* dev_pts) {
+  const int L = s.L;
+  if (!host_direct_ || np * L < PACK_DIRECT) {
+    std::vector<uint8_t> pts;
+    int rc = pack_points(points, np, L, s.d, pts);
+    if (rc) return rc;
+    CUDA_TRY(cudaMemcpyAsync(dev_pts, pts.data(), pts.size(), cudaMemcpyHostToDevice, stream_));
+    CUDA_TRY(cudaStreamSynchronize(stream_));  // pts goes away
+    return 0;
+  }
+  int* scratch = (int*)alloc_core(((size_t)L + 1 + 1) / 2);
+  if (!scratch) return fail(TCI_ERR_OOM, "device memory for the points");
+  std::vector<int> dims(s.d);
+  dims.push_back(0);  // the flag
+  cudaError_t ce = cudaMemcpyAsync(scratch, dims.data(), dims.size() * sizeof(int), cudaMemcpyHostToDevice, stream_);
+  if (ce == cudaSuccess)
+    ce = tci_pack_points_launch(points, np, L, scratch, dev_pts, scratch + L, num_sms, stream_);
+  int bad = 0;
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&bad, scratch + L, sizeof(int), cudaMemcpyDeviceToHost, stream_);
+  const cudaError_t sync = cudaStreamSynchronize(stream_);
+  free_core((double*)scratch);
+  if (ce == cudaSuccess) ce = sync;
+  if (ce != cudaSuccess) return fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
+  stats.launches += 1;
+  return bad ? fail(TCI_ERR_ARG, "pivot index out of range") : 0;
+}
+
+// Train values alone at np points: one launch over all of them.
+int Engine::eval_train(const Solve& s, const int64_t* points, int64_t np, double* out) {
   if (fc_callback_depth()) return reentry();
   if (!s.cores_valid) return fail(TCI_ERR_GENERIC, "site tensors are not available");
   if (np <= 0) return 0;
@@ -1913,8 +1984,11 @@ int Engine::eval_train(const Solve& s, const uint8_t* pts, int64_t np, double* o
                o_pts = o_out + a16((size_t)np * 8), total = o_pts + (size_t)np * L;
   char* d = (char*)alloc_core((total + 7) / 8);
   if (!d) return fail(TCI_ERR_OOM, "device memory for evaluation");
+  if (const int rc = upload_points(s, points, np, (uint8_t*)(d + o_pts))) {
+    free_core((double*)d);
+    return rc;
+  }
   cudaError_t ce = cudaMemcpyAsync(d, tab.data(), L * sizeof(tci_core_ref), cudaMemcpyHostToDevice, stream_);
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(d + o_pts, pts, (size_t)np * L, cudaMemcpyHostToDevice, stream_);
   if (ce == cudaSuccess && timing) ce = cudaEventRecord(ev0_, stream_);
   if (ce == cudaSuccess)
     ce = tci_tt_eval_launch((const tci_core_ref*)d, (int*)(d + o_cls), s.L, rmax, (const uint8_t*)(d + o_pts), np,

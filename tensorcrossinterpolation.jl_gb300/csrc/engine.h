@@ -290,8 +290,15 @@ class Engine {
   int run_tasks(std::vector<Req*>& reqs);
   int run_big(Req& r);
   int run_cluster(Req& r, int ncta);
-  // evaluate(tt, points) for np packed 0-based points (np x L) of the solve's train.
-  int eval_train(const Solve& s, const uint8_t* pts, int64_t np, double* out);
+  // Kernels may read the caller's pageable host memory (coherent host link): large
+  // inputs are then taken in place instead of through host-side copies.
+  bool host_direct() const { return host_direct_; }
+  // Points (np x L, 1-based, host) as bytes into dev_pts (device), range-checked:
+  // packed on the device from the caller's memory, or on the host where that is
+  // small or not readable.  Waits for the check.
+  int upload_points(const Solve& s, const int64_t* points, int64_t np, uint8_t* dev_pts);
+  // evaluate(tt, points) for np points (np x L, 1-based) of the solve's train.
+  int eval_train(const Solve& s, const int64_t* points, int64_t np, double* out);
   // Copy many device arrays to one host buffer: gather on the device into a
   // contiguous staging buffer, then a single device-to-host copy.
   int gather_to_host(const std::vector<const double*>& src, const std::vector<int64_t>& len,
@@ -304,6 +311,7 @@ class Engine {
   bool timing = true;
   const tci_kernel_set* ks_ = &tci_k256::kernels;  // the variant of the current / last batched launch
   int num_sms = 0;
+  bool host_direct_ = false;
   size_t hbm_budget = 0;
   // Autotuned rrLU parameter per (rows, cols) bucket: the trailing-block size
   // (elements) at which a factorization continues on one warp instead of the
@@ -382,6 +390,10 @@ class Engine {
   std::vector<size_t> fl_o_res_;
   std::vector<char> fl_smem_;
 };
+
+// Points (np x L, row-major, 1-based int64) -> flat 0-based uint8 multi-indices,
+// range-checked.
+int pack_points(const int64_t* pts, int64_t np, int L, const std::vector<int>& d, std::vector<uint8_t>& out);
 
 // ------------------------------------------------------------ TCI2 algorithm
 // A solve whose f is the library's own evaluator (values through the device cache).

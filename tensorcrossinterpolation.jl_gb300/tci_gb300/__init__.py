@@ -1326,6 +1326,22 @@ class rrLU:
         return self.error
 
 
+def _own_copy(a):
+    """a.copy(); of a large matrix by four threads, a block of rows each (numpy
+    copies without the GIL): transposing 8 MB takes one thread 1.8 ms."""
+    if a.size < 1 << 18 or a.shape[0] < 4:
+        return a.copy()
+    out = np.empty(a.shape, a.dtype)
+    rows = [a.shape[0] * q // 4 for q in range(5)]
+    th = [threading.Thread(target=np.copyto, args=(out[r0:r1], a[r0:r1])) for r0, r1 in zip(rows[1:], rows[2:])]
+    for t in th:
+        t.start()
+    np.copyto(out[: rows[1]], a[: rows[1]])
+    for t in th:
+        t.join()
+    return out
+
+
 def rrlu(A, maxrank=None, reltol=1e-14, abstol=0.0, leftorthogonal=True, ctx=None):
     """rrlu(A; maxrank, reltol, abstol, leftorthogonal) (matrixlu.jl:217-225) on the GPU."""
     ctx = ctx or default_context()
@@ -1343,23 +1359,29 @@ def rrlu(A, maxrank=None, reltol=1e-14, abstol=0.0, leftorthogonal=True, ctx=Non
                                    abstol, int(bool(leftorthogonal)), _p(rp, I64P), _p(cp, I64P), _p(Lb, F64P),
                                    _p(Ub, F64P), ctypes.byref(npiv), ctypes.byref(err)))
     K = npiv.value
-    return rrLU(rp, cp, Lb[: m * K].reshape((m, K), order="F").copy(), Ub[: K * n].reshape((K, n), order="F").copy(),
-                bool(leftorthogonal), K, err.value)
+    return rrLU(rp, cp, _own_copy(Lb[: m * K].reshape((m, K), order="F")),
+                _own_copy(Ub[: K * n].reshape((K, n), order="F")), bool(leftorthogonal), K, err.value)
 
 
 def rrlu_batched(mats, maxrank=None, reltol=1e-14, abstol=0.0, leftorthogonal=True, ctx=None):
     """Many independent rrLUs in one launch -> list of (rows, cols, npivot, error), 1-based."""
     ctx = ctx or default_context()
-    ms = np.array([a.shape[0] for a in mats], np.int64)
-    ns = np.array([a.shape[1] for a in mats], np.int64)
-    offs = np.concatenate([[0], np.cumsum(ms * ns)[:-1]]).astype(np.int64)
-    flat = np.ascontiguousarray(np.concatenate([np.asarray(a, np.float64).reshape(-1, order="F") for a in mats]))
+    if not len(mats):
+        raise ValueError("need at least one matrix")
+    # the matrices where they are (column-major float64; others are copied): their
+    # places relative to the lowest one, in doubles
+    cols = [np.require(a, np.float64, ["F", "A"]) for a in mats]
+    ms = np.array([a.shape[0] for a in cols], np.int64)
+    ns = np.array([a.shape[1] for a in cols], np.int64)
+    addr = np.array([a.ctypes.data for a in cols], np.int64)
+    base = int(addr.min())
+    offs = np.ascontiguousarray((addr - base) // 8)
     kcap = np.minimum(np.minimum(ms, ns), maxrank if maxrank else np.iinfo(np.int64).max)
     poffs = np.concatenate([[0], np.cumsum(2 * kcap)[:-1]]).astype(np.int64)
     piv = np.zeros(int(2 * kcap.sum()) + 1, np.int64)
     npiv = np.zeros(len(mats), np.int64)
     errs = np.zeros(len(mats))
-    _check(load_library().tci_rrlu_batched(ctx.h, len(mats), _p(flat, F64P), _p(offs, I64P), _p(ms, I64P),
+    _check(load_library().tci_rrlu_batched(ctx.h, len(mats), ctypes.cast(base, F64P), _p(offs, I64P), _p(ms, I64P),
                                            _p(ns, I64P), 0 if maxrank is None else int(maxrank), reltol, abstol,
                                            int(bool(leftorthogonal)), _p(piv, I64P), _p(poffs, I64P),
                                            _p(npiv, I64P), _p(errs, F64P)))
