@@ -31,6 +31,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "tc_gemm.h"
 
@@ -467,13 +468,25 @@ namespace {
 constexpr int EV_EPI_THREADS = 128;
 constexpr int EV_THREADS = 192;
 constexpr int EV_RMAX = 128;                       // bond limit
-constexpr int EV_KC_MAX = EV_RMAX / BK;            // 4 chunks of 32
 constexpr int EV_CHUNK_BYTES = BM * 128;           // 16 KB: 128 rows x 128 B
 constexpr int EV_STAGES = 2;
-constexpr int EV_IMG_MAX = EV_RMAX * 128;          // one image: r1p rows x 128 B
-constexpr int EV_STAGE_BYTES = 2 * EV_IMG_MAX;     // hi + lo
-constexpr int EV_V_BYTES = 2 * EV_KC_MAX * EV_CHUNK_BYTES;  // hi chunks then lo chunks
-constexpr int EV_SMEM = 1024 + EV_V_BYTES + EV_STAGES * EV_STAGE_BYTES + 256;
+constexpr int EV_CTAS = 5;                         // CTAs per SM at most (shared memory: 42 KB at the least)
+
+// What a CTA takes of its SM, by the train's largest bonds.  Each site is a chain
+// (MMAs, read-back, split, write, fence: 2.9 us) with the tensor cores idle in
+// between; small bonds leave room for several CTAs per SM, whose chains overlap.
+// A call with a million points, 40 sites, bonds of 12: 13.6 ms with one CTA per SM,
+// 4.7 with three, 4.2 with four, 3.8 with five; 100,000 points, bonds of 40, three
+// digits (two CTAs): 6.6 -> 3.4 ms; bonds of 128 (one CTA): 6.2 -> 5.0 ms, since
+// MMA steps past a bond's end are left out.
+struct EvLayout {
+  int kc;            // 32-deep chunks of the running vectors
+  uint32_t img;      // bytes of one core image (r1p rows x 128 B)
+  uint32_t cols;     // tensor-memory columns (a power of two)
+  __host__ __device__ uint32_t v_bytes() const { return 2u * (uint32_t)kc * EV_CHUNK_BYTES; }  // hi chunks, lo chunks
+  __host__ __device__ uint32_t stage_bytes() const { return 2u * img; }                        // hi + lo
+  __host__ __device__ uint32_t smem() const { return 1024 + v_bytes() + EV_STAGES * stage_bytes() + 256; }
+};
 
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -543,15 +556,15 @@ struct EvSite {
   int r0, d, r1, r1p, nkc;
 };
 
-__global__ void __launch_bounds__(EV_THREADS, 1)
-    tc_eval_kernel(const EvSite* __restrict__ sites, int L, const uint8_t* __restrict__ pts, int64_t np,
-                   double* __restrict__ out, int* err) {
+__global__ void __launch_bounds__(EV_THREADS, EV_CTAS)
+    tc_eval_kernel(const EvSite* __restrict__ sites, int L, const EvLayout Y, const uint8_t* __restrict__ pts,
+                   int64_t np, double* __restrict__ out, int* err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* V = base;                               // hi chunks [0, 4), lo chunks [4, 8)
-  uint8_t* stages = base + EV_V_BYTES;
+  uint8_t* V = base;  // hi chunks, then lo chunks
+  uint8_t* stages = base + Y.v_bytes();
   // full[2], empty[2], d_full, v_ready, mma_end
-  uint64_t* bars = (uint64_t*)(stages + EV_STAGES * EV_STAGE_BYTES);
+  uint64_t* bars = (uint64_t*)(stages + EV_STAGES * Y.stage_bytes());
   uint32_t* tmem_slot = (uint32_t*)(bars + 2 * EV_STAGES + 3);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + EV_STAGES);
@@ -568,7 +581,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(512)
+                 "r"(Y.cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -594,10 +607,10 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
               }
               const uint32_t fb = full0 + 8 * s;
               const uint8_t* src = S.img + (int64_t)((i * S.nkc + kc) * 2) * img_bytes;
-              const uint32_t dst = smem_u32(stages + s * EV_STAGE_BYTES);
+              const uint32_t dst = smem_u32(stages + s * Y.stage_bytes());
               mbar_expect_tx(fb, 2 * img_bytes);
               bulk_copy(dst, src, img_bytes, fb);
-              bulk_copy(dst + EV_IMG_MAX, src + img_bytes, img_bytes, fb);
+              bulk_copy(dst + Y.img, src + img_bytes, img_bytes, fb);
             }
         }
       for (int j = it - EV_STAGES; j < it; ++j)  // in-flight copies land before the CTA leaves
@@ -616,7 +629,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t idesc = tf32_idesc(BM, S.r1p);
-          const uint32_t vh = smem_u32(V), vl = smem_u32(V + EV_KC_MAX * EV_CHUNK_BYTES);
+          const uint32_t vh = smem_u32(V), vl = smem_u32(V + Y.kc * EV_CHUNK_BYTES);
           for (int i = 0; i < S.d && ok; ++i) {
             const uint32_t dcol = tmem + (uint32_t)(i * S.r1p);
             for (int kc = 0; kc < S.nkc; ++kc, ++it) {
@@ -626,10 +639,10 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
                 break;
               }
               tc_fence_after();
-              const uint32_t bh = smem_u32(stages + s * EV_STAGE_BYTES), bl = bh + EV_IMG_MAX;
+              const uint32_t bh = smem_u32(stages + s * Y.stage_bytes()), bl = bh + Y.img;
               const uint32_t ah = vh + kc * EV_CHUNK_BYTES, al = vl + kc * EV_CHUNK_BYTES;
-#pragma unroll
-              for (int kk = 0; kk < BK / KSUB; ++kk) {
+              const int nkk = (min(S.r0 - kc * BK, BK) + KSUB - 1) / KSUB;  // past r0 both sides are zeros
+              for (int kk = 0; kk < nkk; ++kk) {
                 const uint32_t ko = kk * KSUB * 4;
                 mma_tf32(dcol, sw128_desc(al + ko), sw128_desc(bh + ko), idesc, (kc > 0 || kk > 0) ? 1u : 0u);
                 mma_tf32(dcol, sw128_desc(ah + ko), sw128_desc(bl + ko), idesc, 1u);
@@ -649,7 +662,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
     const int row = threadIdx.x;
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
     uint8_t* Vh = V;
-    uint8_t* Vl = V + EV_KC_MAX * EV_CHUNK_BYTES;
+    uint8_t* Vl = V + Y.kc * EV_CHUNK_BYTES;
     int site_it = 0;
     bool ok = true;
     for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
@@ -664,7 +677,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
         if (L == 1) {
           if (live) out[p] = S.core[i0];
         } else {
-          const int kp = sites[1].nkc * 32;
+          const int kp = (r1 + KSUB - 1) / KSUB * KSUB;  // to the next MMA step's edge
           for (int c = 0; c < kp; ++c) {
             const double v = (live && c < r1) ? S.core[i0 + (int64_t)S.d * c] : 0.0;
             float hi, lo;
@@ -680,13 +693,13 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
       }
       for (int b = 1; b < L; ++b, ++site_it) {
         const EvSite S = sites[b];
+        const int ib = live ? ip[b] : 0;  // ahead of the wait
         const bool have = mbar_wait(d_full, (uint32_t)site_it & 1u, err, 15);
         if (!__all_sync(0xffffffffu, have)) {
           ok = false;  // a wait ran out: stop this warp (the others time out too)
           break;
         }
         tc_fence_after();
-        const int ib = live ? ip[b] : 0;
         if (b == L - 1) {
           // r1 = 1: column 0 of the point's block
           float acc = 0.f;
@@ -698,7 +711,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
             }
           if (live) out[p] = (double)acc;
         } else {
-          const int kp = sites[b + 1].nkc * 32;  // next site's padded input bond
+          const int kp = (S.r1 + KSUB - 1) / KSUB * KSUB;  // zeros up to the next MMA step's edge
           for (int c = 0; c < S.r1p; c += 16) {
             float sel[16];
 #pragma unroll
@@ -724,11 +737,6 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
               }
             }
           }
-          for (int col = S.r1p; col < kp; ++col) {  // zero padding up to the next chunk edge
-            const uint32_t o = (uint32_t)(col >> 5) * EV_CHUNK_BYTES + sw128_off(row, col & 31);
-            *(float*)(Vh + o) = 0.f;
-            *(float*)(Vl + o) = 0.f;
-          }
           tc_fence_before();
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           mbar_arrive(v_ready);
@@ -740,7 +748,7 @@ __global__ void __launch_bounds__(EV_THREADS, 1)
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Y.cols) : "memory");
   }
 }
 
@@ -821,15 +829,28 @@ cudaError_t tci_tc_evaluate_split(int L, const int64_t* dims, const double* cons
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(cptr_dev, cores_dev, (size_t)L * sizeof(double*), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
-  static bool attr = false;
-  if (!attr) {
-    e = cudaFuncSetAttribute(tc_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EV_SMEM);
+  EvLayout Y{1, 16 * 128, 32};
+  for (int b = 1; b < L; ++b) {
+    Y.kc = std::max(Y.kc, host[b].nkc);
+    Y.img = std::max<uint32_t>(Y.img, (uint32_t)host[b].r1p * 128);
+    while (Y.cols < (uint32_t)(host[b].d * host[b].r1p)) Y.cols *= 2;
+  }
+  // CTAs per SM by tensor memory (512 columns) and shared memory; each asks for an
+  // equal share of the latter, so that no SM takes one more than tensor memory has
+  // room for (its allocation would wait for another CTA's end).
+  constexpr uint32_t SM_BYTES = 227 * 1024;
+  int per_sm = (int)std::min<uint32_t>(EV_CTAS, 512 / Y.cols);
+  while (per_sm > 1 && Y.smem() + 1024 > SM_BYTES / per_sm) --per_sm;
+  const uint32_t smem = std::max(Y.smem(), SM_BYTES / per_sm - 1024 - (per_sm > 1 ? 1024u : 0u));
+  static std::atomic<uint32_t> limit{0};
+  if (limit.load() < smem) {
+    e = cudaFuncSetAttribute(tc_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_BYTES);
     if (e != cudaSuccess) return e;
-    attr = true;
+    limit.store(SM_BYTES);
   }
   const int64_t ntiles = (np + BM - 1) / BM;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, nsm));
-  if (np > 0) tc_eval_kernel<<<grid, EV_THREADS, EV_SMEM, st>>>(sites_dev, L, pts_dev, np, out_dev, err_dev);
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)nsm * per_sm));
+  if (np > 0) tc_eval_kernel<<<grid, EV_THREADS, smem, st>>>(sites_dev, L, Y, pts_dev, np, out_dev, err_dev);
   if (nsample > 0)
     ev_fp64_kernel<<<(nsample + 63) / 64, 64, 0, st>>>(sites_dev, cptr_dev, L, pts_dev, nsample, sample_out_dev);
   return cudaGetLastError();
