@@ -30,6 +30,7 @@
 #include <mutex>
 #include <stddef.h>
 #include <stdint.h>
+#include <type_traits>
 #include <string>
 
 #include "ieee_int.h"
@@ -349,26 +350,72 @@ __device__ __forceinline__ char* atw(char* base, int64_t off) { return (char*)((
 __device__ __forceinline__ bool int_states(const tci_task& T) {
   return tci_f_tables(T.fid) > 0 && T.lut != nullptr && T.lutcap0 > 0;
 }
-__device__ void compute_states(const tci_task& T, const double* params, const uint8_t* idx, int count, int len,
-                               int site0, double* s0, double* s1) {
-  if (int_states(T)) {
-    long long* q0 = (long long*)s0;
-    long long* q1 = (long long*)s1;
-    for (int i = threadIdx.x; i < count; i += NT) {
-      long long a0 = 0, a1 = 0;
-      const uint8_t* v = idx + (size_t)i * len;
-      for (int p = 0; p < len; ++p) tci_f_term_int(T.fid, params, site0 + p, v[p], &a0, &a1);
-      q0[i] = a0;
-      q1[i] = a1;
+// The registered f of its two sums, and the sums of `len` sites from site0 on with
+// local values v (site `over` of them taken as `val`).  Out of line: a task's fills,
+// states and points share one copy of the code, which a small task would otherwise
+// wait for more than once.
+__device__ __noinline__ double f_finish(int fid, const double* prm, int nparams, double a0, double a1) {
+  return tci_f_finish(fid, prm, nparams, a0, a1);
+}
+struct FSums {
+  double a0, a1;
+};
+__device__ __noinline__ FSums f_sums(int fid, const double* prm, int site0, int len, const uint8_t* v, int over,
+                                     int val) {
+  FSums a{0.0, 0.0};
+  if ((fid == TCI_F_QTT1D || fid == TCI_F_QTT2D) && len <= 53 && site0 + len <= 1022) {
+    // binary digits: every partial sum is exact, so they are collected as an
+    // integer (an FP64 addition per site takes a warp 64 cycles of its SM quarter)
+    unsigned long long q0 = 0, q1 = 0;
+    for (int p = 0; p < len; ++p) {
+      const int d = p == over ? val : v[p];
+      q0 = 2 * q0 + (fid == TCI_F_QTT1D ? d != 0 : d & 1);
+      q1 = 2 * q1 + (d >> 1 & 1);
     }
-    return;
+    const double ulp = tci_pow2i(-(site0 + len));
+    a.a0 = (double)q0 * ulp;
+    if (fid == TCI_F_QTT2D) a.a1 = (double)q1 * ulp;
+  } else {
+    for (int p = 0; p < len; ++p) tci_f_term(fid, prm, site0 + p, p == over ? val : v[p], &a.a0, &a.a1);
   }
-  for (int i = threadIdx.x; i < count; i += NT) {
-    double a0 = 0.0, a1 = 0.0;
-    const uint8_t* v = idx + (size_t)i * len;
-    for (int p = 0; p < len; ++p) tci_f_term(T.fid, params, site0 + p, v[p], &a0, &a1);
-    s0[i] = a0;
-    s1[i] = a1;
+  return a;
+}
+
+// A list of `count` multi-indices of `len` sites from site0 on, and where their
+// two sums go.
+struct StateList {
+  const uint8_t* idx;
+  int count, len, site0;
+  double *s0, *s1;
+};
+// All lists in one pass over the CTA's threads: of a small task each list has a
+// few entries, and one after the other would use a warp at a time.
+template <int G>
+__device__ void compute_states(const tci_task& T, const double* params, const StateList (&g)[G]) {
+  int total = 0;
+#pragma unroll
+  for (int k = 0; k < G; ++k) total += g[k].count;
+  const bool ints = int_states(T);
+  for (int e = threadIdx.x; e < total; e += NT) {
+    StateList l = g[0];
+    int i = e;
+#pragma unroll
+    for (int k = 1; k < G; ++k)
+      if (i >= l.count) {
+        i -= l.count;
+        l = g[k];
+      }
+    const uint8_t* v = l.idx + (size_t)i * l.len;
+    if (ints) {
+      long long a0 = 0, a1 = 0;
+      for (int p = 0; p < l.len; ++p) tci_f_term_int(T.fid, params, l.site0 + p, v[p], &a0, &a1);
+      ((long long*)l.s0)[i] = a0;
+      ((long long*)l.s1)[i] = a1;
+    } else {
+      const FSums a = f_sums(T.fid, params, l.site0, l.len, v, -1, 0);
+      l.s0[i] = a.a0;
+      l.s1[i] = a.a1;
+    }
   }
 }
 
@@ -378,22 +425,26 @@ __device__ void compute_states(const tci_task& T, const double* params, const ui
 // T.lut and each element is combine_scaled(table0[s0], table1[s1]) -- one FP64
 // operation; the direct path computes the same functions, so the bits are
 // identical.
+using At1 = std::integral_constant<int, 1>;  // elements taken at once by a fill's loop
+using At4 = std::integral_constant<int, 4>;
 struct Filler {
   int fid, nparams;
   const double* prm;
   const double* lut0;
   const double* lut1;
   int lo0, lo1;
-  // element (i, j) from row states r0/r1 and column states c0/c1
+  // element (i, j) from row states r0/r1 and column states c0/c1: from the tables, or either way
+  __device__ __forceinline__ double tab(const double* r0, const double* r1, int i, const double* c0,
+                                        const double* c1, int j) const {
+    const double p0 = lut0[(int)(((const long long*)r0)[i] + ((const long long*)c0)[j]) - lo0];
+    if (!lut1) return p0;
+    const double q1 = lut1[(int)(((const long long*)r1)[i] + ((const long long*)c1)[j]) - lo1];
+    return tci_f_combine_scaled(fid, p0, q1);
+  }
   __device__ __forceinline__ double val(const double* r0, const double* r1, int i, const double* c0,
                                         const double* c1, int j) const {
-    if (lut0) {
-      const double p0 = lut0[(int)(((const long long*)r0)[i] + ((const long long*)c0)[j]) - lo0];
-      if (!lut1) return p0;
-      const double q1 = lut1[(int)(((const long long*)r1)[i] + ((const long long*)c1)[j]) - lo1];
-      return tci_f_combine_scaled(fid, p0, q1);
-    }
-    return tci_f_finish(fid, prm, nparams, r0[i] + c0[j], r1[i] + c1[j]);
+    if (lut0) return tab(r0, r1, i, c0, c1, j);
+    return f_finish(fid, prm, nparams, r0[i] + c0[j], r1[i] + c1[j]);
   }
 };
 
@@ -1062,24 +1113,39 @@ __device__ void task_rrlu(const tci_task& T, const char* blob, char* resb, char*
     double* rs1 = st ? st + m : (double*)cur.take((size_t)m * 8);
     double* cs0 = st ? st + 2 * (size_t)m : (double*)cur.take((size_t)n * 8);
     double* cs1 = st ? st + 2 * (size_t)m + n : (double*)cur.take((size_t)n * 8);
-    compute_states(T, prm, (const uint8_t*)at(blob, T.rows), m, T.nl, 0, rs0, rs1);
-    compute_states(T, prm, (const uint8_t*)at(blob, T.cols), n, T.nr, T.nl, cs0, cs1);
+    compute_states(T, prm, {{(const uint8_t*)at(blob, T.rows), m, T.nl, 0, rs0, rs1},
+                            {(const uint8_t*)at(blob, T.cols), n, T.nr, T.nl, cs0, cs1}});
     __syncthreads();
     double* const rg0[1] = {rs0};
     double* const rg1[1] = {rs1};
     const int rc[1] = {m};
     const Filler F = make_filler(T, prm, rg0, rg1, rc, 1, cs0, cs1, n, (int64_t)m * n, ctl);
     lut_used = F.lut0 != nullptr;
-    for (int j = warp; j < n; j += NW) {
-      double* dst = A + (size_t)j * lda;
-      for (int i = lane; i < m; i += 32) {
-        double v = F.val(rs0, rs1, i, cs0, cs1, j);
-        dst[i] = v;
+    // consecutive elements over the CTA: f's FP64 chains cost a warp the same with
+    // one lane or 32 (7 x 7 of a 40-site quantics function: 16.6k cycles with a
+    // column per warp, 9.8k so, 6.8k with tci_math.h's short forms)
+    const auto loop = [&](const auto& element, auto together) {
+      const int sq = NT / m, sr = NT - sq * m, total = m * n;
+      int j = tid / m, i = tid - j * m;
+#pragma unroll decltype(together)::value
+      for (int e = tid; e < total; e += NT) {
+        const double v = element(i, j);
+        A[e] = v;
         am.push(v, pack_key(i, j));
-        unsigned long long b = abs_bits(v);
+        const unsigned long long b = abs_bits(v);
         mx = b > mx ? b : mx;
+        i += sr;
+        j += sq;
+        if (i >= m) {
+          i -= m;
+          j += 1;
+        }
       }
-    }
+    };
+    if (F.lut0)
+      loop([&](int i, int j) { return F.tab(rs0, rs1, i, cs0, cs1, j); }, At4{});
+    else
+      loop([&](int i, int j) { return F.val(rs0, rs1, i, cs0, cs1, j); }, At1{});
   }
   __syncthreads();
   unsigned long long mxall = block_max_u64(mx, ctl);
@@ -1342,21 +1408,43 @@ __device__ void task_site(const tci_task& T, const char* blob, char* resb, char*
   // the row f states: on chip, or after P in global scratch
   double* rs0 = T.smem_mode == 2 ? T.work + (size_t)r * r : (double*)cur.take((size_t)m * 8);
   double* rs1 = T.smem_mode == 2 ? T.work + (size_t)r * r + m : (double*)cur.take((size_t)m * 8);
-  compute_states(T, prm, (const uint8_t*)at(blob, T.prows), r, T.nl, 0, ps0, ps1);
-  compute_states(T, prm, (const uint8_t*)at(blob, T.cols), r, T.nr, T.nl, cs0, cs1);
-  compute_states(T, prm, (const uint8_t*)at(blob, T.rows), m, T.nl, 0, rs0, rs1);
+  compute_states(T, prm, {{(const uint8_t*)at(blob, T.prows), r, T.nl, 0, ps0, ps1},
+                          {(const uint8_t*)at(blob, T.cols), r, T.nr, T.nl, cs0, cs1},
+                          {(const uint8_t*)at(blob, T.rows), m, T.nl, 0, rs0, rs1}});
   __syncthreads();
   double* const rg0[2] = {ps0, rs0};
   double* const rg1[2] = {ps1, rs1};
   const int rc[2] = {r, m};
   const Filler F = make_filler(T, prm, rg0, rg1, rc, 2, cs0, cs1, r, (int64_t)(r + m) * r, ctl);
-  // A[i, j] = P[j, i] = f(prows[j] ++ cols[i])
-  for (int j = warp; j < r; j += NW)
-    for (int i = lane; i < r; i += 32) A[i + (size_t)j * r] = F.val(ps0, ps1, j, cs0, cs1, i);
-  __syncthreads();
+  uint64_t* rec = (uint64_t*)cur.take((size_t)r * 8);
+  size_t used = (size_t)(cur.p - smem);
+  int RB = (int)((smem_bytes > used ? smem_bytes - used : 0) / ((size_t)r * 8 + 8));
+  RB = RB > NT ? NT : RB;
+  RB = RB < 1 ? 1 : RB;
+  double* W = (double*)cur.take((size_t)RB * r * 8);
+  unsigned long long mx = 0;
+  int nanflag = 0;
+  // A[i, j] = P[j, i] = f(prows[j] ++ cols[i]) and, in the same pass, the first
+  // block of rows, W[rr, q] = f(rows[base + rr] ++ cols[q])
+  auto fill = [&](int base, int rows_here, int na) {
+    const int total = na + rows_here * r;
+    for (int e = tid; e < total; e += NT) {
+      const bool p = e < na;
+      const int f = p ? e : e - na, h = p ? r : rows_here, hi = f / h, lo = f - hi * h;
+      const double v = F.val(p ? ps0 : rs0, p ? ps1 : rs1, p ? hi : base + lo, cs0, cs1, p ? lo : hi);
+      if (p) {
+        A[f] = v;
+      } else {
+        W[lo + (size_t)hi * RB] = v;
+        const unsigned long long b = abs_bits(v);
+        mx = b > mx ? b : mx;
+      }
+    }
+    __syncthreads();
+  };
+  fill(0, min(RB, m), r * r);
   const int singular = site_getrf(A, r, ipiv, ctl);
   // reciprocals of the diagonal (int_divisor), for the back substitution of every row
-  uint64_t* rec = (uint64_t*)cur.take((size_t)r * 8);
   for (int j = tid; j < r; j += NT) rec[j] = int_divisor(A[j + (size_t)j * r]).R;
   // (up to one warp of rows per SM quarter: FP64 products, see row_axpy)
   for (int j = warp; j < r; j += NW) {
@@ -1366,23 +1454,10 @@ __device__ void task_site(const tci_task& T, const char* blob, char* resb, char*
     c = __reduce_max_sync(FULL, c);
     if (lane == 0) colcls[j] = c;
   }
-  size_t used = (size_t)(cur.p - smem);
-  int RB = (int)((smem_bytes > used ? smem_bytes - used : 0) / ((size_t)r * 8 + 8));
-  RB = RB > NT ? NT : RB;
-  RB = RB < 1 ? 1 : RB;
-  double* W = (double*)cur.take((size_t)RB * r * 8);
-  unsigned long long mx = 0;
-  int nanflag = 0;
+  __syncthreads();
   for (int base = 0; base < m; base += RB) {
     const int rows_here = min(RB, m - base);
-    for (int q = warp; q < r; q += NW)
-      for (int rr = lane; rr < rows_here; rr += 32) {
-        const double v = F.val(rs0, rs1, base + rr, cs0, cs1, q);
-        W[rr + (size_t)q * RB] = v;
-        const unsigned long long b = abs_bits(v);
-        mx = b > mx ? b : mx;
-      }
-    __syncthreads();
+    if (base > 0) fill(base, rows_here, 0);
     if (!singular) {
       for (int rr = tid; rr < rows_here; rr += NT) {
         double* w = W + rr;
@@ -1439,28 +1514,28 @@ __device__ void task_site(const tci_task& T, const char* blob, char* resb, char*
 
 // ---------------------------------------------------------------- CORE task
 __device__ void task_core(const tci_task& T, const char* blob, char* resb, char* smem, Ctl& ctl) {
-  const int m = T.m, n = T.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m = T.m, n = T.n, tid = threadIdx.x;
   const double* prm = (const double*)at(blob, T.params);
   SmemCursor cur{smem};
   double* rs0 = (double*)cur.take((size_t)m * 8);
   double* rs1 = (double*)cur.take((size_t)m * 8);
   double* cs0 = (double*)cur.take((size_t)n * 8);
   double* cs1 = (double*)cur.take((size_t)n * 8);
-  compute_states(T, prm, (const uint8_t*)at(blob, T.rows), m, T.nl, 0, rs0, rs1);
-  compute_states(T, prm, (const uint8_t*)at(blob, T.cols), n, T.nr, T.nl, cs0, cs1);
+  compute_states(T, prm, {{(const uint8_t*)at(blob, T.rows), m, T.nl, 0, rs0, rs1},
+                          {(const uint8_t*)at(blob, T.cols), n, T.nr, T.nl, cs0, cs1}});
   __syncthreads();
   double* const rg0[1] = {rs0};
   double* const rg1[1] = {rs1};
   const int rc[1] = {m};
   const Filler F = make_filler(T, prm, rg0, rg1, rc, 1, cs0, cs1, n, (int64_t)m * n, ctl);
   unsigned long long mx = 0;
-  for (int j = warp; j < n; j += NW)
-    for (int i = lane; i < m; i += 32) {
-      double v = F.val(rs0, rs1, i, cs0, cs1, j);
-      T.core_out[i + (size_t)j * m] = v;
-      unsigned long long b = abs_bits(v);
-      mx = b > mx ? b : mx;
-    }
+  for (int e = tid; e < m * n; e += NT) {
+    const int j = e / m, i = e - j * m;
+    const double v = F.val(rs0, rs1, i, cs0, cs1, j);
+    T.core_out[e] = v;
+    const unsigned long long b = abs_bits(v);
+    mx = b > mx ? b : mx;
+  }
   unsigned long long mxall = block_max_u64(mx, ctl);
   if (tid == 0) {
     tci_result_head* h = (tci_result_head*)(atw(resb, T.res));
@@ -1489,9 +1564,8 @@ __device__ void task_eval(const tci_task& T, const char* blob, char* resb, char*
   double* fout = (double*)(base + sizeof(tci_result_head));
   double* tout = fout + np;
   for (int p = tid; p < np; p += NT) {
-    double a0 = 0.0, a1 = 0.0;
-    for (int s = 0; s < L; ++s) tci_f_term(T.fid, prm, s, pts[(size_t)p * L + s], &a0, &a1);
-    fout[p] = tci_f_finish(T.fid, prm, T.nparams, a0, a1);
+    const FSums a = f_sums(T.fid, prm, 0, L, pts + (size_t)p * L, -1, 0);
+    fout[p] = f_finish(T.fid, prm, T.nparams, a.a0, a.a1);
   }
   if (T.cores && T.r <= EVAL_THREAD_RMAX) {
     // bonds up to EVAL_THREAD_RMAX: one thread per point (a warp per point would
@@ -1708,16 +1782,16 @@ __device__ void task_search(const tci_task& T, const char* blob, char* resb, cha
                                                        1, c.r0), env[roff[p] + b]));
       tout[it] = val;
     }
-    double a0 = 0.0, a1 = 0.0;
+    FSums a;
     if (tci_f_tables(T.fid) > 0) {  // the same sums, exact integers, off the FP64 pipe
       long long i0 = 0, i1 = 0;
       for (int s = 0; s < L; ++s) tci_f_term_int(T.fid, prm, s, s == p ? v : st[s], &i0, &i1);
-      a0 = (double)i0;
-      a1 = (double)i1;
+      a.a0 = (double)i0;
+      a.a1 = (double)i1;
     } else {
-      for (int s = 0; s < L; ++s) tci_f_term(T.fid, prm, s, s == p ? v : st[s], &a0, &a1);
+      a = f_sums(T.fid, prm, 0, L, st, p, v);
     }
-    fout[it] = tci_f_finish(T.fid, prm, T.nparams, a0, a1);
+    fout[it] = f_finish(T.fid, prm, T.nparams, a.a0, a.a1);
   }
   if (tid == 0) {
     tci_result_head* h = (tci_result_head*)base;
@@ -2912,22 +2986,26 @@ __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCt
   bt.init();
   unsigned long long mx = 0;
   if (nrb > 0 && ncb > 0) {
-    const int sq = CL_NT / nrb, sr = CL_NT - sq * nrb;
-    int u = tid / nrb, t = tid - u * nrb;
-#pragma unroll 4
-    for (int e = tid; e < nrb * ncb; e += CL_NT) {
-      const double v = fill(r0 + t, c0 + u);
-      B.col(u, rank)[t] = v;
-      mx = max(mx, (unsigned long long)abs_bits(v));
-      const uint32_t key = pack_key(r0 + t, c0 + u);
-      bt.push(v, key, key);
-      t += sr;
-      u += sq;
-      if (t >= nrb) {
-        t -= nrb;
-        u += 1;
+    // fill picks what gives an element and how many are taken at once, so that each
+    // kind has its own loop (loads overlap; f's call among them would part them)
+    fill([&](const auto& element, auto together) {
+      const int sq = CL_NT / nrb, sr = CL_NT - sq * nrb;
+      int u = tid / nrb, t = tid - u * nrb;
+#pragma unroll decltype(together)::value
+      for (int e = tid; e < nrb * ncb; e += CL_NT) {
+        const double v = element(r0 + t, c0 + u);
+        B.col(u, rank)[t] = v;
+        mx = max(mx, (unsigned long long)abs_bits(v));
+        const uint32_t key = pack_key(r0 + t, c0 + u);
+        bt.push(v, key, key);
+        t += sr;
+        u += sq;
+        if (t >= nrb) {
+          t -= nrb;
+          u += 1;
+        }
       }
-    }
+    });
   }
   PivotState S;
   S.init(P.reltol, P.abstol);
@@ -3299,7 +3377,9 @@ __global__ void __launch_bounds__(CL_NT, 1) rrlu_cluster_task_kernel(const tci_t
   tci_result_head* head = (tci_result_head*)(uintptr_t)T.res;
   ClusterResult r;
   if (T.ain) {
-    r = cluster_rrlu<false>(P, smem, ctl, [&](int i, int j) { return __ldcs(T.ain + i + (size_t)j * m); });
+    r = cluster_rrlu<false>(P, smem, ctl, [&](const auto& loop) {
+      loop([&](int i, int j) { return __ldcs(T.ain + i + (size_t)j * m); }, At4{});
+    });
   } else {
     const int nrb = max(0, min(m, r0 + mb) - r0), ncb = max(0, min(n, c0 + nb) - c0), nl = T.nl, nr = T.nr;
     double* rs0 = (double*)(smem + cluster_smem16(m, n, mb, nb));
@@ -3329,10 +3409,9 @@ __global__ void __launch_bounds__(CL_NT, 1) rrlu_cluster_task_kernel(const tci_t
         *(long long*)d0 = a0;
         *(long long*)d1 = a1;
       } else {
-        double a0 = 0.0, a1 = 0.0;
-        for (int p = 0; p < len; ++p) tci_f_term(T.fid, prm, site0 + p, v[p], &a0, &a1);
-        *d0 = a0;
-        *d1 = a1;
+        const FSums a = f_sums(T.fid, prm, site0, len, v, -1, 0);
+        *d0 = a.a0;
+        *d1 = a.a1;
       }
     }
     __syncthreads();
@@ -3344,7 +3423,12 @@ __global__ void __launch_bounds__(CL_NT, 1) rrlu_cluster_task_kernel(const tci_t
     F.lut1 = tables && tci_f_tables(T.fid) > 1 ? T.lut + T.lutcap0 : nullptr;
     F.lo0 = T.lut_base0;
     F.lo1 = 0;
-    r = cluster_rrlu<false>(P, smem, ctl, [&](int i, int j) { return F.val(rs0, rs1, i - r0, cs0, cs1, j - c0); });
+    r = cluster_rrlu<false>(P, smem, ctl, [&](const auto& loop) {
+      if (tables)
+        loop([&](int i, int j) { return F.tab(rs0, rs1, i - r0, cs0, cs1, j - c0); }, At4{});
+      else
+        loop([&](int i, int j) { return F.val(rs0, rs1, i - r0, cs0, cs1, j - c0); }, At1{});
+    });
   }
   if (rank != 0) return;
   __syncthreads();  // the record's arrays before its head
@@ -3494,7 +3578,9 @@ __global__ void __launch_bounds__(CL_NT, 1) rrlu_noalloc_cluster_kernel(const do
   __shared__ ClusterCtl ctl;
   const int m = P.m;
   const ClusterResult r =
-      cluster_rrlu<SPILL>(P, smem, ctl, [&](int i, int j) { return __ldcs(ain + i + (size_t)j * m); });
+      cluster_rrlu<SPILL>(P, smem, ctl, [&](const auto& loop) {
+        loop([&](int i, int j) { return __ldcs(ain + i + (size_t)j * m); }, At4{});
+      });
   if (cg::this_cluster().block_rank() == 0 && threadIdx.x == 0) {
     *O.npivot = r.K;
     *O.error = r.err;

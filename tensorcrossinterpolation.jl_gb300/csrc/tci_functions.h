@@ -13,6 +13,7 @@
 // index (the reference's index minus one).
 #pragma once
 #include "fc_slot.h"
+#include "ieee_int.h"
 #include "tci_math.h"
 
 enum {
@@ -48,6 +49,17 @@ enum {
 
 #define TCI_TWO_THOUSAND_PI 6283.185307179587   /* 2000*pi rounded to double */
 #define TCI_FOUR_HUNDRED_PI 1256.6370614359173  /* 400*pi rounded to double  */
+
+// a / b for a constant b, its significand and sign / exponent given: on the integer
+// pipes, where the device's FP64 division takes a warp as long as nine multiply-adds.
+TCI_HD IntDivisor tci_const_divisor(uint64_t mant, uint32_t se, uint64_t R) {
+  IntDivisor d;
+  d.mant = mant;
+  d.R = R;  // floor(2^116 / mant)
+  d.se = se;
+  return d;
+}
+TCI_HD double tci_quo(double a, double b, const IntDivisor& d) { return int_safe(a) ? int_div(a, d) : a / b; }
 
 TCI_HD void tci_f_term(int fid, const double* params, int site, int v,
                        double* acc0, double* acc1) {
@@ -150,12 +162,14 @@ TCI_HD double tci_f_finish(int fid, const double* params, int nparams, double ac
       double t1 = tci_exp(-x);
       double t2 = tci_cos(TCI_TWO_THOUSAND_PI * x);
       double dx = x - 0.3;
-      double t3 = tci_exp(-(dx * dx) / 1e-4);
+      double t3 = tci_exp(tci_quo(-(dx * dx), 1e-4, tci_const_divisor(0x001a36e2eb1c432dull, 0x3f100000u,
+                                                              0x9c3ffffffffffde4ull)));
       return t1 * t2 + 0.5 * t3;
     }
     case TCI_F_QTT2D: {
       double dx = acc0 - 0.5, dy = acc1 - 0.5;
-      double g = tci_exp(-(dx * dx + dy * dy) / 0.01);
+      double g = tci_exp(tci_quo(-(dx * dx + dy * dy), 0.01, tci_const_divisor(0x00147ae147ae147bull, 0x3f800000u,
+                                                                          0xc7fffffffffffed4ull)));
       return g * tci_cos(TCI_FOUR_HUNDRED_PI * (acc0 + acc1));
     }
     case TCI_F_DENSE: {

@@ -22,6 +22,15 @@
 // The Taylor coefficients are 1/k! rounded to double.  The split constants
 // were computed with 300-bit arithmetic (head = value truncated to 32 or 33
 // significant bits, tail = remainder rounded to double).
+//
+// On the device an FP64 instruction takes a warp 64 cycles of its SM quarter, with
+// one lane or 32, so the number of them is the cost.  In the usual range of
+// arguments the steps above are taken with fewer, to the same bits: range tests on
+// the bit patterns; rint by an addition that leaves the integer in the low word;
+// the exact products joined with their subtraction (one rounding either way); the
+// power of two added to the exponent; one chain of multiply-adds for sine and
+// cosine, each lane with its own coefficients.  exp 25 -> 19 instructions, cos with
+// mixed quadrants 58 -> 19.
 #pragma once
 #include <stdint.h>
 #include <math.h>
@@ -57,12 +66,14 @@ TCI_HD double tci_scale2(double p, int k) {
 #define TCI_PIO2_3 2.0222662487959506e-21
 #define TCI_TWO_OVER_PI 0.6366197723675814
 
-TCI_HD double tci_exp(double x) {
-  if (x != x) return x;
-  if (x > 709.782712893384) return tci_bits_to_double(0x7ff0000000000000ULL);
-  if (x < -745.1332191019412) return 0.0;
-  double n = rint(x * TCI_INV_LN2);
-  double r = (x - n * TCI_LN2_HI) - n * TCI_LN2_LO;
+// v rounded to an integer as rint does, |v| < 2^31 (a zero is +0).
+TCI_HD double tci_round(double v, uint32_t* low) {
+  const double t = v + 6755399441055744.0;  // 1.5 * 2^52: the sum's last place is 1
+  *low = (uint32_t)tci_double_to_bits(t);
+  return t - 6755399441055744.0;
+}
+
+TCI_HD double tci_exp_poly(double r) {
   double p = 1.6059043836821613e-10;           // 1/13!
   p = fma(p, r, 2.08767569878681e-09);         // 1/12!
   p = fma(p, r, 2.505210838544172e-08);        // 1/11!
@@ -76,8 +87,23 @@ TCI_HD double tci_exp(double x) {
   p = fma(p, r, 0.16666666666666666);          // 1/3!
   p = fma(p, r, 0.5);                          // 1/2!
   p = fma(p, r, 1.0);
-  p = fma(p, r, 1.0);
-  return tci_scale2(p, (int)n);
+  return fma(p, r, 1.0);
+}
+
+TCI_HD double tci_exp(double x) {
+  const uint32_t ax = (uint32_t)(tci_double_to_bits(x) >> 32) & 0x7fffffffu;
+  if (ax < 0x40860000u) {  // |x| < 704: the result is in (2^-1017, 2^1017)
+    uint32_t k;
+    const double n = tci_round(x * TCI_INV_LN2, &k);
+    const double r = fma(-n, TCI_LN2_HI, x) - n * TCI_LN2_LO;
+    return tci_bits_to_double(tci_double_to_bits(tci_exp_poly(r)) + ((uint64_t)k << 52));
+  }
+  if (x != x) return x;
+  if (x > 709.782712893384) return tci_bits_to_double(0x7ff0000000000000ULL);
+  if (x < -745.1332191019412) return 0.0;
+  double n = rint(x * TCI_INV_LN2);
+  double r = (x - n * TCI_LN2_HI) - n * TCI_LN2_LO;
+  return tci_scale2(tci_exp_poly(r), (int)n);
 }
 
 // sin(r)/r - 1 style polynomial for |r| <= pi/4: r + r^3 * S(r^2)
@@ -108,6 +134,26 @@ TCI_HD double tci_cos_poly(double r) {
 }
 
 TCI_HD double tci_cos(double x) {
+  const uint32_t ax = (uint32_t)(tci_double_to_bits(x) >> 32) & 0x7fffffffu;
+  if (ax < 0x41300000u) {  // |x| < 2^20: |n| < 2^20
+    uint32_t q;
+    const double n = tci_round(x * TCI_TWO_OVER_PI, &q);
+    const double r = fma(-n, TCI_PIO2_2, fma(-n, TCI_PIO2_1, x)) - n * TCI_PIO2_3;
+    const double z = r * r;
+    const bool odd = q & 1;  // the sine's polynomial, one coefficient shorter (0 * z + c = c)
+    double p = odd ? 0.0 : 1.5619206968586225e-16;
+    p = fma(p, z, odd ? 2.8114572543455206e-15 : -4.779477332387385e-14);
+    p = fma(p, z, odd ? -7.647163731819816e-13 : 1.1470745597729725e-11);
+    p = fma(p, z, odd ? 1.6059043836821613e-10 : -2.08767569878681e-09);
+    p = fma(p, z, odd ? -2.505210838544172e-08 : 2.755731922398589e-07);
+    p = fma(p, z, odd ? 2.7557319223985893e-06 : -2.48015873015873e-05);
+    p = fma(p, z, odd ? -0.0001984126984126984 : 0.001388888888888889);
+    p = fma(p, z, odd ? 0.008333333333333333 : -0.041666666666666664);
+    p = fma(p, z, odd ? -0.16666666666666666 : 0.5);
+    p = fma(odd ? r * z : -z, p, odd ? r : 1.0);
+    // quadrants 1 and 2 change the sign
+    return tci_bits_to_double(tci_double_to_bits(p) ^ ((uint64_t)((q ^ (q >> 1)) & 1u) << 63));
+  }
   if (x != x) return x;
   if (x - x != 0.0) return (x - x);  // +-Inf -> NaN
   double n = rint(x * TCI_TWO_OVER_PI);

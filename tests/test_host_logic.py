@@ -48,3 +48,8 @@ def test_index_sets_randomized(T, tmp_path):
 def test_integer_products_and_quotients(T, tmp_path):
     """int_mul / int_div (ieee_int.h) equal the host's IEEE operations."""
     _run_checker(T, tmp_path, "ieee_int_check")
+
+
+def test_exponential_cosine_and_constant_quotients(T, tmp_path):
+    """tci_math.h's short forms equal the plain ones."""
+    _run_checker(T, tmp_path, "tci_math_check")
