@@ -507,6 +507,25 @@ struct MsTimer {
 };
 }  // namespace
 
+// A lone RRLU task of a single solve from this many elements on runs on a
+// cluster beside the resident kernel (a launch, some 5 us, instead of a ring
+// ticket).  A 30-site quantics solve of rank 80 takes 143 ms without, and with
+// the line at 256 elements 44.5, at 1024 45.6, at 6000 50.3; a 40-site one of
+// rank 11 11.04, 10.81, 11.04, 11.04; an 8-site Lorentzian 4.51 and 3.0 at any.
+static constexpr int64_t COOP_ELEMS = 256;
+
+// The same for a launch whose only task is an RRLU task of f, as a single solve of
+// a caller's f makes: a launch either way.  8 sites of 10 values, ranks to 13: 24.0 ms
+// on one CTA, 21.0 so (100,000 evaluations by the caller included).
+int Engine::lone_cluster_ctas(const Req& r) const {
+  const tci_task& t = r.t;
+  if (t.kind != TCI_TASK_RRLU || t.post != TCI_POST_NONE || t.ain || r.ain_host || t.maxrank < 1 ||
+      (t.lutcap0 > 0 && !t.lut_full) || (int64_t)t.m * t.n < COOP_ELEMS)
+    return 0;
+  const int most = tci_k256::tci_rrlu_cluster_most(nullptr);
+  return most >= 16 ? tci_k256::tci_rrlu_cluster_ctas(t, most) : 0;
+}
+
 int Engine::launch() {
   if (pending_.empty() || inflight_) return 0;
   MsTimer timer(stats.host_launch_ms);
@@ -597,6 +616,8 @@ int Engine::launch() {
   const int grid = std::max(1, std::min<int>((int)nt, num_sms * ks_->ctas_per_sm));
   cta_stride = (cta_stride + 31) / 32 * 32;  // 256-byte aligned areas
   work_total = cta_stride * (size_t)grid;
+  const int ncta = nt == 1 ? lone_cluster_ctas(*batch[0]) : 0;
+  if (ncta) work_total = std::max(work_total, (size_t)std::max(batch[0]->t.maxrank, 1));  // pivot values
   int rc = ensure(blob_total, res_total, work_total);
   if (rc) {
     std::vector<Waiter> ws;
@@ -639,8 +660,17 @@ int Engine::launch() {
   // ---- upload, launch, download
   CUDA_TRY(cudaMemcpyAsync(dblob_, hblob_, blob_total, cudaMemcpyHostToDevice, stream_));
   if (timing) CUDA_TRY(cudaEventRecord(ev0_, stream_));
-  CUDA_TRY(ks_->step_launch(dblob_, dres_, (const int*)(dblob_ + off_order), (int)nt, dcounter_, grid, dwork_,
-                           cta_stride, stream_));
+  if (ncta) {
+    tci_task t = tasks[0];  // absolute addresses, as on the resident kernel
+    t.params = (int64_t)(uintptr_t)(dblob_ + o_params[0]);
+    t.rows = (int64_t)(uintptr_t)(dblob_ + o_rows[0]);
+    t.cols = (int64_t)(uintptr_t)(dblob_ + o_cols[0]);
+    t.res = (int64_t)(uintptr_t)(dres_ + o_res[0]);
+    CUDA_TRY(tci_k256::tci_rrlu_cluster_launch(t, ncta, dwork_, stream_));
+  } else {
+    CUDA_TRY(ks_->step_launch(dblob_, dres_, (const int*)(dblob_ + off_order), (int)nt, dcounter_, grid, dwork_,
+                             cta_stride, stream_));
+  }
   if (timing) CUDA_TRY(cudaEventRecord(ev1_, stream_));
   CUDA_TRY(cudaMemcpyAsync(hres_, dres_, res_total, cudaMemcpyDeviceToHost, stream_));
   CUDA_TRY(cudaEventRecord(done_, stream_));
@@ -940,13 +970,6 @@ void Engine::set_resident(ResidentQueue* q, BlockPool* host_pool, BlockPool* scr
   res_smem_ = q ? q->ks->resident_smem_bytes() : 0;
   res_threads_ = q ? q->ks->threads : 0;
 }
-
-// A lone RRLU task of a single solve from this many elements on runs on a
-// cluster beside the resident kernel (a launch, some 5 us, instead of a ring
-// ticket).  A 30-site quantics solve of rank 80 takes 143 ms without, and with
-// the line at 256 elements 44.5, at 1024 45.6, at 6000 50.3; a 40-site one of
-// rank 11 11.04, 10.81, 11.04, 11.04; an 8-site Lorentzian 4.51 and 3.0 at any.
-static constexpr int64_t COOP_ELEMS = 256;
 
 int Engine::cooperative_ctas(const Req& r, size_t batch) const {
   const tci_task& t = r.t;

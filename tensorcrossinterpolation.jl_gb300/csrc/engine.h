@@ -334,6 +334,7 @@ class Engine {
     size_t first, count;
   };
   int ensure(size_t blob, size_t res, size_t work);
+  int lone_cluster_ctas(const Req& r) const;
   int cooperative_ctas(const Req& r, size_t batch) const;
   void account(const Req& r, int smem_mode);
   int device_ = 0;

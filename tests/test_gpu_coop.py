@@ -51,3 +51,16 @@ def test_nan_and_zero(T, oracle):
         g = T.rrlu(M)
         assert g.npivot == r["npivot"] and np.array_equal(g.rowpermutation - 1, r["rowpermutation"])
         assert np.array_equal(g.L, r["L"], equal_nan=True) and np.array_equal(g.U, r["U"], equal_nan=True)
+
+
+@pytest.mark.parametrize("L,d,maxbond", [(5, 4, 4), (5, 16, 16), (6, 10, 40), (4, 25, 60)])
+def test_caller_f(T, oracle, L, d, maxbond):
+    """A caller's f: its factorizations, launched one at a time, against the same
+    solve with the values from the registered function."""
+    f = T.BatchFunction(lambda p: 1.5 / ((p.astype(np.float64) ** 2).sum(1) + 1.0))
+    kw = dict(tolerance=1e-10, maxbonddim=maxbond, maxiter=6)
+    got, ranks, errors = T.crossinterpolate2(float, f, [d] * L, **kw)
+    ref, rranks, rerrors = oracle.crossinterpolate2([d] * L, oracle.F_LORENTZ, [1.5], **kw)
+    assert list(ranks) == list(rranks) and np.array_equal(errors, rerrors)
+    for b in range(1, L + 1):
+        assert np.array_equal(got.sitetensor(b), ref.core(b))
