@@ -233,6 +233,7 @@ Engine::~Engine() {
   if (task_log_) std::fflush(task_log_);
   if (stream_) cudaStreamSynchronize(stream_);
   if (hblob_) cudaFreeHost(hblob_);
+  if (hscr_) cudaFreeHost(hscr_);
   if (hres_) cudaFreeHost(hres_);
   if (dblob_) cudaFree(dblob_);
   if (dres_) cudaFree(dres_);
@@ -244,6 +245,22 @@ Engine::~Engine() {
   if (hgat_) cudaFreeHost(hgat_);
   if (dgat_) cudaFree(dgat_);
   if (stream_) cudaStreamDestroy(stream_);
+}
+
+char* Engine::pinned_scratch(size_t bytes) {
+  if (bytes <= hscr_cap_) return hscr_;
+  if (stream_) cudaStreamSynchronize(stream_);
+  if (hscr_) cudaFreeHost(hscr_);
+  hscr_ = nullptr;
+  hscr_cap_ = 0;
+  const size_t cap = std::max(bytes, (size_t)2 << 20);
+  if (cudaHostAlloc((void**)&hscr_, cap, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    hscr_ = nullptr;
+    return nullptr;
+  }
+  hscr_cap_ = cap;
+  return hscr_;
 }
 
 #define CUDA_TRY(x)                                                             \
@@ -516,7 +533,7 @@ static constexpr int64_t COOP_ELEMS = 256;
 
 // The same for a launch whose only task is an RRLU task of f, as a single solve of
 // a caller's f makes: a launch either way.  8 sites of 10 values, ranks to 13: 24.0 ms
-// on one CTA, 21.0 so (100,000 evaluations by the caller included).
+// on one CTA, 21.0 so (before the misses of a product were put in order on the device).
 int Engine::lone_cluster_ctas(const Req& r) const {
   const tci_task& t = r.t;
   if (t.kind != TCI_TASK_RRLU || t.post != TCI_POST_NONE || t.ain || r.ain_host || t.maxrank < 1 ||

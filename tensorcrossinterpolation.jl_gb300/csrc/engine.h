@@ -244,6 +244,8 @@ class Engine {
   ~Engine();
   int init();
   cudaStream_t stream() const { return stream_; }
+  // Pinned memory kept with the engine (null: none to be had); the next call may move it.
+  char* pinned_scratch(size_t bytes);
 
   // Queue tasks for the next step and remember the coroutine to resume.
   void enqueue(std::vector<Req*>& reqs, std::coroutine_handle<> h, GpuOp* op);
@@ -369,6 +371,8 @@ class Engine {
   size_t hblob_cap_ = 0;
   char* dblob_ = nullptr;
   size_t dblob_cap_ = 0;
+  char* hscr_ = nullptr;
+  size_t hscr_cap_ = 0;
   char* hres_ = nullptr;
   size_t hres_cap_ = 0;
   char* dres_ = nullptr;

@@ -148,6 +148,84 @@ int FCache::grow(uint64_t need, cudaStream_t s) {
   return 0;
 }
 
+// Pinned memory for one product's points and values; larger ones take the general way.
+static constexpr size_t FC_PINNED_MAX = 16 << 20;
+
+static bool distinct_keys(const int64_t* k, int64_t n) {
+  std::vector<std::pair<int64_t, int64_t>> v((size_t)n);
+  for (int64_t i = 0; i < n; ++i) v[(size_t)i] = {k[2 * i], k[2 * i + 1]};
+  std::sort(v.begin(), v.end());
+  return std::adjacent_find(v.begin(), v.end()) == v.end();
+}
+
+// prefill for one product of distinct rows and columns (a Pi matrix; lists of
+// points are left to the general way): !done if it does not apply.
+int FCache::prefill_product(Engine& e, const FcProduct& p, const std::vector<int64_t>& keys, bool& done) {
+  const int64_t n = p.nr * p.nc;
+  if (p.nr < 2 || p.nc < 2 || n > INT32_MAX) return 0;
+  const int64_t* rk = keys.data();
+  const int64_t* ck = rk + 2 * p.nr;
+  if (!distinct_keys(rk, p.nr) || !distinct_keys(ck, p.nc)) return 0;
+  cudaStream_t s = e.stream();
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  const size_t kb = up(keys.size() * 8), rb = up((size_t)p.nr * p.rl), cb = up((size_t)p.nc * p.cl);
+  const size_t in = kb + rb + cb;
+  // host: [count][keys, rows, columns][points][values]; the points' place for the
+  // worst case if that fits, else once their number is known
+  const size_t point = (size_t)(L + 1) * 8, head = 256 + in;
+  if (head + 512 > FC_PINNED_MAX) return 0;
+  const bool sure = head + (size_t)n * point + 512 <= FC_PINNED_MAX;
+  char* h = e.pinned_scratch(sure ? head + (size_t)n * point + 512 : FC_PINNED_MAX);
+  if (!h) return 0;
+  const size_t fb = up((size_t)fc_blocks(n) * 256), ob = up(fc_blocks(n) * 4);
+  int rc = scratch(in + fb + ob + (size_t)n * 8);
+  if (rc) return rc;
+  std::memcpy(h + 256, keys.data(), keys.size() * 8);
+  std::memcpy(h + 256 + kb, p.rows, (size_t)p.nr * p.rl);
+  std::memcpy(h + 256 + kb + rb, p.cols, (size_t)p.nc * p.cl);
+  char* dv = (char*)dscr;
+  const int64_t *drk = (const int64_t*)dv, *dck = drk + 2 * p.nr;
+  uint32_t* flags = (uint32_t*)(dv + in);
+  unsigned* offsets = (unsigned*)(dv + in + fb);
+  uint64_t* where = (uint64_t*)(dv + in + fb + ob);
+  volatile unsigned long long* all = (volatile unsigned long long*)h;
+  int64_t* pts = (int64_t*)(h + head);
+  auto points = [&] {
+    fc_points_launch(flags, offsets, p.nr, p.nc, (const uint8_t*)dv + kb, p.rl, (const uint8_t*)dv + kb + rb, p.cl,
+                     where, pts, s);
+  };
+  cudaMemcpyAsync(dv, h + 256, in, cudaMemcpyHostToDevice, s);
+  fc_flag_launch(table, cap - 1, drk, p.nr, dck, p.nc, flags, offsets, (unsigned long long*)h, s);
+  if (sure) points();
+  if (cudaStreamSynchronize(s) != cudaSuccess) return fc_fail(TCI_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+  const int64_t u = (int64_t)*all;
+  if (u == 0) {
+    done = true;
+    return 0;
+  }
+  if (!sure) {
+    if (head + (size_t)u * point + 512 > FC_PINNED_MAX) return 0;
+    points();
+    if (cudaStreamSynchronize(s) != cudaSuccess)
+      return fc_fail(TCI_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+  }
+  done = true;
+  double* vals = (double*)(h + head + up((size_t)u * L * 8));
+  std::memset(vals, 0, (size_t)u * 8);
+  ++cb_depth;
+  const int frc = fn(user, L, u, pts, vals);
+  --cb_depth;
+  if (frc) return fc_fail(TCI_ERR_GENERIC, "caller-supplied f failed (code " + std::to_string(frc) + ")");
+  ++calls;
+  evaluated += u;
+  rc = grow(count + (uint64_t)u, s);
+  if (rc) return rc;
+  fc_store_launch(table, cap - 1, drk, p.nr, dck, where, vals, u, s);
+  if (cudaStreamSynchronize(s) != cudaSuccess) return fc_fail(TCI_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+  count += (uint64_t)u;
+  return 0;
+}
+
 int FCache::prefill(Engine& e, const std::vector<Req*>& reqs) {
   cudaStream_t s = e.stream();
   std::vector<Prod> prods;
@@ -207,6 +285,11 @@ int FCache::prefill(Engine& e, const std::vector<Req*>& reqs) {
       else
         ck[2 * j] = ck[2 * j + 1] = 0;
     }
+  }
+  if (prods.size() == 1 && fn) {
+    bool done = false;
+    const int rc = prefill_product(e, prods[0], hk, done);
+    if (rc || done) return rc;
   }
   const size_t kbytes = (nk * 8 + 255) / 256 * 256;
   const size_t cbytes = (prods.size() * 8 + 255) / 256 * 256;

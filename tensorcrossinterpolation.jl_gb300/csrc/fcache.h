@@ -9,7 +9,9 @@
 // products on the device and compacts the misses; the host turns the misses
 // into multi-indices, drops repeats, asks the caller's evaluator for exactly
 // those points (in column-major order of first appearance) and an insert
-// kernel stores them.  Hits never leave the device.
+// kernel stores them.  Hits never leave the device.  A single product without
+// repeats (a Pi matrix) has its misses put in order and its points written out by
+// kernels instead, straight into the buffer that the evaluator gets.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -80,6 +82,7 @@ struct FCache {
 
  private:
   int grow(uint64_t need, cudaStream_t s);
+  int prefill_product(Engine& e, const FcProduct& p, const std::vector<int64_t>& keys, bool& done);
   int scratch(size_t bytes);
   void write_params();
   void key_of(const uint8_t* v, int len, int site0, int64_t& k0, int64_t& k1) const;
@@ -96,6 +99,16 @@ int fc_callback_depth();
 void fc_probe_launch(const tci_fc_entry* tab, uint64_t mask, const int64_t* rk, int64_t nr, const int64_t* ck,
                      int64_t nc, unsigned long long* count, uint64_t* miss, cudaStream_t s);
 void fc_insert_launch(tci_fc_entry* tab, uint64_t mask, const tci_fc_entry* in, int64_t n, cudaStream_t s);
+// One product's misses in order (fcache.cu): flags (a bit per element), the number
+// of misses before each block of elements (fc_blocks of them) and in all, then the
+// misses' elements and points; and their values into the table.
+size_t fc_blocks(int64_t n);
+void fc_flag_launch(const tci_fc_entry* tab, uint64_t mask, const int64_t* rk, int64_t nr, const int64_t* ck,
+                    int64_t nc, uint32_t* flags, unsigned* counts, unsigned long long* all, cudaStream_t s);
+void fc_points_launch(const uint32_t* flags, const unsigned* offsets, int64_t nr, int64_t nc, const uint8_t* rows,
+                      int rl, const uint8_t* cols, int cl, uint64_t* where, int64_t* pts, cudaStream_t s);
+void fc_store_launch(tci_fc_entry* tab, uint64_t mask, const int64_t* rk, int64_t nr, const int64_t* ck,
+                     const uint64_t* where, const double* vals, int64_t n, cudaStream_t s);
 void fc_rehash_launch(tci_fc_entry* dst, uint64_t dmask, const tci_fc_entry* src, uint64_t scap, cudaStream_t s);
 
 }  // namespace tci
