@@ -714,6 +714,38 @@ __device__ __forceinline__ void swap_scale_body(double* A, int lda, int m, int n
   }
   if (is_nan_bits(p.piv)) fl.nan = true;
 }
+// swap_scale_body by one warp for at most 32 scaled lines: each lane takes an entry
+// by the place it comes from (rows K and R exchanged), so that all lanes run the
+// same few instructions; the lines are read before any is written.  A pivot of an
+// 8 x 8 matrix by one warp, with rank1_low: 3.1k cycles -> 2.55k.
+__device__ __forceinline__ void swap_scale_warp(double* A, int lda, int m, int n, int K, const Pick& p, bool leftorth,
+                                                int lane, JoinFlags& fl) {
+  const PivotDivisor D(p.piv);
+  const int mi = leftorth ? m : n, nj = leftorth ? n : m;
+  const int R = leftorth ? p.r : p.c, C = leftorth ? p.c : p.r;
+  const int si = leftorth ? 1 : lda, sj = leftorth ? lda : 1;
+  for (int w0 = 0; w0 < mi + nj; w0 += 32) {
+    const int w = w0 + lane, j = w - mi;
+    const bool line = w < mi;
+    const int from = w == R ? K : (w == K ? R : w);
+    const int ov = line ? from * si + C * sj : R * si + j * sj, oa = line ? from * si + K * sj : K * si + j * sj;
+    const int tv = line ? w * si + K * sj : oa, ta = line ? w * si + C * sj : ov;
+    const bool on = line || (j < nj && j != K && j != C), past = line ? w > K : j > K;
+    double v = 0.0, a = 0.0;
+    if (on) {
+      v = A[ov];
+      a = A[oa];
+    }
+    __syncwarp();
+    if (line && past) v = D.quo(v);
+    if (on) {
+      A[tv] = v;
+      if (line ? C != K : R != K) A[ta] = a;
+    }
+    if (on && (past || (line && w == K && C != K))) fl.join(past ? v : a);
+  }
+  if (is_nan_bits(p.piv)) fl.nan = true;
+}
 // Every thread gets how the update's products are taken.  The flags go through
 // a shared word per pivot parity (a barrier with a reduction costs three plain
 // ones); rrlu_loop clears it.
@@ -781,35 +813,44 @@ __device__ __forceinline__ void tile_products(const double (&x)[R], const double
 // Tracking: only elements whose |v| has a top word of at least the warp's
 // largest so far less one can be the maximum or lie within 16 ulps of it, so
 // a tile costs one vote and is pushed element by element only if it reaches that.
-template <int MODE>
+template <int MODE, int R = 2>
 __device__ __forceinline__ void rank1_tiles(double* A, int lda, int K, int m, int n, const double* x, const double* y,
                                             int ystride, int warp, int nw, ArgTrack& at) {
   const int lane = threadIdx.x & 31, lr = lane & 7, lc = lane >> 3;
-  const int nti = (m - K + 15) >> 4, ntj = (n - K + 7) >> 3;
-  int tj = warp / nti, ti = warp - tj * nti;
-  const int dj = nw / nti, di = nw - dj * nti;
+  const int nti = (m - K + 8 * R - 1) / (8 * R), ntj = (n - K + 7) >> 3;
+  // warp and nw over nti by an approximate reciprocal: a half added, a quotient is at
+  // least 0.5 / nti from an integer (an integer division is some 25 instructions)
+  const float rn = __fdividef(1.0f, (float)nti);
+  int tj = nw == 1 ? 0 : (int)(((float)warp + 0.5f) * rn), ti = warp - tj * nti;
+  const int dj = nw == 1 ? (nti == 1 ? 1 : 0) : (int)(((float)nw + 0.5f) * rn), di = nw - dj * nti;
   uint32_t top = 0;  // top word of the largest |v| pushed by the warp
   while (tj < ntj) {
-    const int i0 = K + 16 * ti + lr, j0 = K + 8 * tj + lc;
-    const bool vi[2] = {i0 < m, i0 + 8 < m}, vj[2] = {j0 < n, j0 + 4 < n};
-    const int ii[2] = {min(i0, m - 1), min(i0 + 8, m - 1)}, jj[2] = {min(j0, n - 1), min(j0 + 4, n - 1)};
+    const int i0 = K + 8 * R * ti + lr, j0 = K + 8 * tj + lc;
+    const bool vj[2] = {j0 < n, j0 + 4 < n};
+    const int jj[2] = {min(j0, n - 1), min(j0 + 4, n - 1)};
+    bool vi[R];
+    int ii[R];
+#pragma unroll
+    for (int a = 0; a < R; ++a) {
+      vi[a] = i0 + 8 * a < m;
+      ii[a] = min(i0 + 8 * a, m - 1);
+    }
     double* const p[2] = {A + (size_t)jj[0] * lda, A + (size_t)jj[1] * lda};
-    double v[2][2], xv[2], yv[2], q[2][2];
+    double v[R][2], xv[R], yv[2], q[R][2];
 #pragma unroll
     for (int b = 0; b < 2; ++b)
 #pragma unroll
-      for (int a = 0; a < 2; ++a) v[a][b] = p[b][ii[a]];
+      for (int a = 0; a < R; ++a) v[a][b] = p[b][ii[a]];
 #pragma unroll
-    for (int a = 0; a < 2; ++a) {
-      xv[a] = x[ii[a]];
-      yv[a] = y[(size_t)jj[a] * ystride];
-    }
+    for (int a = 0; a < R; ++a) xv[a] = x[ii[a]];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) yv[b] = y[(size_t)jj[b] * ystride];
     tile_products<MODE>(xv, yv, q);
     uint32_t h = 0;
 #pragma unroll
     for (int b = 0; b < 2; ++b)
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
+      for (int a = 0; a < R; ++a) {
         v[a][b] = __dsub_rn(v[a][b], q[a][b]);
         if (vi[a] && vj[b]) p[b][ii[a]] = v[a][b];
         h = max(h, (uint32_t)__double2hiint(v[a][b]) & 0x7fffffffu);
@@ -818,7 +859,7 @@ __device__ __forceinline__ void rank1_tiles(double* A, int lda, int K, int m, in
 #pragma unroll
       for (int b = 0; b < 2; ++b)
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
+        for (int a = 0; a < R; ++a)
           if (vi[a] && vj[b]) at.push(v[a][b], pack_key(ii[a], jj[b]));
       top = __reduce_max_sync(FULL, at.A ? (uint32_t)((at.A - 1) >> 32) : 0u);
     }
@@ -856,6 +897,16 @@ __device__ __forceinline__ ArgTrack rank1_update(double* A, int lda, int K, int 
   return at;
 }
 
+// Eight rows or fewer, one warp: 8 x 8 tiles (inline: a call costs as much as they
+// save, 500 cycles).
+__device__ __forceinline__ ArgTrack rank1_low(double* A, int lda, int K, int m, int n, const double* x,
+                                              const double* y) {
+  ArgTrack at;
+  at.init();
+  rank1_tiles<PROD_DENSE, 1>(A, lda, K, m, n, x, y, lda, 0, 1, at);
+  return at;
+}
+
 // Trailing blocks of at most this many elements are finished by warp 0 alone:
 // with one warp no CTA barrier is needed per pivot.  Measured: up to ~6 elements
 // per lane one warp beats the barriers of the whole CTA.
@@ -869,13 +920,16 @@ __device__ int rrlu_warp_tail(double* A, int lda, int m, int n, int K, int kmax,
   const int lane = threadIdx.x & 31;
   while (true) {
     fl.factors = 0;
-    swap_scale_body(A, lda, m, n, K, p, leftorth, lane, 32, fl);
+    if ((leftorth ? m : n) <= 32) swap_scale_warp(A, lda, m, n, K, p, leftorth, lane, fl);
+    else swap_scale_body(A, lda, m, n, K, p, leftorth, lane, 32, fl);
     int mode = PROD_DENSE;
     if (__any_sync(FULL, fl.factors != 0)) mode = __any_sync(FULL, fl.factors >= 2) ? PROD_FP64 : PROD_MIXED;
     __syncwarp();
     ++K;
     if (K == kmax) break;
-    const ArgTrack at = rank1_update(A, lda, K, m, n, A + (size_t)(K - 1) * lda, A + (K - 1), lda, 0, 1, mode);
+    const double *x = A + (size_t)(K - 1) * lda, *y = A + (K - 1);
+    const ArgTrack at = mode == PROD_DENSE && m - K <= 8 ? rank1_low(A, lda, K, m, n, x, y)
+                                                         : rank1_update(A, lda, K, m, n, x, y, lda, 0, 1, mode);
     uint64_t a = at.A, b = at.B;
     uint32_t k = at.k;
     warp_track(a, k, b);
