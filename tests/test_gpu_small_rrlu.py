@@ -1,7 +1,7 @@
 """Factorizations finished by one warp: shapes around its 32 scaled lines and the
-eight rows of its smaller tiles, both directions, with ties, zeros and NaN, on
 eight rows of its smaller tiles, both directions, with ties, zeros and NaN, against
 the oracle bit for bit."""
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
