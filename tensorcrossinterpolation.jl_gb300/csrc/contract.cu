@@ -208,6 +208,48 @@ __global__ void __launch_bounds__(CT, 2)
   }
 }
 
+// The same with one thread per output, FP64 products: a small result has too few
+// tiles for the SMs, and spreads over them so.  The offsets along k are formed once
+// per CTA; eight loads in flight.  A product of host matrices, tiles and so:
+// 60 x 60 x 60 125 and 52 us, 256 x 512 x 100 310 and 228, 512 x 512 x 100 348 and 323,
+// 700 x 700 x 100 360 and 427: the line lies at 2^18 outputs.
+constexpr int EACH_K = 256;
+__global__ void __launch_bounds__(128)
+    gemm_each_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A, tci_map3 a_row, tci_map3 a_k,
+                     const double* __restrict__ B, tci_map3 b_k, tci_map3 b_col, double* __restrict__ C, tci_map3 c_row,
+                     tci_map3 c_col) {
+  __shared__ int64_t ka[EACH_K], kb[EACH_K];
+  const int64_t e = gtid();
+  const bool on = e < M * N;
+  const int64_t j = on ? e / M : 0, i = on ? e - j * M : 0;
+  const double* a = A + map_at(a_row, i);
+  const double* b = B + map_at(b_col, j);
+  double acc = 0.0;
+  for (int64_t k0 = 0; k0 < K; k0 += EACH_K) {
+    const int kc = (int)(K - k0 < EACH_K ? K - k0 : EACH_K);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kc; k += 128) {
+      ka[k] = map_at(a_k, k0 + k);
+      kb[k] = map_at(b_k, k0 + k);
+    }
+    __syncthreads();
+    int k = 0;
+    for (; k + 4 <= kc; k += 4) {
+      double x[4], y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        x[q] = __ldg(a + ka[k + q]);
+        y[q] = __ldg(b + kb[k + q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc = __dadd_rn(acc, __dmul_rn(x[q], y[q]));
+    }
+    for (; k < kc; ++k) acc = __dadd_rn(acc, __dmul_rn(__ldg(a + ka[k]), __ldg(b + kb[k])));
+  }
+  if (on) C[map_at(c_row, i) + map_at(c_col, j)] = acc;
+}
+constexpr int64_t EACH_OUTPUTS = 1 << 18;
+
 // The tile's width by the number of columns: a wider one than needed computes
 // columns past the edge.
 cudaError_t gemm_map(int64_t M, int64_t N, int64_t K, const double* A, tci_map3 a_row, tci_map3 a_k, const double* B,
@@ -217,7 +259,10 @@ cudaError_t gemm_map(int64_t M, int64_t N, int64_t K, const double* A, tci_map3 
     const int64_t t = (M + bm - 1) / bm * ((N + bn - 1) / bn);
     return (unsigned)(t < 65535 * 16 ? t : 65535 * 16);
   };
-  if (N <= 16)
+  if (M * N <= EACH_OUTPUTS)
+    gemm_each_kernel<<<(unsigned)((M * N + 127) / 128), 128, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row,
+                                                                      c_col);
+  else if (N <= 16)
     gemm_map_kernel<16, 2><<<grid(128, 16), CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
   else if (N <= 32)
     gemm_map_kernel<32, 4><<<grid(128, 32), CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
