@@ -1237,15 +1237,19 @@ int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxran
   r.t.core_out = dout;
   std::vector<Req*> reqs{&r};
   // A fresh L or U has no pages yet; a device copy into it would fault them in one
-  // by one, and far from the core that reads them next.  Another thread touches
-  // them (contents kept) while the device works.
+  // by one (some 4 us each), and far from the core that reads them next.  They are
+  // touched (contents kept) by another thread while the device works, or, few as
+  // they are, by this one after it.
+  auto touch = [](double* a, size_t count) {
+    volatile char* p = (volatile char*)a;
+    for (size_t q = 0; p && q < count * 8; q += 4096) p[q] = p[q];
+  };
   std::thread toucher;
-  const size_t touch = (size_t)std::max(m, n) * (size_t)kmax * 8;
-  if (touch >= ((size_t)1 << 20))
+  const bool many = (size_t)std::max(m, n) * (size_t)kmax * 8 >= ((size_t)1 << 20);
+  if (many)
     toucher = std::thread([=] {
-      const size_t nl = L ? (size_t)m * (size_t)kmax * 8 : 0, nu = U ? (size_t)kmax * (size_t)n * 8 : 0;
-      for (size_t q = 0; q < nl; q += 4096) ((volatile char*)L)[q] = ((volatile char*)L)[q];
-      for (size_t q = 0; q < nu; q += 4096) ((volatile char*)U)[q] = ((volatile char*)U)[q];
+      touch(L, (size_t)m * (size_t)kmax);
+      touch(U, (size_t)kmax * (size_t)n);
     });
   int rc = e.run_tasks(reqs);
   if (toucher.joinable()) toucher.join();
@@ -1258,6 +1262,10 @@ int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxran
   // the permutations, and L and U as compact matrices, straight to the caller
   std::vector<int32_t> perms((size_t)(m + n));
   const size_t nl = (size_t)m * K, nu = (size_t)K * n;
+  if (!many) {
+    touch(L, nl);
+    touch(U, nu);
+  }
   double* lu = (L || U) && nl + nu > 0 ? e.alloc_core(nl + nu) : nullptr;
   cudaError_t ce = (L || U) && nl + nu > 0 && !lu ? cudaErrorMemoryAllocation : cudaSuccess;
   if (ce == cudaSuccess && m + n > 0)
