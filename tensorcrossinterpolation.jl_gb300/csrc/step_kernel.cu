@@ -2054,7 +2054,7 @@ __device__ void resident_dispatch(tci_queue_slot* __restrict__ hs, uint32_t hmas
   }
 }
 
-// Persistent kernel of the resident mode (cooperative launch, one CTA per SM).
+// Persistent kernel of the resident mode (every CTA resident: tci_resident_launch).
 // CTA 0 hosts the dispatcher; every other CTA claims the next device ticket
 // with one atomic, waits until it is dispatched (or the dispatcher has left:
 // tickets past the last dispatched one are never used), runs the task and
@@ -3348,7 +3348,7 @@ cudaError_t tci_rrlu_big_launch(const double* ain, double* work, double* fact, c
                                      stream);
 }
 
-// Launch the resident kernel: one CTA per SM, all resident at once
+// Launch the resident kernel on every SM, all CTAs resident at once
 // (cooperative launch), after clearing the per-launch part of its state.
 // slots/qc are mapped pinned host memory, st device memory.
 // cluster > 1: in clusters of that many CTAs, which leaves the other GPCs whole
