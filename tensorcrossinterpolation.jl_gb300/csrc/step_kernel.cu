@@ -3015,6 +3015,9 @@ __device__ __forceinline__ void cluster_update(const ClusterBlock<SPILL>& B, int
 template <bool SPILL, class Fill>
 __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCtl& ctl, const Fill& fill) {
   const cg::cluster_group cl = cg::this_cluster();
+  // The first exchange writes to every CTA's shared memory, which is there once that
+  // CTA has started: all arrive here, and the fill covers the wait.
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   const int tid = threadIdx.x, ncta = P.pr * P.pc, rank = (int)cl.block_rank(), m = P.m, n = P.n;
   const bool leftorth = P.leftorth != 0;
   const int bp = rank / P.pc, bq = rank % P.pc, mb = P.mb, nb = P.nb;
@@ -3075,6 +3078,7 @@ __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCt
   PivotState S;
   S.init(P.reltol, P.abstol);
   int K = 0;
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // every CTA has started
   while (P.kmax > 0) {
     // ---- the pivot: argmax of abs2 over the cluster's trailing blocks
     const int par = K & 1;
