@@ -31,8 +31,8 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <atomic>
 
+#include "device_once.h"
 #include "tc_gemm.h"
 
 namespace {
@@ -356,13 +356,11 @@ template <int BN, int STAGES>
 cudaError_t launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int Mp, int Np, int kiters,
                       double* C, tci_map3 crow, tci_map3 ccol, int* err, cudaStream_t st) {
   using S = TcSmem<BN, STAGES>;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         S::TOTAL);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static DeviceOnce limit;
+  const cudaError_t e = limit([] {
+    return cudaFuncSetAttribute(tc_gemm_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+  });
+  if (e != cudaSuccess) return e;
   if (Mp / BM > 65535) return cudaErrorInvalidValue;
   dim3 grid((unsigned)(Np / BN), (unsigned)(Mp / BM));
   tc_gemm_kernel<BN, STAGES><<<grid, TC_THREADS, S::TOTAL, st>>>(ta, tb, M, N, Mp, Np, kiters, C, crow, ccol, err);
@@ -842,12 +840,10 @@ cudaError_t tci_tc_evaluate_split(int L, const int64_t* dims, const double* cons
   int per_sm = (int)std::min<uint32_t>(EV_CTAS, 512 / Y.cols);
   while (per_sm > 1 && Y.smem() + 1024 > SM_BYTES / per_sm) --per_sm;
   const uint32_t smem = std::max(Y.smem(), SM_BYTES / per_sm - 1024 - (per_sm > 1 ? 1024u : 0u));
-  static std::atomic<uint32_t> limit{0};
-  if (limit.load() < smem) {
-    e = cudaFuncSetAttribute(tc_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_BYTES);
-    if (e != cudaSuccess) return e;
-    limit.store(SM_BYTES);
-  }
+  static DeviceOnce limit;
+  e = limit(
+      [] { return cudaFuncSetAttribute(tc_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_BYTES); });
+  if (e != cudaSuccess) return e;
   const int64_t ntiles = (np + BM - 1) / BM;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)nsm * per_sm));
   if (np > 0) tc_eval_kernel<<<grid, EV_THREADS, smem, st>>>(sites_dev, L, Y, pts_dev, np, out_dev, err_dev);

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 
+#include "device_once.h"
 #include "ieee_int.h"
 #include "tci_tasks.h"
 
@@ -190,10 +191,10 @@ int tci_tt_eval_max_bond() { return 225 * 1024 / 16; }
 cudaError_t tci_tt_eval_launch(const tci_core_ref* cores, int* cls, int L, int rmax, const uint8_t* pts, int64_t np,
                                double* out, int num_sms, cudaStream_t st) {
   if (np <= 0) return cudaSuccess;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(tt_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-  if (attr != cudaSuccess) return attr;
-  cudaError_t e = cudaMemsetAsync(cls, 0, (size_t)L * sizeof(int), st);
+  static DeviceOnce limit;
+  cudaError_t e = limit(
+      [] { return cudaFuncSetAttribute(tt_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024); });
+  if (e == cudaSuccess) e = cudaMemsetAsync(cls, 0, (size_t)L * sizeof(int), st);
   if (e != cudaSuccess) return e;
   core_class_kernel<<<dim3(L, 4), 256, 0, st>>>(cores, cls);
   // Points per CTA: as many as shared memory takes, up to 256, but no more than
