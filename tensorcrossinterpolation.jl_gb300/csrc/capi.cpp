@@ -43,6 +43,8 @@ struct tci_ctx {
   // destroy objects of the same context from inside it.  Entry points that
   // compute refuse to run there (Engine::run / run_tasks).
   std::recursive_mutex mu;
+  int depth = 0;   // calls that hold `mu`
+  int device = 0;
   int64_t peak_live = 0;  // most solves live at once in a batched / serving drive (stats)
   Engine& eng_ref() { return *engp; }
   // Solves destroyed while another thread held `mu` (a server holds it until it
@@ -62,6 +64,24 @@ struct tci_ctx {
 struct tci_solve {
   tci_ctx* ctx = nullptr;
   Solve s;
+};
+
+// The lock of an entry point, for as long as its call is at work on the device.
+class CtxLock {
+ public:
+  explicit CtxLock(tci_ctx* c) : c_(c) {
+    c_->mu.lock();
+    if (c_->depth++ == 0) DeviceUsers::enter(c_->device);
+  }
+  ~CtxLock() {
+    if (--c_->depth == 0) DeviceUsers::leave(c_->device);
+    c_->mu.unlock();
+  }
+  CtxLock(const CtxLock&) = delete;
+  CtxLock& operator=(const CtxLock&) = delete;
+
+ private:
+  tci_ctx* c_;
 };
 
 void tci_ctx::release_dead() {
@@ -171,6 +191,7 @@ int tci_ctx_create(int device, size_t hbm_budget, tci_ctx** out) {
   int neng = resident ? (int)std::min(16u, std::max(4u, hw ? hw : 12u)) : 8;
   if (const char* s = std::getenv("TCI_ENGINES")) neng = std::max(1, std::min(32, std::atoi(s)));
   std::unique_ptr<tci_ctx> c(new tci_ctx());
+  c->device = device;
   c->dpool.reset(new BlockPool(BlockPool::DEVICE, device, true));
   c->xpool.reset(new BlockPool(BlockPool::HOST, device, true));
   for (int i = 0; i < neng; ++i) {
@@ -220,7 +241,7 @@ int tci_ctx_synchronize(tci_ctx* ctx) {
 
 int tci_ctx_set_resident_limits(tci_ctx* ctx, int32_t idle_us, int64_t wait_us) {
   if (idle_us < 100 || wait_us < 1) return fail(TCI_ERR_ARG, "idle_us must be >= 100 and wait_us >= 1");
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (!ctx->rq) return 0;  // batched launches only: nothing waits
   int rc = ctx->rq->stop();  // the next launch takes the new limits
   ctx->rq->qc->idle_us = idle_us;
@@ -293,7 +314,7 @@ static int run_solve(tci_ctx* ctx, Solve& s, CoTask& t) {
 
 int tci_solve_create(tci_ctx* ctx, int32_t L, const int64_t* localdims, int32_t fid, const double* fparams,
                      int64_t nparams, const int64_t* pivots, int64_t np, tci_solve** out) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   ctx->release_dead();
   int rc = make_solve(ctx, L, localdims, fid, fparams, nparams, out);
   if (rc) return rc;
@@ -331,7 +352,7 @@ int tci_fcache_stats(const tci_solve* s, int64_t* entries, int64_t* evaluated, i
 int tci_crossinterpolate2(tci_ctx* ctx, int32_t L, const int64_t* localdims, int32_t fid,
                           const double* fparams, int64_t nparams, const int64_t* pivots, int64_t np,
                           const tci_opts* opts, tci_solve** out) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   ctx->release_dead();
   int rc = make_solve(ctx, L, localdims, fid, fparams, nparams, out);
   if (rc) return rc;
@@ -360,7 +381,7 @@ int tci_crossinterpolate2(tci_ctx* ctx, int32_t L, const int64_t* localdims, int
 }
 
 int tci_optimize(tci_solve* s, const tci_opts* opts) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   tci_opts o;
   if (opts)
     o = *opts;
@@ -372,7 +393,7 @@ int tci_optimize(tci_solve* s, const tci_opts* opts) {
 
 int tci_updatepivots(tci_solve* s, int32_t b, int32_t leftorthogonal, double reltol, double abstol,
                      int64_t maxbonddim) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   if (b < 1 || b > s->s.L - 1) return fail(TCI_ERR_ARG, "bond index out of range");
   CoTask t = co_updatepivots(s->ctx->eng_ref(), s->s, b - 1, leftorthogonal != 0, reltol, abstol,
                              maxbonddim <= 0 ? TYPEMAX : maxbonddim, nullptr, nullptr);
@@ -381,7 +402,7 @@ int tci_updatepivots(tci_solve* s, int32_t b, int32_t leftorthogonal, double rel
 
 int tci_sweep2site(tci_solve* s, int32_t niter, int32_t iter1, double abstol, int64_t maxbonddim,
                    int32_t sweepstrategy, int32_t strictlynested, int32_t fillsitetensors) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   CoTask t = co_sweep2site(s->ctx->eng_ref(), s->s, niter, iter1, abstol, maxbonddim <= 0 ? TYPEMAX : maxbonddim,
                            sweepstrategy, strictlynested != 0, fillsitetensors != 0);
   return run_solve(s->ctx, s->s, t);
@@ -389,20 +410,20 @@ int tci_sweep2site(tci_solve* s, int32_t niter, int32_t iter1, double abstol, in
 
 int tci_sweep1site(tci_solve* s, int32_t forward, double reltol, double abstol, int64_t maxbonddim,
                    int32_t updatetensors) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   CoTask t = co_sweep1site(s->ctx->eng_ref(), s->s, forward != 0, reltol, abstol,
                            maxbonddim <= 0 ? TYPEMAX : maxbonddim, updatetensors != 0);
   return run_solve(s->ctx, s->s, t);
 }
 
 int tci_fillsitetensors(tci_solve* s) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   CoTask t = co_fillsitetensors(s->ctx->eng_ref(), s->s);
   return run_solve(s->ctx, s->s, t);
 }
 
 int tci_addglobalpivots(tci_solve* s, const int64_t* pivots, int64_t np) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   int rc = 0;
   auto piv = to_pivots(pivots, np, s->s.L, s->s.d, &rc);
   if (rc) return rc;
@@ -455,7 +476,7 @@ int tci_get_sets(const tci_solve* s, int32_t b, int64_t* I, int64_t* nI, int64_t
 // and nJ x (L-b)); the site tensors are invalidated (tensorci2.jl:528-529 style
 // replacement of the index sets, as a restart would do).
 int tci_set_sets(tci_solve* s, int32_t b, const int64_t* I, int64_t nI, const int64_t* J, int64_t nJ) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   Solve& v = s->s;
   if (b < 1 || b > v.L) return fail(TCI_ERR_ARG, "site index out of range");
   if (nI < 0 || nJ < 0) return fail(TCI_ERR_ARG, "negative set size");
@@ -511,7 +532,7 @@ int tci_get_core(const tci_solve* s, int32_t b, double* out, int64_t* dims) {
 int tci_get_cores_pinned(tci_ctx* ctx, int64_t n, tci_solve* const* solves, double** out, int64_t* total_elems) {
   *out = nullptr;
   *total_elems = 0;
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   std::vector<const double*> src;
   std::vector<int64_t> len;
   int64_t total = 0;
@@ -557,7 +578,7 @@ int tci_get_core_dims_batched(int64_t n, tci_solve* const* solves, int64_t* dims
 
 int tci_get_cores_batched(tci_ctx* ctx, int64_t n, tci_solve* const* solves, double* out,
                           const int64_t* out_offsets) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   std::vector<const double*> src;
   std::vector<int64_t> len;
   int64_t expect = -1;
@@ -603,12 +624,12 @@ static int train_values(tci_ctx* ctx, const Solve& s, const int64_t* points, int
 }
 
 int tci_evaluate(tci_solve* s, const int64_t* points, int64_t np, double* out) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   return train_values(s->ctx, s->s, points, np, out);
 }
 
 int tci_sum(tci_solve* s, double* out) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   CoTask t = co_sum(s->ctx->eng_ref(), s->s, out);
   return run_solve(s->ctx, s->s, t);
 }
@@ -703,7 +724,7 @@ int tci_evaluate_prec(tci_solve* s, const int64_t* points, int64_t np, double* o
     return tci_evaluate(s, points, np, out);
   }
   if (precision != TCI_PREC_TF32X3) return fail(TCI_ERR_ARG, "unknown precision");
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   return split_evaluate(s->ctx, s->s, points, np, out, err_est);
 }
 
@@ -987,7 +1008,7 @@ int drive(tci_ctx* ctx, std::deque<Job>& jobs, bool use_arrival, int64_t max_liv
 
 int tci_crossinterpolate2_batched(tci_ctx* ctx, int64_t n, const tci_request* reqs, int64_t max_live,
                                   tci_solve** out) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   ctx->release_dead();
   std::deque<Job> jobs((size_t)n);
   for (int64_t i = 0; i < n; ++i) jobs[i].req = reqs[i];
@@ -998,7 +1019,7 @@ int tci_crossinterpolate2_batched(tci_ctx* ctx, int64_t n, const tci_request* re
 
 int tci_serve_run(tci_ctx* ctx, int64_t n, const tci_request* reqs, const double* arrival, int64_t max_live,
                   double* latency, int64_t* rank, double* wall) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   std::deque<Job> jobs((size_t)n);
   for (int64_t i = 0; i < n; ++i) {
     jobs[i].req = reqs[i];
@@ -1040,7 +1061,7 @@ struct tci_server {
 namespace {
 void server_main(tci_server* srv) {
   tci_ctx* ctx = srv->ctx;
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);  // the server owns the context until it stops
+  CtxLock lk(ctx);  // the server owns the context until it stops
   std::deque<Job> jobs;
   JobFeed feed;
   feed.pull = [srv](std::deque<Job>& js, std::vector<int64_t>& order) {
@@ -1140,7 +1161,7 @@ int tci_serve_stop(tci_server* srv) {
 // ---------------------------------------------------------------- f and host helpers
 int tci_feval(tci_ctx* ctx, int32_t fid, const double* fparams, int64_t nparams, int32_t L,
               const int64_t* localdims, const int64_t* points, int64_t np, double* out) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   Solve s;
   int rc = solve_init(s, L, localdims, fid, fparams, nparams, nullptr, 0);
   if (rc) return rc;
@@ -1159,7 +1180,7 @@ int tci_feval(tci_ctx* ctx, int32_t fid, const double* fparams, int64_t nparams,
 
 int tci_optfirstpivot(tci_ctx* ctx, int32_t fid, const double* fparams, int64_t nparams, int32_t L,
                       const int64_t* localdims, int64_t* pivot, int32_t maxsweep) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   Solve s;
   int rc = solve_init(s, L, localdims, fid, fparams, nparams, nullptr, 0);
   if (rc) return rc;
@@ -1175,7 +1196,7 @@ int tci_optfirstpivot(tci_ctx* ctx, int32_t fid, const double* fparams, int64_t 
 
 int tci_estimatetrueerror(tci_solve* s, int32_t nsearch, const int64_t* initialpoints, int64_t np, uint64_t seed,
                           int64_t cap, int64_t* pivots, double* errors, int64_t* nout) {
-  std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+  CtxLock lk(s->ctx);
   const int L = s->s.L;
   int rc = 0;
   std::vector<std::vector<uint8_t>> starts;
@@ -1214,7 +1235,7 @@ int tci_convergencecriterion(const int64_t* ranks, const double* errors, const i
 int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxrank, double reltol,
              double abstol, int32_t leftorthogonal, int64_t* rowperm, int64_t* colperm, double* L, double* U,
              int64_t* npivot, double* error) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (m < 0 || n < 0 || m > INT32_MAX || n > INT32_MAX || m * n > INT32_MAX)
     return fail(TCI_ERR_ARG, "matrix size out of range");
   Engine& e = ctx->eng_ref();
@@ -1292,7 +1313,7 @@ int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxran
 int tci_rrlu_batched(tci_ctx* ctx, int64_t nmat, const double* A, const int64_t* offsets, const int64_t* ms,
                      const int64_t* ns, int64_t maxrank, double reltol, double abstol, int32_t leftorthogonal,
                      int64_t* piv, const int64_t* piv_offsets, int64_t* npivots, double* errors) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   Engine& e = ctx->eng_ref();
   std::vector<Req> rs((size_t)nmat);
   std::vector<Req*> ptrs;
@@ -1459,7 +1480,7 @@ int tune_time(Engine& e, const TuneSet& S, int32_t c, double& ms) {
 }  // namespace
 
 int tci_autotune_rrlu(tci_ctx* ctx, int32_t reps, double* speedup, double* ms_default, double* ms_tuned) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (ctx->rq) {  // plain launches: the calibration times the batched step kernel
     int rc = ctx->rq->stop();
     if (rc) return rc;
@@ -1531,7 +1552,7 @@ int tci_autotune_rrlu(tci_ctx* ctx, int32_t reps, double* speedup, double* ms_de
 }
 
 int tci_autotune_table(tci_ctx* ctx, int32_t* table, int32_t* nbuckets, int32_t set) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (nbuckets) *nbuckets = Engine::TUNE_BUCKETS;
   if (!table) return 0;
   if (set) {
@@ -1595,7 +1616,7 @@ int tci_tt4_contract(tci_ctx* ctx, int32_t L, const int64_t* a_dims, const doubl
                      const int64_t* b_dims, const double* const* b_cores, int32_t algorithm, int32_t method,
                      double tolerance, int64_t maxbonddim, tci_tt4** out) {
   *out = nullptr;
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (algorithm != TCI_CONTRACT_NAIVE && algorithm != TCI_CONTRACT_ZIPUP)
     return fail(TCI_ERR_ARG, "Unknown algorithm.");
   if (method != TCI_FACTORIZE_LU && method != TCI_FACTORIZE_CI) return fail(TCI_ERR_GENERIC, "Not implemented yet.");
@@ -1637,7 +1658,7 @@ int tci_tt4_contract_prec(tci_ctx* ctx, int32_t L, const int64_t* a_dims, const 
   *out = nullptr;
   if (precision != TCI_PREC_TF32X3) return fail(TCI_ERR_ARG, "unknown precision");
   if (algorithm != TCI_CONTRACT_ZIPUP) return fail(TCI_ERR_ARG, "split precision is implemented for algorithm = :zipup");
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (method != TCI_FACTORIZE_LU && method != TCI_FACTORIZE_CI) return fail(TCI_ERR_GENERIC, "Not implemented yet.");
   if (L < 1) return fail(TCI_ERR_ARG, "empty tensor train");
   if (ctx->rq) {  // plain launches: the tensor-core kernels need the SMs
@@ -1668,7 +1689,7 @@ int tci_matmul(tci_ctx* ctx, int64_t M, int64_t N, int64_t K, const double* A, c
                int32_t precision, double* err_est) {
   if (M < 0 || N < 0 || K < 0) return fail(TCI_ERR_ARG, "negative matrix dimension");
   if (precision != TCI_PREC_FP64 && precision != TCI_PREC_TF32X3) return fail(TCI_ERR_ARG, "unknown precision");
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (err_est) *err_est = 0.0;
   if (M == 0 || N == 0) return 0;
   if (ctx->rq) {
@@ -1702,7 +1723,7 @@ int tci_matmul(tci_ctx* ctx, int64_t M, int64_t N, int64_t K, const double* A, c
 int tci_tt4_compress(tci_ctx* ctx, int32_t L, const int64_t* dims, const double* const* cores, int32_t method,
                      double tolerance, int64_t maxbonddim, int32_t normalizeerror, tci_tt4** out) {
   *out = nullptr;
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (L < 1) return fail(TCI_ERR_ARG, "empty tensor train");
   if (method != TCI_FACTORIZE_LU && method != TCI_FACTORIZE_CI) return fail(TCI_ERR_GENERIC, "Not implemented yet.");
   Engine& e = ctx->eng_ref();
@@ -1724,7 +1745,7 @@ int tci_tt4_contract_tci(tci_ctx* ctx, int32_t L, const int64_t* a_dims, const d
                          int64_t np, int32_t ninitialpivots, tci_value_fn f, void* user, const tci_opts* opts,
                          tci_tt4** out) {
   *out = nullptr;
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (L < 1) return fail(TCI_ERR_ARG, "empty tensor train");
   Engine& e = ctx->eng_ref();
   TT4 a, b;
@@ -1781,7 +1802,7 @@ int tci_tt4_dims(const tci_tt4* t, int64_t* dims) {
 
 int tci_tt4_get_core(const tci_tt4* t, int32_t b, double* out) {
   if (b < 1 || b > (int32_t)t->tt.cores.size()) return fail(TCI_ERR_ARG, "site index out of range");
-  std::lock_guard<std::recursive_mutex> lk(t->ctx->mu);
+  CtxLock lk(t->ctx);
   Engine& e = t->ctx->eng_ref();
   const Tensor4& c = t->tt.cores[b - 1];
   cudaError_t ce = cudaMemcpyAsync(out, c.p, c.elems() * sizeof(double), cudaMemcpyDeviceToHost, e.stream());
@@ -1793,7 +1814,7 @@ int tci_tt4_get_core(const tci_tt4* t, int32_t b, double* out) {
 int tci_tt4_destroy(tci_tt4* t) {
   if (!t) return 0;
   {
-    std::lock_guard<std::recursive_mutex> lk(t->ctx->mu);
+    CtxLock lk(t->ctx);
     t->tt.release(t->ctx->eng_ref());
   }
   delete t;
@@ -1845,7 +1866,7 @@ extern "C" {
 
 int tci_tt_evaluate(tci_ctx* ctx, int32_t L, const int64_t* dims, const double* const* cores, const int64_t* points,
                     int64_t np, double* out) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (L < 1) return fail(TCI_ERR_ARG, "empty tensor train");
   Engine& e = ctx->eng_ref();
   Solve s;
@@ -1863,7 +1884,7 @@ int tci_tt_evaluate_prec(tci_ctx* ctx, int32_t L, const int64_t* dims, const dou
     return tci_tt_evaluate(ctx, L, dims, cores, points, np, out);
   }
   if (precision != TCI_PREC_TF32X3) return fail(TCI_ERR_ARG, "unknown precision");
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (L < 1) return fail(TCI_ERR_ARG, "empty tensor train");
   Engine& e = ctx->eng_ref();
   Solve s;
@@ -1875,7 +1896,7 @@ int tci_tt_evaluate_prec(tci_ctx* ctx, int32_t L, const int64_t* dims, const dou
 }
 
 int tci_tt_sum(tci_ctx* ctx, int32_t L, const int64_t* dims, const double* const* cores, double* out) {
-  std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+  CtxLock lk(ctx);
   if (L < 1) return fail(TCI_ERR_ARG, "empty tensor train");
   Engine& e = ctx->eng_ref();
   Solve s;

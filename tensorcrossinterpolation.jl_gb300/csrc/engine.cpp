@@ -531,6 +531,12 @@ struct MsTimer {
 // rank 11 11.04, 10.81, 11.04, 11.04; an 8-site Lorentzian 4.51 and 3.0 at any.
 static constexpr int64_t COOP_ELEMS = 256;
 
+// Cluster kernels wait for SMs while other work on the device holds them (of this
+// process or not), the ring's tasks do not: the rest of a solve whose bonds have
+// waited this long goes through the ring.  Beside back-to-back 8192^3 bf16 products
+// an 8-site Lorentzian took 29.5 ms waiting at each bond.
+static constexpr double COOP_WAIT_MS = 5.0;
+
 // The same for a launch whose only task is an RRLU task of f, as a single solve of
 // a caller's f makes: a launch either way.  8 sites of 10 values, ranks to 13: 24.0 ms
 // on one CTA, 21.0 so (before the misses of a product were put in order on the device).
@@ -868,6 +874,35 @@ void BlockPool::free(void* p) {
 }
 
 // ---------------------------------------------------------------- resident ring
+namespace {
+struct DeviceCount {
+  std::mutex mu;
+  int users = 0;
+};
+DeviceCount& device_count(int device) {
+  static DeviceCount c[64];
+  return c[device & 63];
+}
+}  // namespace
+
+void DeviceUsers::enter(int device) {
+  DeviceCount& c = device_count(device);
+  std::lock_guard<std::mutex> lk(c.mu);
+  ++c.users;
+}
+void DeviceUsers::leave(int device) {
+  DeviceCount& c = device_count(device);
+  std::lock_guard<std::mutex> lk(c.mu);
+  --c.users;
+}
+bool DeviceUsers::alone(int device, const std::function<void()>& enqueue) {
+  DeviceCount& c = device_count(device);
+  std::lock_guard<std::mutex> lk(c.mu);
+  if (c.users > 1) return false;
+  enqueue();
+  return true;
+}
+
 int ResidentQueue::init(int dev, int num_sms, int idle_us) {
   device = dev;
   this->num_sms = num_sms;
@@ -904,6 +939,7 @@ ResidentQueue::~ResidentQueue() {
 int ResidentQueue::start(const tci_kernel_set* k, int clusters, int cluster_ctas) {
   std::lock_guard<std::mutex> lk(mu);
   if (running) return k == ks && cluster == cluster_ctas ? 0 : fail(TCI_ERR_GENERIC, "resident kernel already running in another variant");
+  if (clusters > 0 && !DeviceUsers::alone(device, [] {})) clusters = cluster_ctas = 0;
   ks = k;
   cluster = cluster_ctas;
   grid = clusters > 0 ? clusters * cluster : num_sms * ks->ctas_per_sm;
@@ -1080,17 +1116,24 @@ int Engine::submit() {
           break;
         }
         f.dblocks.push_back(pivs);
-        r.ticket = t.ticket = ++coop_seq_;
-        const cudaError_t ce = tci_k256::tci_rrlu_cluster_launch(t, ncta, pivs, stream_);
+        cudaError_t ce = cudaSuccess;
+        const bool out = DeviceUsers::alone(device_, [&] {
+          r.ticket = t.ticket = ++coop_seq_;
+          ce = tci_k256::tci_rrlu_cluster_launch(t, ncta, pivs, stream_);
+        });
         if (ce != cudaSuccess) {
           rc = fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
           break;
         }
-        stats.launches += 1;
-        stats.h2d_bytes += (int64_t)o_res;
-        stats.d2h_bytes += (int64_t)r.res_bytes;
-        f.reqs.push_back(&r);
-        continue;
+        if (out) {
+          stats.launches += 1;
+          stats.h2d_bytes += (int64_t)o_res;
+          stats.d2h_bytes += (int64_t)r.res_bytes;
+          f.cluster = true;
+          f.sent = std::chrono::steady_clock::now();
+          f.reqs.push_back(&r);
+          continue;
+        }
       }
       t.cost = task_cost(t);
       // small inputs are copied to shared memory in one parallel pass when the
@@ -1157,6 +1200,12 @@ int Engine::poll(bool& progressed) {
     flights_.pop_back();
     inflight_tasks_ -= g.reqs.size();
     stats.tasks += (int64_t)g.reqs.size();
+    if (g.cluster) {
+      // what the task took beside its own cycles (at 1 GHz or more) and a launch
+      const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - g.sent).count();
+      coop_wait_ms_ += std::max(0.0, ms - (double)g.reqs[0]->head()->cycles * 1e-6 - 0.1);
+      if (coop_wait_ms_ > COOP_WAIT_MS) coop_most_ = 0;
+    }
     for (Req* r : g.reqs) account(*r, r->t.smem_mode);
     const int status = g.w.op->status;  // nonzero: a task of this op could not be submitted
     g.w.op->status = status;
@@ -1401,8 +1450,10 @@ int Engine::run_resident(CoTask& t) {
   int clusters = 0;
   const int most = tci_k256::tci_rrlu_cluster_most(&clusters);
   coop_most_ = most >= 16 && clusters > 4 ? most : 0;
-  int rc = coop_most_ ? att_rq_->start(&tci_k512::kernels, 4, coop_most_) : att_rq_->start(&tci_k512::kernels);
+  int rc = att_rq_->start(&tci_k512::kernels, coop_most_ ? 4 : 0, coop_most_);
   if (rc) return rc;
+  if (!att_rq_->cluster) coop_most_ = 0;
+  coop_wait_ms_ = 0;
   set_resident(att_rq_, att_h_, att_s_);
   t.h.resume();
   auto now = [] { return std::chrono::steady_clock::now(); };
@@ -1437,7 +1488,7 @@ int Engine::run_resident(CoTask& t) {
     }
   }
   const int src = att_rq_->stop();
-  if (coop_most_ && has_flights()) cudaStreamSynchronize(stream_);  // after an error: no task may outlive its record
+  if (has_flights()) cudaStreamSynchronize(stream_);  // after an error: no task may outlive its record
   coop_most_ = 0;
   abandon();
   set_resident(nullptr, nullptr, nullptr);

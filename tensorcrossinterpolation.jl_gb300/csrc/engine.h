@@ -5,9 +5,11 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <chrono>
 #include <coroutine>
 #include <cstdio>
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -163,6 +165,18 @@ class BlockPool {
   size_t reserved_ = 0;
 };
 
+// The contexts of the process with a call in progress on each device.  A single solve
+// has cluster kernels beside its resident one only while its context is the only one
+// at work: another's kernels may hold the SMs that a cluster needs, and every bond
+// would wait for them.
+struct DeviceUsers {
+  static void enter(int device);
+  static void leave(int device);
+  // Runs `enqueue` unless a second context is at work (none enters meanwhile);
+  // whether it ran.
+  static bool alone(int device, const std::function<void()>& enqueue);
+};
+
 // The ring of the resident kernel, shared by the engines of a context.
 struct ResidentQueue {
   int device = 0;
@@ -184,9 +198,10 @@ struct ResidentQueue {
   ~ResidentQueue();
   // launch the kernel unless it is running: the throughput variant (k256) for
   // batched and served solves, the latency variant (k512) for a single solve
-  // clusters > 0: that many clusters of `cluster` CTAs instead of every SM, with
-  // the rest of the device left to cluster kernels
-  int start(const tci_kernel_set* k, int clusters = 0, int cluster = 0);
+  // clusters > 0: that many clusters of `cluster_ctas` CTAs instead of every SM, with
+  // the rest of the device left to cluster kernels; every SM all the same, and
+  // `cluster` 0, while a second context is at work on the device
+  int start(const tci_kernel_set* k, int clusters = 0, int cluster_ctas = 0);
   int ensure_alive(); // relaunch it if every CTA has left (idle limit)
   int stop();         // ask the CTAs to leave once the ring is drained; wait
   int publish(const tci_task& t, uint64_t& ticket);
@@ -345,6 +360,8 @@ class Engine {
     Waiter w;
     std::vector<Req*> reqs;
     std::vector<void*> hblocks, dblocks;
+    bool cluster = false;  // one task on a cluster kernel, enqueued at `sent`
+    std::chrono::steady_clock::time_point sent{};
   };
   ResidentQueue* rq_ = nullptr;
   ResidentQueue* att_rq_ = nullptr;
@@ -362,6 +379,7 @@ class Engine {
   // beside the resident kernel (0: none)
   int coop_most_ = 0;
   uint64_t coop_seq_ = 0;
+  double coop_wait_ms_ = 0;  // what the solve's cluster kernels have waited for SMs
   std::vector<char> big_res_;  // host copy of the last multi-CTA rrLU's result record
   cudaStream_t stream_ = nullptr;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
