@@ -549,6 +549,10 @@ int Engine::lone_cluster_ctas(const Req& r) const {
   return most >= 16 ? tci_k256::tci_rrlu_cluster_ctas(t, most) : 0;
 }
 
+// Host doubles and int64 that the device may read in place: on their natural alignment
+// (a packed record or a view into a byte buffer need not be; the host copies those).
+bool Engine::in_place(const void* p) const { return host_direct_ && ((uintptr_t)p & 7) == 0; }
+
 int Engine::launch() {
   if (pending_.empty() || inflight_) return 0;
   MsTimer timer(stats.host_launch_ms);
@@ -624,7 +628,7 @@ int Engine::launch() {
     o_cores[i] = off;
     off = a16(off + (size_t)r.ncores * sizeof(tci_core_ref));
     o_ain[i] = off;
-    if (r.ain_host && !host_direct_) off = a16(off + (size_t)r.t.m * r.t.n * 8);
+    if (r.ain_host && !in_place(r.ain_host)) off = a16(off + (size_t)r.t.m * r.t.n * 8);
     o_res[i] = res_total;
     r.res_bytes = result_bytes(r.t);
     res_total += r.res_bytes;
@@ -666,7 +670,7 @@ int Engine::launch() {
     if (!t.lut_full) t.lut = nullptr;
     // a given matrix is read once: in place across the host link (190 GB/s, against
     // 14 for one thread copying it to the upload buffer) where the device can
-    if (r.ain_host) t.ain = host_direct_ ? r.ain_host : (const double*)(dblob_ + o_ain[i]);
+    if (r.ain_host) t.ain = in_place(r.ain_host) ? r.ain_host : (const double*)(dblob_ + o_ain[i]);
     t.cost = task_cost(t);
     tasks[i] = t;
     if (t.nparams) std::memcpy(hblob_ + o_params[i], r.params, (size_t)t.nparams * 8);
@@ -674,7 +678,7 @@ int Engine::launch() {
     if (r.cols_bytes) std::memcpy(hblob_ + o_cols[i], r.cols, r.cols_bytes);
     if (r.prows_bytes) std::memcpy(hblob_ + o_prows[i], r.prows, r.prows_bytes);
     if (r.ncores) std::memcpy(hblob_ + o_cores[i], r.cores, (size_t)r.ncores * sizeof(tci_core_ref));
-    if (r.ain_host && !host_direct_) std::memcpy(hblob_ + o_ain[i], r.ain_host, (size_t)r.t.m * r.t.n * 8);
+    if (r.ain_host && !in_place(r.ain_host)) std::memcpy(hblob_ + o_ain[i], r.ain_host, (size_t)r.t.m * r.t.n * 8);
   }
   int* order = (int*)(hblob_ + off_order);
   std::iota(order, order + nt, 0);
@@ -2036,7 +2040,7 @@ static constexpr int64_t PACK_DIRECT = 1 << 16;
 
 int Engine::upload_points(const Solve& s, const int64_t* points, int64_t np, uint8_t* dev_pts) {
   const int L = s.L;
-  if (!host_direct_ || np * L < PACK_DIRECT) {
+  if (!in_place(points) || np * L < PACK_DIRECT) {
     std::vector<uint8_t> pts;
     int rc = pack_points(points, np, L, s.d, pts);
     if (rc) return rc;

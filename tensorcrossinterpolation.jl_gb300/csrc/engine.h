@@ -309,7 +309,7 @@ class Engine {
   int run_cluster(Req& r, int ncta);
   // Kernels may read the caller's pageable host memory (coherent host link): large
   // inputs are then taken in place instead of through host-side copies.
-  bool host_direct() const { return host_direct_; }
+  bool in_place(const void* p) const;
   // Points (np x L, 1-based, host) as bytes into dev_pts (device), range-checked:
   // packed on the device from the caller's memory, or on the host where that is
   // small or not readable.  Waits for the check.
