@@ -38,7 +38,7 @@ CU_SOURCES = [
     ("tc_gemm.cu", "tc_gemm.cu.o", []),
 ]
 CXX_SOURCES = ["engine.cpp", "capi.cpp", "contract.cpp", "fcache.cpp", "contract_tci.cpp", "pivotsearch.cpp"]
-HEADERS = ["device_once.h", "ieee_int.h", "kernels.h", "tci_tasks.h", "tci_functions.h", "tci_math.h", "tci_rng.h", "engine.h", "contract.h", "contract_tci.h", "fcache.h", "fc_slot.h", "tc_gemm.h"]
+HEADERS = ["device_once.h", "ieee_int.h", "kernels.h", "tci_tasks.h", "tci_functions.h", "tci_math.h", "tci_rng.h", "engine.h", "contract.h", "contract_tci.h", "fcache.h", "fc_slot.h", "page_touch.h", "tc_gemm.h"]
 
 
 def _newer(target, deps):

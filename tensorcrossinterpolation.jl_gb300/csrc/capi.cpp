@@ -18,6 +18,7 @@
 #include "contract.h"
 #include "contract_tci.h"
 #include "engine.h"
+#include "page_touch.h"
 #include "tc_gemm.h"
 
 cudaError_t tci_lu_factors_launch(const double* F, int m, int n, int K, int leftorth, double* L, double* U,
@@ -1257,23 +1258,12 @@ int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxran
   if (!dout) return fail(TCI_ERR_OOM, "device memory");
   r.t.core_out = dout;
   std::vector<Req*> reqs{&r};
-  // A fresh L or U has no pages yet; a device copy into it would fault them in one
-  // by one (some 4 us each), and far from the core that reads them next.  They are
-  // touched (contents kept) by another thread while the device works, or, few as
-  // they are, by this one after it.
-  auto touch = [](double* a, size_t count) {
-    volatile char* p = (volatile char*)a;
-    for (size_t q = 0; p && q < count * 8; q += 4096) p[q] = p[q];
-  };
-  std::thread toucher;
-  const bool many = (size_t)std::max(m, n) * (size_t)kmax * 8 >= ((size_t)1 << 20);
-  if (many)
-    toucher = std::thread([=] {
-      touch(L, (size_t)m * (size_t)kmax);
-      touch(U, (size_t)kmax * (size_t)n);
-    });
+  // large results are touched by another thread while the device works
+  PageToucher toucher;
+  const bool touched = (size_t)std::max(m, n) * (size_t)kmax * 8 >= ((size_t)1 << 20) &&
+                       toucher.start(L, (size_t)m * (size_t)kmax, U, (size_t)kmax * (size_t)n);
   int rc = e.run_tasks(reqs);
-  if (toucher.joinable()) toucher.join();
+  toucher.join();
   if (rc) {
     e.free_core(dout);
     return rc;
@@ -1283,9 +1273,9 @@ int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxran
   // the permutations, and L and U as compact matrices, straight to the caller
   std::vector<int32_t> perms((size_t)(m + n));
   const size_t nl = (size_t)m * K, nu = (size_t)K * n;
-  if (!many) {
-    touch(L, nl);
-    touch(U, nu);
+  if (!touched) {
+    touch_pages(L, nl);
+    touch_pages(U, nu);
   }
   double* lu = (L || U) && nl + nu > 0 ? e.alloc_core(nl + nu) : nullptr;
   cudaError_t ce = (L || U) && nl + nu > 0 && !lu ? cudaErrorMemoryAllocation : cudaSuccess;
