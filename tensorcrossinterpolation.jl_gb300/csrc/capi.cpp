@@ -1,6 +1,7 @@
 // C ABI of libtci_gpu.so (include/tci_gb300.h): thin wrappers that build the
 // solve state, run the coroutine algorithm on the context's engine and copy
 // results into caller buffers.
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -49,16 +50,20 @@ struct tci_ctx {
   int64_t peak_live = 0;  // most solves live at once in a batched / serving drive (stats)
   Engine& eng_ref() { return *engp; }
   // Solves destroyed while another thread held `mu` (a server holds it until it
-  // stops): released by the next holder.  Waiting for the lock instead would
-  // deadlock a thread whose garbage collector finalizes an old solve while that
-  // thread is the one to stop the server.
+  // stops): released by that holder when it gives the lock up and, in a drive, on
+  // the way.  Waiting for the lock instead would deadlock a thread whose garbage
+  // collector finalizes an old solve while that thread is the one to stop the server.
   std::mutex dead_mu;
   std::vector<tci_solve*> dead;
+  std::atomic<size_t> ndead{0};  // dead.size()
   void bury(tci_solve* s) {
     std::lock_guard<std::mutex> lk(dead_mu);
     dead.push_back(s);
+    ndead.store(dead.size());
   }
-  void release_dead();  // with `mu` held
+  void release_dead();           // with `mu` held
+  void release_dead_running();   // the same while the resident kernel is at work
+  void release_dead_if_unheld();
   ~tci_ctx();
 };
 
@@ -72,11 +77,17 @@ class CtxLock {
  public:
   explicit CtxLock(tci_ctx* c) : c_(c) {
     c_->mu.lock();
-    if (c_->depth++ == 0) DeviceUsers::enter(c_->device);
+    if (c_->depth++ > 0) return;
+    DeviceUsers::enter(c_->device);
+    c_->release_dead();
   }
   ~CtxLock() {
-    if (--c_->depth == 0) DeviceUsers::leave(c_->device);
+    if (--c_->depth == 0) {
+      c_->release_dead();
+      DeviceUsers::leave(c_->device);
+    }
     c_->mu.unlock();
+    c_->release_dead_if_unheld();
   }
   CtxLock(const CtxLock&) = delete;
   CtxLock& operator=(const CtxLock&) = delete;
@@ -86,14 +97,44 @@ class CtxLock {
 };
 
 void tci_ctx::release_dead() {
+  if (!ndead.load()) return;
   std::vector<tci_solve*> gone;
   {
     std::lock_guard<std::mutex> lk(dead_mu);
     gone.swap(dead);
+    ndead.store(0);
   }
   for (tci_solve* s : gone) {
     engp->release_solve(s->s);
     delete s;
+  }
+}
+// A caller-supplied f's cache is CUDA memory of its own, whose release would wait for
+// the resident kernel: such solves stay on the list.
+void tci_ctx::release_dead_running() {
+  std::vector<tci_solve*> gone;
+  {
+    std::lock_guard<std::mutex> lk(dead_mu);
+    const auto rest = std::partition(dead.begin(), dead.end(), [](tci_solve* s) { return s->s.fcache != nullptr; });
+    gone.assign(rest, dead.end());
+    dead.erase(rest, dead.end());
+    ndead.store(dead.size());
+  }
+  for (tci_solve* s : gone) {
+    engp->release_solve(s->s);
+    delete s;
+  }
+}
+// After a solve was buried, and after the lock was given up: between the two, either
+// the one that buried finds the lock free or the one that held it finds the solve
+// (each writes before it looks).
+void tci_ctx::release_dead_if_unheld() {
+  for (;;) {
+    std::atomic_thread_fence(std::memory_order_seq_cst);
+    if (!ndead.load()) return;
+    std::unique_lock<std::recursive_mutex> lk(mu, std::try_to_lock);
+    if (!lk.owns_lock()) return;
+    release_dead();
   }
 }
 tci_ctx::~tci_ctx() {
@@ -316,7 +357,6 @@ static int run_solve(tci_ctx* ctx, Solve& s, CoTask& t) {
 int tci_solve_create(tci_ctx* ctx, int32_t L, const int64_t* localdims, int32_t fid, const double* fparams,
                      int64_t nparams, const int64_t* pivots, int64_t np, tci_solve** out) {
   CtxLock lk(ctx);
-  ctx->release_dead();
   int rc = make_solve(ctx, L, localdims, fid, fparams, nparams, out);
   if (rc) return rc;
   auto piv = to_pivots(pivots, np, L, (*out)->s.d, &rc);
@@ -336,8 +376,7 @@ int tci_solve_destroy(tci_solve* s) {
   if (!s) return 0;
   tci_ctx* ctx = s->ctx;
   ctx->bury(s);
-  std::unique_lock<std::recursive_mutex> lk(ctx->mu, std::try_to_lock);
-  if (lk.owns_lock()) ctx->release_dead();
+  ctx->release_dead_if_unheld();
   return 0;
 }
 
@@ -354,7 +393,6 @@ int tci_crossinterpolate2(tci_ctx* ctx, int32_t L, const int64_t* localdims, int
                           const double* fparams, int64_t nparams, const int64_t* pivots, int64_t np,
                           const tci_opts* opts, tci_solve** out) {
   CtxLock lk(ctx);
-  ctx->release_dead();
   int rc = make_solve(ctx, L, localdims, fid, fparams, nparams, out);
   if (rc) return rc;
   std::vector<int64_t> ones;
@@ -825,7 +863,12 @@ int drive(tci_ctx* ctx, std::deque<Job>& jobs, bool use_arrival, int64_t max_liv
     const int64_t share = std::max<int64_t>(1, (max_live + G - 1) / G);
     double last_progress = now_s(), last_done = last_progress;
     double last_switch = now_s();
+    size_t kept = 0;  // destroyed solves left on the context's list
     for (;;) {
+      if (g == 0 && ctx->ndead.load() != kept) {
+        ctx->release_dead_running();
+        kept = ctx->ndead.load();
+      }
       // Kernel variant by load (worker 0): with fewer live solves than SMs and no
       // admission waiting, every task gets a whole SM (k512); from two live
       // solves per SM on, two task CTAs share an SM (k256).  Tasks are
@@ -1010,7 +1053,6 @@ int drive(tci_ctx* ctx, std::deque<Job>& jobs, bool use_arrival, int64_t max_liv
 int tci_crossinterpolate2_batched(tci_ctx* ctx, int64_t n, const tci_request* reqs, int64_t max_live,
                                   tci_solve** out) {
   CtxLock lk(ctx);
-  ctx->release_dead();
   std::deque<Job> jobs((size_t)n);
   for (int64_t i = 0; i < n; ++i) jobs[i].req = reqs[i];
   int rc = drive(ctx, jobs, false, max_live, true, nullptr);
