@@ -2186,14 +2186,7 @@ __global__ void __launch_bounds__(NT, TCI_CTAS_PER_SM)
 struct BigBar {
   unsigned int count, gen;
   int error;
-  unsigned int pad;
-};
-// A CTA's partial of one pivot step as the others wait for it: each word carries 32
-// bits of the maximum (A with the sign of its element, B, key, place) and, above
-// them, the step's number plus one, so that the words are their own flag.
-struct __align__(16) BigSlot {
-  unsigned long long w[6];
-  unsigned int nan, pad[3];
+  unsigned int arrived;  // partials published so far (G per pivot step; never reset)
 };
 struct BigPartial {
   unsigned long long A, B;
@@ -2274,6 +2267,10 @@ __device__ __forceinline__ unsigned ld_acquire_gpu_u32(const unsigned* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void red_release_gpu_add_u32(unsigned* p, unsigned v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 constexpr long long BIG_BAR_POLLS = 1LL << 24;  // bounded wait of one grid barrier (a few seconds)
 
 // Grid-wide barrier (sense by generation).  Returns false once any CTA has hit
@@ -2377,37 +2374,19 @@ __device__ void block_track_to0(BigTrack& t, BigCtl& ctl) {
   }
 }
 
-// Publish this CTA's partial of step `tag` - 1 (one thread, after a CTA barrier that
-// follows the CTA's update).  The fence is cumulative: it also covers the other
-// threads' update writes, which the CTA barrier ordered before it, so that a CTA
-// that sees the words and then fences sees the update too.
-__device__ __forceinline__ void big_publish(BigSlot& o, const BigTrack& t, unsigned tag) {
-  const unsigned long long hi = (unsigned long long)tag << 32;
-  const uint32_t sign = (uint32_t)__double2hiint(t.v) & 0x80000000u;  // A is at most 2^63 - 2^52 + 1
-  const uint32_t d[6] = {(uint32_t)t.A, (uint32_t)(t.A >> 32) | (t.A ? sign : 0u), (uint32_t)t.B, (uint32_t)(t.B >> 32),
-                         t.k, t.ph};
-  __threadfence();
-#pragma unroll
-  for (int q = 0; q < 6; q += 2)
-    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(&o.w[q]), "l"(hi | d[q]), "l"(hi | d[q + 1])
-                 : "memory");
-}
-// Whether the slot holds the partial of step `tag` - 1, and the partial.
-__device__ __forceinline__ bool big_look(const BigSlot& o, unsigned tag, BigTrack& t) {
-  unsigned long long w[6];
-#pragma unroll
-  for (int q = 0; q < 6; q += 2)
-    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[q]), "=l"(w[q + 1]) : "l"(&o.w[q]) : "memory");
-  bool all = true;
-#pragma unroll
-  for (int q = 0; q < 6; ++q) all = all && (uint32_t)(w[q] >> 32) == tag;
-  const uint32_t ah = (uint32_t)w[1];
-  t.A = ((uint64_t)(ah & 0x7fffffffu) << 32) | (uint32_t)w[0];
-  t.B = ((uint64_t)(uint32_t)w[3] << 32) | (uint32_t)w[2];
-  t.k = (uint32_t)w[4];
-  t.ph = (uint32_t)w[5];
-  t.v = t.A ? __longlong_as_double((long long)((t.A - 1) | ((uint64_t)(ah & 0x80000000u) << 32))) : 0.0;
-  return all;
+// Publish this CTA's partial (one thread, after a CTA barrier that follows the
+// CTA's update): the fields, then one arrival on the grid's counter with release
+// semantics (cumulative: it also covers the other threads' update writes, which
+// the CTA barrier ordered before it), so that a CTA that sees the count with
+// acquire also sees the partial and the update.  The arrival is a reduction (no
+// round trip).
+__device__ __forceinline__ void big_publish(BigPartial& o, const BigTrack& t, BigBar* bar) {
+  o.A = t.A;
+  o.B = t.B;
+  o.k = t.k;
+  o.ph = t.ph;
+  o.v = t.v;
+  red_release_gpu_add_u32(&bar->arrived, 1u);
 }
 
 // Partials one lane of the gathering warp loads at once, and the most it handles
@@ -2415,45 +2394,53 @@ __device__ __forceinline__ bool big_look(const BigSlot& o, unsigned tag, BigTrac
 constexpr int BIG_GATHER_Q = 5;
 constexpr int BIG_GATHER_MAX = 2 * BIG_GATHER_Q;
 
-// Warp 0: wait for the G partials of step `tag` - 1, every lane polling its share,
-// and combine them; every lane gets the result.  This wait is the pivot step's only
-// grid-wide synchronisation: a CTA publishes after its update, so once all G are
-// in, every update of the step is done and visible.  Returns false if the wait hit
-// its bound or another CTA has flagged an error (the flag is then set).
-// The words being their own flag, the partials arrive with the poll that sees them
-// (a counter to wait for first is one more trip through L2, and G atomics on it):
-// a 2048 x 2048 host matrix, 512 pivots: 13.6 -> 12.9 ms a call; a pivot of 530 x 517
-// spends 7.6k cycles from its update's end to the next decision, 9 to 10k before.
-__device__ bool big_gather(const BigSlot* cur, int G, unsigned tag, BigBar* bar, BigTrack& g) {
+// Warp 0: wait until `target` partials have arrived in all (lane 0 polls the
+// counter, bounded), then combine the G partials of this step, every lane
+// loading its share at once; every lane gets the result.  This wait is the pivot
+// step's only grid-wide synchronisation: a CTA publishes after its update, so
+// once all G are in, every update of the step is done and visible.  Returns
+// false if the wait hit its bound or another CTA has flagged an error (the flag
+// is then set).
+// Partials that are their own flags, polled by every CTA, save the counter's trip
+// and cost more: 174 x 1653 to rank 136 takes 0.94 ms so and 1.10 to 1.15 with them,
+// 513 x 512 to full rank 3.05 and 3.9 to 4.1, 2048 x 2048 to rank 512 8.94 and 9.07.
+__device__ bool big_gather(const BigPartial* cur, int G, unsigned target, BigBar* bar, BigTrack& g) {
   const int lane = threadIdx.x & 31;
   g.init();
   int ok = 1;
-  for (int base = 0; ok && base < G; base += 32 * BIG_GATHER_Q) {
-    unsigned missing = 0;  // of this lane's slots
-#pragma unroll
-    for (int q = 0; q < BIG_GATHER_Q; ++q)
-      if (base + lane + 32 * q < G) missing |= 1u << q;
-    for (long long it = 0;; ++it) {
-#pragma unroll
-      for (int q = 0; q < BIG_GATHER_Q; ++q) {
-        BigTrack t;
-        if ((missing >> q & 1u) && big_look(cur[base + lane + 32 * q], tag, t)) {
-          missing &= ~(1u << q);
-          big_combine(g.A, g.k, g.ph, g.B, g.v, t.A, t.k, t.ph, t.B, t.v);
-        }
+  if (lane == 0) {
+    unsigned sleep_ns = 16;
+    for (long long it = 0; ld_acquire_gpu_u32(&bar->arrived) < target; ++it) {
+      if (it > BIG_BAR_POLLS || *(volatile int*)&bar->error) {
+        atomicExch(&bar->error, 1);
+        ok = 0;
+        break;
       }
-      if (!__any_sync(FULL, missing)) break;
-      if ((it & 63) == 63) {
-        const int err = lane == 0 ? (it > BIG_BAR_POLLS ? 1 : *(volatile int*)&bar->error) : 0;
-        if (__shfl_sync(FULL, err, 0)) {
-          if (lane == 0) atomicExch(&bar->error, 1);
-          ok = 0;
-          break;
-        }
-      }
+      __nanosleep(sleep_ns);
+      sleep_ns = sleep_ns < 64 ? sleep_ns * 2 : 64;
     }
   }
-  __threadfence();  // the updates behind the partials, for the CTA barrier that follows
+  ok = __shfl_sync(FULL, ok, 0);
+  __syncwarp();  // lane 0's acquire orders the warp's loads below
+  for (int base = 0; ok && base < G; base += 32 * BIG_GATHER_Q) {
+    uint64_t qa[BIG_GATHER_Q], qb[BIG_GATHER_Q];
+    uint32_t qk[BIG_GATHER_Q], qp[BIG_GATHER_Q];
+    double qv[BIG_GATHER_Q];
+#pragma unroll
+    for (int q = 0; q < BIG_GATHER_Q; ++q) {
+      if (base + lane + 32 * q < G) {
+        const BigPartial* p = cur + base + lane + 32 * q;
+        qa[q] = __ldcg(&p->A);
+        qb[q] = __ldcg(&p->B);
+        qk[q] = __ldcg(&p->k);
+        qp[q] = __ldcg(&p->ph);
+        qv[q] = __ldcg(&p->v);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < BIG_GATHER_Q; ++q)
+      if (base + lane + 32 * q < G) big_combine(g.A, g.k, g.ph, g.B, g.v, qa[q], qk[q], qp[q], qb[q], qv[q]);
+  }
   uint64_t a = g.A, b = g.B;
   uint32_t kk = g.k, ph = g.ph;
   double v = g.v;
@@ -2471,7 +2458,7 @@ struct BigArgs {
   double* A;              // m x n working copy (physical positions never change)
   double* fact;           // m x n factors in logical order, then int32 rowperm[m], colperm[n]
   char* res;              // result record (tci_result_head, rowp[kcap], colp[kcap], diag[kcap])
-  BigSlot* parts;         // 2 x gridDim.x partials (double-buffered by pivot parity)
+  BigPartial* parts;      // 2 x gridDim.x partials (double-buffered by pivot parity)
   double* pivs;           // signed pivot of every step (kmax)
   BigBar* bar;
   int m, n, kmax, kcap, leftorth;
@@ -2598,7 +2585,7 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
     }
   }
   block_track(bt, ctl);
-  if (tid == 0) big_publish(P.parts[b], bt, 1);  // buffer 0: read at pivot 0
+  if (tid == 0) big_publish(P.parts[b], bt, P.bar);  // buffer 0: read at pivot 0
   bool ok = true;
   int K = 0;
   tci_result_head* head = (tci_result_head*)P.res;
@@ -2651,13 +2638,13 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
   while (ok) {
     // the partials of pivot K are in buffer K & 1: a CTA writes the next set to
     // the other buffer, so a fast CTA never overwrites what a slow one reads
-    BigSlot* const cur = P.parts + (size_t)(K & 1) * G;
+    BigPartial* const cur = P.parts + (size_t)(K & 1) * G;
     // ---- the pivot: argmax of abs2 over the trailing block, from the G partials
     // (warp 0 waits for them); unless the exact pass is needed, lane 0 also takes
     // the decision
     if (tid < 32) {
       BigTrack g;
-      const bool got = big_gather(cur, G, (unsigned)K + 1, P.bar, g);
+      const bool got = big_gather(cur, G, (unsigned)(K + 1) * (unsigned)G, P.bar, g);
       if (tid == 0) {
         ctl.bar_err = got ? 0 : 1;
         if (got) {
@@ -2714,23 +2701,28 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
       if (!ok) break;
       block_track(et, ctl);
       if (tid == 0) {
-        big_publish(cur[b], et, (unsigned)K + 1);
+        BigPartial& o = cur[b];
+        o.A = et.A;
+        o.B = 0;
+        o.k = et.k;
+        o.ph = et.ph;
+        o.v = et.v;
       }
       ok = big_barrier(P.bar, G, gen, ctl);
       if (!ok) break;
       BigTrack g;
       g.init();
       for (int t = tid; t < G; t += BIG_NT) {
-        BigTrack o;
-        big_look(cur[t], (unsigned)K + 1, o);
-        big_combine(g.A, g.k, g.ph, g.B, g.v, o.A, o.k, o.ph, o.B, o.v);
+        const BigPartial* q = cur + t;
+        big_combine(g.A, g.k, g.ph, g.B, g.v, __ldcg(&q->A), __ldcg(&q->k), __ldcg(&q->ph), __ldcg(&q->B),
+                    __ldcg(&q->v));
       }
       block_track(g, ctl);
       if (tid == 0) {
         if (g.A) {
           ctl.kmax = (int)g.ph;
           ctl.K = (int)g.k;
-          ctl.piv = __ldcg(&P.A[(g.ph & 0xffffu) + (size_t)(g.ph >> 16) * m]);  // A held squares here
+          ctl.piv = g.v;
         }
         decide();
       }
@@ -2774,7 +2766,7 @@ __global__ void __launch_bounds__(BIG_NT, 1) rrlu_big_kernel(BigArgs P) {
     block_track_to0(bt, ctl);
     // read at pivot K (already incremented); no grid barrier: the next gather
     // waits for every CTA's partial
-    if (tid == 0) big_publish(P.parts[(size_t)(K & 1) * G + b], bt, (unsigned)K + 1);
+    if (tid == 0) big_publish(P.parts[(size_t)(K & 1) * G + b], bt, P.bar);
   }
   if (ok) ok = big_barrier(P.bar, G, gen, ctl);  // every pivot value is recorded
   if (!ok) {
@@ -3312,7 +3304,7 @@ bool tci_rrlu_big_fits(int64_t m, int64_t n, int G) {
   return m >= 1 && n >= 1 && m <= 65535 && n <= 65535 && tci_rrlu_big_smem(m, n, G) <= tci_big_smem_limit();
 }
 size_t tci_rrlu_big_scratch_bytes(int grid, int kmax) {
-  return 64 + 2 * (size_t)grid * sizeof(BigSlot) + (size_t)std::max(kmax, 1) * sizeof(double);
+  return 64 + 2 * (size_t)grid * sizeof(BigPartial) + (size_t)std::max(kmax, 1) * sizeof(double);
 }
 
 // Launch on up to `grid` CTAs (all co-resident: cooperative launch).  scratch
@@ -3331,8 +3323,8 @@ cudaError_t tci_rrlu_big_launch(const double* ain, double* work, double* fact, c
   a.fact = fact;
   a.res = res;
   a.bar = (BigBar*)scratch;
-  a.parts = (BigSlot*)((char*)scratch + 64);
-  a.pivs = (double*)((char*)scratch + 64 + 2 * (size_t)grid * sizeof(BigSlot));
+  a.parts = (BigPartial*)((char*)scratch + 64);
+  a.pivs = (double*)((char*)scratch + 64 + 2 * (size_t)grid * sizeof(BigPartial));
   a.m = m;
   a.n = n;
   a.kmax = kmax;
