@@ -1328,8 +1328,10 @@ class rrLU:
 
 def _own_copy(a):
     """a.copy(); of a large matrix by four threads, a block of rows each (numpy
-    copies without the GIL): transposing 8 MB takes one thread 1.8 ms."""
-    if a.size < 1 << 18 or a.shape[0] < 4:
+    copies without the GIL): transposing 8 MB takes one thread 1.8 ms, four 0.6.
+    Starting them takes some 0.2 ms: 200 x 1400 0.17 ms by one thread and 0.25 by
+    four, 300 x 1200 0.20 and 0.25, 400 x 1000 0.29 and 0.27, 512 x 1000 0.81 and 0.41."""
+    if a.size < 400000 or a.shape[0] < 4:
         return a.copy()
     out = np.empty(a.shape, a.dtype)
     rows = [a.shape[0] * q // 4 for q in range(5)]
