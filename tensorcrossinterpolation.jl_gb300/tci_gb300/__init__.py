@@ -1327,10 +1327,18 @@ class rrLU:
 
 
 def _own_copy(a):
-    """a.copy(); of a large matrix by four threads, a block of rows each (numpy
-    copies without the GIL): transposing 8 MB takes one thread 1.8 ms, four 0.6.
-    Starting them takes some 0.2 ms: 200 x 1400 0.17 ms by one thread and 0.25 by
-    four, 300 x 1200 0.20 and 0.25, 400 x 1000 0.29 and 0.27, 512 x 1000 0.81 and 0.41."""
+    """a.copy() of a column-major matrix, which comes from the device: none of it is in
+    a cache, and the transposing copy reads it with a column's stride.  Up to 512 rows
+    some 64 KB of columns at a time, in the order of memory: 200 x 1400 0.34 -> 0.24 ms,
+    256 x 1440 0.72 -> 0.42, 512 x 2048 2.9 -> 0.9.  With longer columns, and many, by
+    four threads, a block of rows each (numpy copies without the GIL; starting them
+    takes 0.2 ms): 1000 x 512 0.20 and 0.25 ms, 2048 x 512 1.6 and 0.6."""
+    width = 8192 // max(a.shape[0], 1)
+    if 16 <= width < a.shape[1]:
+        out = np.empty(a.shape, a.dtype)
+        for j in range(0, a.shape[1], width):
+            out[:, j:j + width] = a[:, j:j + width]
+        return out
     if a.size < 400000 or a.shape[0] < 4:
         return a.copy()
     out = np.empty(a.shape, a.dtype)
