@@ -1344,10 +1344,15 @@ def _own_copy(a):
     out = np.empty(a.shape, a.dtype)
     rows = [a.shape[0] * q // 4 for q in range(5)]
     th = [threading.Thread(target=np.copyto, args=(out[r0:r1], a[r0:r1])) for r0, r1 in zip(rows[1:], rows[2:])]
-    for t in th:
-        t.start()
+    started = 0
+    try:
+        for t in th:
+            t.start()
+            started += 1
+    except RuntimeError:  # no more threads to be had: the rest here
+        np.copyto(out[rows[1 + started]:], a[rows[1 + started]:])
     np.copyto(out[: rows[1]], a[: rows[1]])
-    for t in th:
+    for t in th[:started]:
         t.join()
     return out
 
