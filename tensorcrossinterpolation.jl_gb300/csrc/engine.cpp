@@ -526,10 +526,14 @@ struct MsTimer {
 
 // A lone RRLU task of a single solve from this many elements on runs on a
 // cluster beside the resident kernel (a launch, some 5 us, instead of a ring
-// ticket).  A 30-site quantics solve of rank 80 takes 143 ms without, and with
-// the line at 256 elements 44.5, at 1024 45.6, at 6000 50.3; a 40-site one of
-// rank 11 11.04, 10.81, 11.04, 11.04; an 8-site Lorentzian 4.51 and 3.0 at any.
-static constexpr int64_t COOP_ELEMS = 256;
+// ticket).  Below some 45 x 45 one CTA is faster (a pivot costs it 2 to 4 thousand
+// cycles, a cluster 5), above it the cluster's update.  Milliseconds a solve with the
+// line at 256, 1200, 1800, 2500 and 4000 elements, and in brackets with no clusters:
+// Lorentzian of 8 sites of 4 values 1.95 1.71 1.69 1.67 1.69 (1.86), of 5 2.15 2.07
+// 2.05 1.99 2.00 (2.12), of 11 3.14 3.07 3.06 3.05 3.06 (5.48); quantics of 40 sites
+// 8.66 8.34 8.38 8.36 8.38 (11.6); two-dimensional of 24 sites 13.67 13.49 13.55
+// 13.79 13.93 (39.0), of 30 48.4 47.9 47.9 48.3 49.3 (220).
+static constexpr int64_t COOP_ELEMS = 1800;
 
 // Cluster kernels wait for SMs while other work on the device holds them (of this
 // process or not), the ring's tasks do not: the rest of a solve whose bonds have
