@@ -208,11 +208,9 @@ __global__ void __launch_bounds__(CT, 2)
   }
 }
 
-// The same with one thread per output, FP64 products: a small result has too few
-// tiles for the SMs, and spreads over them so.  The offsets along k are formed once
-// per CTA; eight loads in flight.  A product of host matrices, tiles and so:
-// 60 x 60 x 60 125 and 52 us, 256 x 512 x 100 310 and 228, 512 x 512 x 100 348 and 323,
-// 700 x 700 x 100 360 and 427: the line lies at 2^18 outputs.
+// The same with one thread per output, FP64 products: it spreads evenly over the SMs
+// where tiles do not.  The offsets along k are formed once per CTA; eight loads in
+// flight.
 constexpr int EACH_K = 256;
 __global__ void __launch_bounds__(128)
     gemm_each_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A, tci_map3 a_row, tci_map3 a_k,
@@ -248,26 +246,35 @@ __global__ void __launch_bounds__(128)
   }
   if (on) C[map_at(c_row, i) + map_at(c_col, j)] = acc;
 }
-constexpr int64_t EACH_OUTPUTS = 1 << 18;
 
-// The tile's width by the number of columns: a wider one than needed computes
-// columns past the edge.
+// Tiles or one thread per output.  The tile's width goes by the number of columns: a
+// wider one than needed computes columns past the edge.  Up to one tile per SM takes
+// the time of one, from there on each pair per SM the time of two; against that, one
+// thread per output costs 1.75 times as much an output (two FP64 instructions a term
+// instead of one) and has no edges.  A product of host matrices, microseconds, one
+// thread per output and tiles: 60 x 60 x 60 52 and 125, 512 x 513 x 2000 2277 and 2722,
+// 20000 x 40 x 300 1406 and 1919, 4864 x 65 x 200 402 and 405, 16384 x 16 x 1024 1930
+// and 1568, 4864 x 128 x 200 678 and 459, 900 x 900 x 900 3065 and 2453.
 cudaError_t gemm_map(int64_t M, int64_t N, int64_t K, const double* A, tci_map3 a_row, tci_map3 a_k, const double* B,
                      tci_map3 b_k, tci_map3 b_col, double* C, tci_map3 c_row, tci_map3 c_col, cudaStream_t st) {
   if (M <= 0 || N <= 0) return cudaSuccess;
-  auto grid = [&](int64_t bm, int64_t bn) {
-    const int64_t t = (M + bm - 1) / bm * ((N + bn - 1) / bn);
-    return (unsigned)(t < 65535 * 16 ? t : 65535 * 16);
-  };
-  if (M * N <= EACH_OUTPUTS)
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int64_t bn = N <= 16 ? 16 : N <= 32 ? 32 : 64, bm = bn == 64 ? 64 : 128;
+  const int64_t tiles = (M + bm - 1) / bm * ((N + bn - 1) / bn);
+  const int64_t turns = tiles <= sms ? 1 : 2 * ((tiles + 2 * sms - 1) / (2 * sms));
+  const unsigned grid = (unsigned)(tiles < 65535 * 16 ? tiles : 65535 * 16);
+  if ((double)(turns * bm * bn) * sms > 1.75 * (double)M * (double)N)
     gemm_each_kernel<<<(unsigned)((M * N + 127) / 128), 128, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row,
                                                                       c_col);
-  else if (N <= 16)
-    gemm_map_kernel<16, 2><<<grid(128, 16), CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
-  else if (N <= 32)
-    gemm_map_kernel<32, 4><<<grid(128, 32), CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
+  else if (bn == 16)
+    gemm_map_kernel<16, 2><<<grid, CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
+  else if (bn == 32)
+    gemm_map_kernel<32, 4><<<grid, CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
   else
-    gemm_map_kernel<64, 4><<<grid(64, 64), CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
+    gemm_map_kernel<64, 4><<<grid, CT, 0, st>>>(M, N, K, A, a_row, a_k, B, b_k, b_col, C, c_row, c_col);
   return cudaGetLastError();
 }
 
