@@ -89,7 +89,9 @@ typedef struct tci_server tci_server;
 /* Fill `o` with the reference's defaults (tensorci2.jl:700-720). */
 void tci_opts_default(tci_opts* o);
 
-/* Library / device set-up.  hbm_budget = 0: no limit beyond the device. */
+/* Library / device set-up.  hbm_budget = 0: no limit beyond the device.
+ * tci_ctx_destroy gives the handle up; the context and its memory go with the
+ * last solve, train, server or exported buffer that came from it, in any order. */
 int tci_ctx_create(int device, size_t hbm_budget, tci_ctx** out);
 int tci_ctx_destroy(tci_ctx* ctx);
 const char* tci_last_error(void);

@@ -9,6 +9,7 @@
 #include <mutex>
 #include <optional>
 #include <thread>
+#include <unordered_set>
 #include <cstdlib>
 #include <algorithm>
 #include <condition_variable>
@@ -64,11 +65,40 @@ struct tci_ctx {
   void release_dead();           // with `mu` held
   void release_dead_running();   // the same while the resident kernel is at work
   void release_dead_if_unheld();
-  ~tci_ctx();
+  // The caller's handle, every solve, train, server and exported buffer, and every
+  // call in progress: the context goes with the last of them.  (A garbage collector
+  // finalizes a context and the solves that refer to it in any order.)
+  std::atomic<int64_t> refs{1};
+  std::unordered_set<void*> exported;  // buffers of xpool in the caller's hands (under dead_mu)
+};
+
+// One of a context's references.
+class CtxRef {
+ public:
+  CtxRef() = default;
+  explicit CtxRef(tci_ctx* c) : c_(c) {
+    if (c_) c_->refs.fetch_add(1);
+  }
+  CtxRef(const CtxRef& o) : CtxRef(o.c_) {}
+  CtxRef& operator=(const CtxRef&) = delete;
+  ~CtxRef() { drop(c_); }
+  void set(tci_ctx* c) {
+    c->refs.fetch_add(1);
+    drop(c_);
+    c_ = c;
+  }
+  operator tci_ctx*() const { return c_; }
+  tci_ctx* operator->() const { return c_; }
+  static void drop(tci_ctx* c) {
+    if (c && c->refs.fetch_sub(1) == 1) delete c;
+  }
+
+ private:
+  tci_ctx* c_ = nullptr;
 };
 
 struct tci_solve {
-  tci_ctx* ctx = nullptr;
+  CtxRef ctx;
   Solve s;
 };
 
@@ -93,7 +123,7 @@ class CtxLock {
   CtxLock& operator=(const CtxLock&) = delete;
 
  private:
-  tci_ctx* c_;
+  CtxRef c_;
 };
 
 void tci_ctx::release_dead() {
@@ -137,10 +167,6 @@ void tci_ctx::release_dead_if_unheld() {
     release_dead();
   }
 }
-tci_ctx::~tci_ctx() {
-  if (engp) release_dead();
-}
-
 namespace {
 
 int fail(int code, const std::string& msg) {
@@ -267,7 +293,7 @@ int tci_ctx_create(int device, size_t hbm_budget, tci_ctx** out) {
 }
 
 int tci_ctx_destroy(tci_ctx* ctx) {
-  delete ctx;
+  CtxRef::drop(ctx);
   return 0;
 }
 
@@ -331,7 +357,7 @@ int tci_ctx_stats(tci_ctx* ctx, tci_stats* out, int32_t reset) {
 static int make_solve(tci_ctx* ctx, int32_t L, const int64_t* localdims, int32_t fid, const double* fparams,
                       int64_t nparams, tci_solve** out) {
   auto* h = new tci_solve();
-  h->ctx = ctx;
+  h->ctx.set(ctx);
   int rc = solve_init(h->s, L, localdims, fid, fparams, nparams, nullptr, 0);
   if (rc) {
     delete h;
@@ -374,7 +400,7 @@ int tci_solve_create(tci_ctx* ctx, int32_t L, const int64_t* localdims, int32_t 
 
 int tci_solve_destroy(tci_solve* s) {
   if (!s) return 0;
-  tci_ctx* ctx = s->ctx;
+  const CtxRef ctx(s->ctx);
   ctx->bury(s);
   ctx->release_dead_if_unheld();
   return 0;
@@ -591,13 +617,23 @@ int tci_get_cores_pinned(tci_ctx* ctx, int64_t n, tci_solve* const* solves, doub
     ctx->xpool->free(buf);
     return rc;
   }
+  {
+    std::lock_guard<std::mutex> dl(ctx->dead_mu);
+    ctx->exported.insert(buf);
+  }
+  ctx->refs.fetch_add(1);
   *out = buf;
   *total_elems = total;
   return 0;
 }
 
 int tci_host_free(tci_ctx* ctx, void* p) {
+  {
+    std::lock_guard<std::mutex> lk(ctx->dead_mu);
+    if (!ctx->exported.erase(p)) return 0;
+  }
   ctx->xpool->free(p);
+  CtxRef::drop(ctx);
   return 0;
 }
 
@@ -1083,7 +1119,7 @@ int tci_serve_run(tci_ctx* ctx, int64_t n, const tci_request* reqs, const double
 }  // extern "C"
 
 struct tci_server {
-  tci_ctx* ctx = nullptr;
+  CtxRef ctx;
   int64_t max_live = 0;
   std::mutex mu;
   std::condition_variable cv;
@@ -1145,7 +1181,7 @@ extern "C" {
 
 int tci_serve_start(tci_ctx* ctx, int64_t max_live, tci_server** out) {
   auto* srv = new tci_server();
-  srv->ctx = ctx;
+  srv->ctx.set(ctx);
   srv->max_live = max_live;
   srv->th = std::thread(server_main, srv);
   *out = srv;
@@ -1602,7 +1638,7 @@ int tci_autotune_table(tci_ctx* ctx, int32_t* table, int32_t* nbuckets, int32_t 
 }  // extern "C"
 
 struct tci_tt4 {
-  tci_ctx* ctx = nullptr;
+  CtxRef ctx;
   TT4 tt;
 };
 
@@ -1660,7 +1696,7 @@ int tci_tt4_contract(tci_ctx* ctx, int32_t L, const int64_t* a_dims, const doubl
   if (!rc) rc = upload_tt4(e, L, b_dims, b_cores, b);
   if (!rc) rc = tt4_check_pair(a, b, true);
   std::unique_ptr<tci_tt4> res(new tci_tt4());
-  res->ctx = ctx;
+  res->ctx.set(ctx);
   if (!rc) {
     if (algorithm == TCI_CONTRACT_NAIVE) {
       rc = tt4_contract_naive(e, a, b, res->tt);
@@ -1703,7 +1739,7 @@ int tci_tt4_contract_prec(tci_ctx* ctx, int32_t L, const int64_t* a_dims, const 
   if (!rc) rc = upload_tt4(e, L, b_dims, b_cores, b);
   if (!rc) rc = tt4_check_pair(a, b, true);
   std::unique_ptr<tci_tt4> res(new tci_tt4());
-  res->ctx = ctx;
+  res->ctx.set(ctx);
   SplitRun split;
   if (!rc) rc = tt4_contract_zipup(e, a, b, tolerance, maxbonddim, res->tt, method == TCI_FACTORIZE_CI, &split);
   a.release(e);
@@ -1760,7 +1796,7 @@ int tci_tt4_compress(tci_ctx* ctx, int32_t L, const int64_t* dims, const double*
   if (method != TCI_FACTORIZE_LU && method != TCI_FACTORIZE_CI) return fail(TCI_ERR_GENERIC, "Not implemented yet.");
   Engine& e = ctx->eng_ref();
   std::unique_ptr<tci_tt4> res(new tci_tt4());
-  res->ctx = ctx;
+  res->ctx.set(ctx);
   int rc = upload_tt4(e, L, dims, cores, res->tt);
   if (!rc) rc = tt4_check(res->tt);
   if (!rc) rc = tt4_compress(e, res->tt, tolerance, maxbonddim, normalizeerror != 0, method == TCI_FACTORIZE_CI);
@@ -1813,7 +1849,7 @@ int tci_tt4_contract_tci(tci_ctx* ctx, int32_t L, const int64_t* a_dims, const d
     if (rc) return rc;
   }
   std::unique_ptr<tci_tt4> res(new tci_tt4());
-  res->ctx = ctx;
+  res->ctx.set(ctx);
   rc = tt4_contract_tci(e, std::move(a), std::move(b), piv, ninitialpivots > 0 ? ninitialpivots : 10, f, user, o,
                         res->tt);
   if (rc) {
