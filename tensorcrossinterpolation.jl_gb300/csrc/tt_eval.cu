@@ -76,12 +76,47 @@ __device__ __forceinline__ void row_times_cols(const double* __restrict__ v, int
   }
 }
 
+// The sum for one output, eight terms' loads and products before their additions.
+template <int MODE>
+__device__ __forceinline__ double row_times_col(const double* __restrict__ v, int P, const double* __restrict__ col,
+                                                int r0) {
+  double acc = 0.0;
+  for (int t = 0; t < r0; t += 8) {
+    double x[8], c[8], q[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int tk = min(t + k, r0 - 1);
+      x[k] = v[(size_t)tk * P];
+      c[k] = __ldg(col + tk);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      q[k] = MODE == VAL_DENSE ? int_mul_dense(dense_split(x[k]), dense_split(c[k]))
+                               : (MODE == VAL_ZEROS ? int_mul(int_split(x[k]), int_split(c[k])) : __dmul_rn(x[k], c[k]));
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (t + k < r0) acc = __dadd_rn(acc, q[k]);
+  }
+  return acc;
+}
+
 // One site for the CTA's points: w = v * T[:, i, :].  Returns the largest class
 // of the values written by this thread.
 template <int MODE>
 __device__ __forceinline__ int site_step(const tci_core_ref& c, const uint8_t* __restrict__ pts, int L, int s, int np,
                                          int P, const double* v, double* w) {
   int cls = VAL_DENSE;
+  if (P * c.r1 <= NT) {  // few points: a thread for each output
+    const int p = threadIdx.x % P, q = threadIdx.x / P;
+    if (q < c.r1 && p < np) {
+      const double* col = c.p + (size_t)c.r0 * (pts[(size_t)p * L + s] + (size_t)c.d * q);
+      const double a = P * c.r1 <= NT / 4 ? row_times_col<VAL_UNSAFE>(v + p, P, col, c.r0)
+                                          : row_times_col<MODE>(v + p, P, col, c.r0);
+      w[(size_t)q * P + p] = a;
+      cls = val_class(a);
+    }
+    return cls;
+  }
   const int nq = (c.r1 + 3) >> 2;
   for (int e = threadIdx.x; e < P * nq; e += NT) {
     const int p = e % P, q0 = (e / P) * 4;  // P is a power of two
