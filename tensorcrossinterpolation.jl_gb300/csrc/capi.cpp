@@ -1311,6 +1311,11 @@ int tci_convergencecriterion(const int64_t* ranks, const double* errors, const i
 }
 
 // ---------------------------------------------------------------- rrLU
+// Elements up to which the host forms L and U: a kernel, two more copies and a block
+// for them take some 25 us, what the host's pass over 150 x 150 does.  A call by the
+// host and by the device: 10 x 10 69 and 93 us, 64 x 64 246 and 268, 100 x 100 to rank
+// 10 103 and 124, 256 x 256 1143 and 1145, 400 x 400 to rank 200 1657 and 1530.
+static constexpr int64_t HOST_FACTORS = 1 << 15;
 int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxrank, double reltol,
              double abstol, int32_t leftorthogonal, int64_t* rowperm, int64_t* colperm, double* L, double* U,
              int64_t* npivot, double* error) {
@@ -1348,26 +1353,45 @@ int tci_rrlu(tci_ctx* ctx, const double* A, int64_t m, int64_t n, int64_t maxran
   }
   const tci_result_head* h = r.head();
   const int K = h->npivot;
-  // the permutations, and L and U as compact matrices, straight to the caller
-  std::vector<int32_t> perms((size_t)(m + n));
   const size_t nl = (size_t)m * K, nu = (size_t)K * n;
-  if (!touched) {
-    touch_pages(L, nl);
-    touch_pages(U, nu);
+  const bool wanted = (L || U) && nl + nu > 0;
+  // A small matrix comes as it is, in one copy with the permutations, and the host
+  // forms L and U; of a large one L and U are formed on the device and go straight to
+  // the caller, without the host's pass.
+  const size_t nf = wanted && m * n <= HOST_FACTORS ? (size_t)(m * n) : 0;
+  std::vector<double> fact(nf + ((size_t)(m + n) * 4 + 7) / 8);
+  const double* F = fact.data();
+  const int32_t* perms = (const int32_t*)(F + nf);
+  cudaError_t ce = cudaSuccess;
+  if (m + n > 0)
+    ce = cudaMemcpyAsync(fact.data(), dout + (m * n - nf), nf * 8 + (size_t)(m + n) * 4, cudaMemcpyDeviceToHost,
+                         e.stream());
+  double* lu = nullptr;
+  if (ce == cudaSuccess && wanted && !nf) {
+    if (!touched) {
+      touch_pages(L, nl);
+      touch_pages(U, nu);
+    }
+    lu = e.alloc_core(nl + nu);
+    ce = lu ? tci_lu_factors_launch(dout, (int)m, (int)n, K, leftorthogonal ? 1 : 0, lu, lu + nl, e.stream())
+            : cudaErrorMemoryAllocation;
+    if (ce == cudaSuccess && L) ce = cudaMemcpyAsync(L, lu, nl * 8, cudaMemcpyDeviceToHost, e.stream());
+    if (ce == cudaSuccess && U) ce = cudaMemcpyAsync(U, lu + nl, nu * 8, cudaMemcpyDeviceToHost, e.stream());
   }
-  double* lu = (L || U) && nl + nu > 0 ? e.alloc_core(nl + nu) : nullptr;
-  cudaError_t ce = (L || U) && nl + nu > 0 && !lu ? cudaErrorMemoryAllocation : cudaSuccess;
-  if (ce == cudaSuccess && m + n > 0)
-    ce = cudaMemcpyAsync(perms.data(), dout + m * n, perms.size() * 4, cudaMemcpyDeviceToHost, e.stream());
-  if (ce == cudaSuccess && lu)
-    ce = tci_lu_factors_launch(dout, (int)m, (int)n, K, leftorthogonal ? 1 : 0, lu, lu + nl, e.stream());
-  if (ce == cudaSuccess && lu && L) ce = cudaMemcpyAsync(L, lu, nl * 8, cudaMemcpyDeviceToHost, e.stream());
-  if (ce == cudaSuccess && lu && U) ce = cudaMemcpyAsync(U, lu + nl, nu * 8, cudaMemcpyDeviceToHost, e.stream());
   const cudaError_t sync = cudaStreamSynchronize(e.stream());
   if (lu) e.free_core(lu);
   e.free_core(dout);
   if (ce == cudaSuccess) ce = sync;
   if (ce != cudaSuccess) return fail(ce == cudaErrorMemoryAllocation ? TCI_ERR_OOM : TCI_ERR_CUDA, cudaGetErrorString(ce));
+  // L = tril(A[:, 1:K]), U = triu(A[1:K, :]), unit diagonal on L or U (matrixlu.jl:162-174)
+  if (nf && L)
+    for (int64_t j = 0; j < K; ++j)
+      for (int64_t i = 0; i < m; ++i)
+        L[i + j * m] = i < j ? 0.0 : (i == j && leftorthogonal ? 1.0 : F[i + j * m]);
+  if (nf && U)
+    for (int64_t j = 0; j < n; ++j)
+      for (int64_t i = 0; i < K; ++i)
+        U[i + j * K] = i > j ? 0.0 : (i == j && !leftorthogonal ? 1.0 : F[i + j * m]);
   if (rowperm)
     for (int64_t i = 0; i < m; ++i) rowperm[i] = perms[i] + 1;
   if (colperm)
