@@ -1383,14 +1383,30 @@ def rrlu_batched(mats, maxrank=None, reltol=1e-14, abstol=0.0, leftorthogonal=Tr
     ctx = ctx or default_context()
     if not len(mats):
         raise ValueError("need at least one matrix")
-    # the matrices where they are (column-major float64; others are copied): their
-    # places relative to the lowest one, in doubles
-    cols = [np.require(a, np.float64, ["F", "A"]) for a in mats]
-    ms = np.array([a.shape[0] for a in cols], np.int64)
-    ns = np.array([a.shape[1] for a in cols], np.int64)
-    addr = np.array([a.ctypes.data for a in cols], np.int64)
-    base = int(addr.min())
-    offs = np.ascontiguousarray((addr - base) // 8)
+    ms = np.array([a.shape[0] for a in mats], np.int64)
+    ns = np.array([a.shape[1] for a in mats], np.int64)
+    sizes = ms * ns
+    if sizes.sum() < 2048 * len(mats):
+        # small ones one after the other: finding where an array lies takes numpy 2 us,
+        # copying 16 KB 1 (300 of 16 x 16 in all 0.67 ms so, 0.91 in place)
+        keep = [np.concatenate([np.asarray(a, np.float64).reshape(-1, order="F") for a in mats])]
+        base = keep[0].ctypes.data
+        offs = np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.int64)
+    else:
+        # column-major float64 where it is, everything else copied into one array;
+        # their places relative to the lowest one, in doubles
+        keep = [np.asarray(a, np.float64) for a in mats]
+        here = np.array([a.flags.f_contiguous and a.flags.aligned for a in keep])
+        ends = np.cumsum(np.where(here, 0, sizes))
+        flat = np.empty(int(ends[-1]))
+        addr = flat.ctypes.data + 8 * (ends - sizes)
+        for i, a in enumerate(keep):
+            if here[i]:
+                addr[i] = a.ctypes.data
+            else:
+                flat[ends[i] - sizes[i]:ends[i]].reshape(a.shape, order="F")[...] = a
+        base = int(addr.min())
+        offs = np.ascontiguousarray((addr - base) // 8)
     kcap = np.minimum(np.minimum(ms, ns), maxrank if maxrank else np.iinfo(np.int64).max)
     poffs = np.concatenate([[0], np.cumsum(2 * kcap)[:-1]]).astype(np.int64)
     piv = np.zeros(int(2 * kcap.sum()) + 1, np.int64)
