@@ -1642,21 +1642,19 @@ int solve_init(Solve& s, int L, const int64_t* localdims, int fid, const double*
   // sum (v - c)^2 over [0, sum max((d - c)^2, (1 - c)^2)]
   s.lutcap0 = s.lutcap1 = 0;
   if (fid == TCI_F_LORENTZ || fid == TCI_F_SERVED) {
-    int64_t hi0 = 0, hi1 = 0;
+    // (in doubles: far centres have squares beyond 64 bits)
+    double hi0 = 0, hi1 = 0;
     for (int p = 0; p < L; ++p) {
-      hi0 += (int64_t)s.d[p] * s.d[p];
+      hi0 += (double)s.d[p] * s.d[p];
       if (fid == TCI_F_SERVED) {
-        int64_t c = (int64_t)params[3 + p];
-        int64_t a = (int64_t)s.d[p] - c, b = 1 - c;
+        const double c = std::trunc(params[3 + p]), a = s.d[p] - c, b = 1 - c;
         hi1 += std::max(a * a, b * b);
       }
     }
-    if (hi0 - L + 1 <= (1 << 20)) s.lutcap0 = (int)(hi0 - L + 1);
-    if (fid == TCI_F_SERVED) {
-      if (hi1 + 1 <= (1 << 20) && s.lutcap0 > 0)
-        s.lutcap1 = (int)(hi1 + 1);
-      else
-        s.lutcap0 = 0;
+    const double most = 1 << 20;
+    if (hi0 - L + 1 <= most && (fid == TCI_F_LORENTZ || hi1 + 1 <= most)) {  // (not for a NaN)
+      s.lutcap0 = (int)(hi0 - L + 1);
+      if (fid == TCI_F_SERVED) s.lutcap1 = (int)hi1 + 1;
     }
   }
   s.pivoterrors.clear();

@@ -1837,7 +1837,7 @@ __device__ void task_search(const tci_task& T, const char* blob, char* resb, cha
       tout[it] = val;
     }
     FSums a;
-    if (tci_f_tables(T.fid) > 0) {  // the same sums, exact integers, off the FP64 pipe
+    if (tci_f_tables(T.fid) > 0 && T.lutcap0 > 0) {  // the same sums, exact integers, off the FP64 pipe
       long long i0 = 0, i1 = 0;
       for (int s = 0; s < L; ++s) tci_f_term_int(T.fid, prm, s, s == p ? v : st[s], &i0, &i1);
       a.a0 = (double)i0;
