@@ -351,19 +351,22 @@ __device__ __forceinline__ bool int_states(const tci_task& T) {
   return tci_f_tables(T.fid) > 0 && T.lut != nullptr && T.lutcap0 > 0;
 }
 // The registered f of its two sums, and the sums of `len` sites from site0 on with
-// local values v (site `over` of them taken as `val`).  Out of line: a task's fills,
-// states and points share one copy of the code, which a small task would otherwise
-// wait for more than once.
+// local values v (site `over` of them taken as `val`).  Out of line: a task's fills
+// and states share one copy of the code, which a small task would otherwise wait for
+// more than once.
 __device__ __noinline__ double f_finish(int fid, const double* prm, int nparams, double a0, double a1) {
   return tci_f_finish(fid, prm, nparams, a0, a1);
 }
 struct FSums {
   double a0, a1;
 };
+__device__ __forceinline__ bool f_digits(int fid, int site0, int len) {
+  return (fid == TCI_F_QTT1D || fid == TCI_F_QTT2D) && len <= 53 && site0 + len <= 1022;
+}
 __device__ __noinline__ FSums f_sums(int fid, const double* prm, int site0, int len, const uint8_t* v, int over,
                                      int val) {
   FSums a{0.0, 0.0};
-  if ((fid == TCI_F_QTT1D || fid == TCI_F_QTT2D) && len <= 53 && site0 + len <= 1022) {
+  if (f_digits(fid, site0, len)) {
     // binary digits: every partial sum is exact, so they are collected as an
     // integer (an FP64 addition per site takes a warp 64 cycles of its SM quarter)
     unsigned long long q0 = 0, q1 = 0;
@@ -379,6 +382,23 @@ __device__ __noinline__ FSums f_sums(int fid, const double* prm, int site0, int 
     for (int p = 0; p < len; ++p) tci_f_term(fid, prm, site0 + p, p == over ? val : v[p], &a.a0, &a.a1);
   }
   return a;
+}
+
+// f at one multi-index, inline: in a task of points there is nothing to share the code
+// with, and the calls made the search of a product function 14 % slower.
+__device__ __forceinline__ double f_point(const tci_task& T, const double* prm, const uint8_t* v, int over, int val) {
+  FSums a{0.0, 0.0};
+  if (tci_f_tables(T.fid) > 0 && T.lutcap0 > 0) {  // the same sums, exact integers, off the FP64 pipe
+    long long i0 = 0, i1 = 0;
+    for (int s = 0; s < T.L; ++s) tci_f_term_int(T.fid, prm, s, s == over ? val : v[s], &i0, &i1);
+    a.a0 = (double)i0;
+    a.a1 = (double)i1;
+  } else if (f_digits(T.fid, 0, T.L)) {
+    a = f_sums(T.fid, prm, 0, T.L, v, over, val);
+  } else {
+    for (int s = 0; s < T.L; ++s) tci_f_term(T.fid, prm, s, s == over ? val : v[s], &a.a0, &a.a1);
+  }
+  return tci_f_finish(T.fid, prm, T.nparams, a.a0, a.a1);
 }
 
 // A list of `count` multi-indices of `len` sites from site0 on, and where their
@@ -1617,10 +1637,7 @@ __device__ void task_eval(const tci_task& T, const char* blob, char* resb, char*
   char* base = atw(resb, T.res);
   double* fout = (double*)(base + sizeof(tci_result_head));
   double* tout = fout + np;
-  for (int p = tid; p < np; p += NT) {
-    const FSums a = f_sums(T.fid, prm, 0, L, pts + (size_t)p * L, -1, 0);
-    fout[p] = f_finish(T.fid, prm, T.nparams, a.a0, a.a1);
-  }
+  for (int p = tid; p < np; p += NT) fout[p] = f_point(T, prm, pts + (size_t)p * L, -1, 0);
   if (T.cores && T.r <= EVAL_THREAD_RMAX) {
     // bonds up to EVAL_THREAD_RMAX: one thread per point (a warp per point would
     // leave most lanes idle), the running vector in the thread's own column of
@@ -1836,16 +1853,7 @@ __device__ void task_search(const tci_task& T, const char* blob, char* resb, cha
                                                        1, c.r0), env[roff[p] + b]));
       tout[it] = val;
     }
-    FSums a;
-    if (tci_f_tables(T.fid) > 0 && T.lutcap0 > 0) {  // the same sums, exact integers, off the FP64 pipe
-      long long i0 = 0, i1 = 0;
-      for (int s = 0; s < L; ++s) tci_f_term_int(T.fid, prm, s, s == p ? v : st[s], &i0, &i1);
-      a.a0 = (double)i0;
-      a.a1 = (double)i1;
-    } else {
-      a = f_sums(T.fid, prm, 0, L, st, p, v);
-    }
-    fout[it] = f_finish(T.fid, prm, T.nparams, a.a0, a.a1);
+    fout[it] = f_point(T, prm, st, p, v);
   }
   if (tid == 0) {
     tci_result_head* h = (tci_result_head*)base;
