@@ -882,34 +882,13 @@ void BlockPool::free(void* p) {
 }
 
 // ---------------------------------------------------------------- resident ring
-namespace {
-struct DeviceCount {
-  std::mutex mu;
-  int users = 0;
-};
-DeviceCount& device_count(int device) {
-  static DeviceCount c[64];
-  return c[device & 63];
+static std::atomic<int>& device_users(int device) {
+  static std::atomic<int> n[64];
+  return n[device & 63];
 }
-}  // namespace
-
-void DeviceUsers::enter(int device) {
-  DeviceCount& c = device_count(device);
-  std::lock_guard<std::mutex> lk(c.mu);
-  ++c.users;
-}
-void DeviceUsers::leave(int device) {
-  DeviceCount& c = device_count(device);
-  std::lock_guard<std::mutex> lk(c.mu);
-  --c.users;
-}
-bool DeviceUsers::alone(int device, const std::function<void()>& enqueue) {
-  DeviceCount& c = device_count(device);
-  std::lock_guard<std::mutex> lk(c.mu);
-  if (c.users > 1) return false;
-  enqueue();
-  return true;
-}
+void DeviceUsers::enter(int device) { device_users(device).fetch_add(1); }
+void DeviceUsers::leave(int device) { device_users(device).fetch_sub(1); }
+bool DeviceUsers::alone(int device) { return device_users(device).load() <= 1; }
 
 int ResidentQueue::init(int dev, int num_sms, int idle_us) {
   device = dev;
@@ -947,7 +926,7 @@ ResidentQueue::~ResidentQueue() {
 int ResidentQueue::start(const tci_kernel_set* k, int clusters, int cluster_ctas) {
   std::lock_guard<std::mutex> lk(mu);
   if (running) return k == ks && cluster == cluster_ctas ? 0 : fail(TCI_ERR_GENERIC, "resident kernel already running in another variant");
-  if (clusters > 0 && !DeviceUsers::alone(device, [] {})) clusters = cluster_ctas = 0;
+  if (clusters > 0 && !DeviceUsers::alone(device)) clusters = cluster_ctas = 0;
   ks = k;
   cluster = cluster_ctas;
   grid = clusters > 0 ? clusters * cluster : num_sms * ks->ctas_per_sm;
@@ -1035,7 +1014,7 @@ void Engine::set_resident(ResidentQueue* q, BlockPool* host_pool, BlockPool* scr
 int Engine::cooperative_ctas(const Req& r, size_t batch) const {
   const tci_task& t = r.t;
   if (!coop_most_ || batch != 1 || inflight_tasks_ != 0 || t.kind != TCI_TASK_RRLU || t.post != TCI_POST_NONE ||
-      t.ain || r.ain_host || (int64_t)t.m * t.n < COOP_ELEMS)
+      t.ain || r.ain_host || (int64_t)t.m * t.n < COOP_ELEMS || !DeviceUsers::alone(device_))
     return 0;
   return tci_k256::tci_rrlu_cluster_ctas(t, coop_most_);
 }
@@ -1124,24 +1103,19 @@ int Engine::submit() {
           break;
         }
         f.dblocks.push_back(pivs);
-        cudaError_t ce = cudaSuccess;
-        const bool out = DeviceUsers::alone(device_, [&] {
-          r.ticket = t.ticket = ++coop_seq_;
-          ce = tci_k256::tci_rrlu_cluster_launch(t, ncta, pivs, stream_);
-        });
+        r.ticket = t.ticket = ++coop_seq_;
+        const cudaError_t ce = tci_k256::tci_rrlu_cluster_launch(t, ncta, pivs, stream_);
         if (ce != cudaSuccess) {
           rc = fail(TCI_ERR_CUDA, cudaGetErrorString(ce));
           break;
         }
-        if (out) {
-          stats.launches += 1;
-          stats.h2d_bytes += (int64_t)o_res;
-          stats.d2h_bytes += (int64_t)r.res_bytes;
-          f.cluster = true;
-          f.sent = std::chrono::steady_clock::now();
-          f.reqs.push_back(&r);
-          continue;
-        }
+        stats.launches += 1;
+        stats.h2d_bytes += (int64_t)o_res;
+        stats.d2h_bytes += (int64_t)r.res_bytes;
+        f.cluster = true;
+        f.sent = std::chrono::steady_clock::now();
+        f.reqs.push_back(&r);
+        continue;
       }
       t.cost = task_cost(t);
       // small inputs are copied to shared memory in one parallel pass when the

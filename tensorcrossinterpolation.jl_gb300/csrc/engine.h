@@ -9,7 +9,6 @@
 #include <coroutine>
 #include <cstdio>
 #include <cstdint>
-#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -172,9 +171,9 @@ class BlockPool {
 struct DeviceUsers {
   static void enter(int device);
   static void leave(int device);
-  // Runs `enqueue` unless a second context is at work (none enters meanwhile);
-  // whether it ran.
-  static bool alone(int device, const std::function<void()>& enqueue);
+  // No second context is at work.  (One that enters right after costs a bond the wait
+  // that all of them had before, once.)
+  static bool alone(int device);
 };
 
 // The ring of the resident kernel, shared by the engines of a context.
