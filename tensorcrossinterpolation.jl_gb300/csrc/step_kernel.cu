@@ -16,10 +16,12 @@
 //          abstracttensortrain.jl:124-132).
 //
 // Bit-exactness of the pivots: the rank-1 update is a separate IEEE multiply and
-// subtract (__dmul_rn/__dsub_rn, as the reference's loop at matrixlu.jl:128-134
-// is compiled without FMA), scaling is an IEEE division (matrixlu.jl:119-123),
-// and the argmax compares abs2 = v*v with strict '>' and breaks ties towards the
-// first element in column-major order of the physically permuted matrix
+// subtract (as the reference's loop at matrixlu.jl:128-134 is compiled without FMA),
+// scaling is an IEEE division (matrixlu.jl:119-123); the products and quotients are
+// formed on the integer pipes, correctly rounded (ieee_int.h), and by __dmul_rn and
+// __ddiv_rn for operands outside its range.  The argmax compares abs2 = v*v with
+// strict '>' and breaks ties towards the first element in column-major order of the
+// physically permuted matrix
 // (matrixlu.jl:16-31).  The comparison of v*v is skipped for elements whose |v|
 // is more than 16 ulps below the running maximum, where v*v is provably smaller.
 #include <cooperative_groups.h>
@@ -2186,10 +2188,9 @@ __global__ void __launch_bounds__(NT, TCI_CTAS_PER_SM)
 // trailing block), and the stored factors are divided the same way when they
 // are written out.  Per pivot: every CTA reduces the G partial argmaxes (same
 // result everywhere), takes the decision, forms its x and y slices, updates its
-// block of the trailing matrix fused with its partial argmax, and meets the
-// others at ONE grid barrier.  The arithmetic per element is the same
-// __dmul_rn/__dsub_rn/__ddiv_rn sequence as rrlu_loop, so the factors are
-// bit-identical.
+// block of the trailing matrix fused with its partial argmax, and publishes that; the
+// next pivot's wait for the partials is the only one on the other CTAs.  Products,
+// quotients and subtractions are those of rrlu_loop, so the factors are bit-identical.
 
 struct BigBar {
   unsigned int count, gen;
