@@ -3236,6 +3236,10 @@ __device__ ClusterResult cluster_rrlu(const ClusterJob& P, char* smem, ClusterCt
   return r;
 }
 
+// The smallest cluster to try for a matrix of `elems` elements, of at most `most` CTAs:
+// up to 100 x 100 the update does not fill eight.
+inline int cluster_first(int64_t elems, int most) { return most > 8 && elems >= 10000 ? 16 : 8; }
+
 // CTA grid of a cluster of `ncta` (a power of two) for an m x n matrix: the
 // smallest block perimeter (x and y exchanged per pivot).
 struct ClusterGrid {
@@ -3553,8 +3557,7 @@ int tci_rrlu_cluster_most(int* clusters) {
 // CTAs for an RRLU task on clusters of at most `most`; 0 if it does not fit.
 int tci_rrlu_cluster_ctas(const tci_task& t, int most) {
   if (t.m > 65535 || t.n > 65535 || t.m < 1 || t.n < 1) return 0;
-  for (int c = 8; c <= most; c *= 2) {
-    if (c == 8 && most > 8 && (int64_t)t.m * t.n >= 10000) continue;
+  for (int c = cluster_first((int64_t)t.m * t.n, most); c <= most; c *= 2) {
     const ClusterGrid g = cluster_grid(t.m, t.n, c);
     const size_t state = t.ain ? 0 : cluster_state_smem(g.mb, g.nb, t.nl, t.nr);
     if (cluster_smem16(t.m, t.n, g.mb, g.nb) + state <= CL_SMEM) return c;
@@ -3695,7 +3698,7 @@ __global__ void rrlu_noalloc_epilogue(const double* fact, const char* resb, int 
 // array's size nothing remains to spill to.
 int noalloc_cluster(int64_t m, int64_t n, int most, int* nres) {
   if (m * n < NOALLOC_CLUSTER_ELEMS) return 0;
-  for (int c = m * n < NOALLOC_CLUSTER_ELEMS * 4 ? 8 : 16; c <= most; c *= 2) {
+  for (int c = cluster_first(m * n, most); c <= most; c *= 2) {
     const ClusterGrid g = cluster_grid((int)m, (int)n, c);
     const size_t fixed = cluster_smem((int)m, (int)n, g.mb, g.nb, 0);
     if (fixed >= CL_SMEM) continue;
